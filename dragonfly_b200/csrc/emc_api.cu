@@ -17,6 +17,7 @@
 #include "emc_device.cuh"
 #include "emc_bg.cuh"
 #include "emc_dense.cuh"
+#include "emc_hot.cuh"
 #include "emc_pairs.cuh"
 
 using namespace dfg;
@@ -256,6 +257,7 @@ extern "C" int dfg_set_frames(dfg_ctx *ctx, int num_data, const int *ones, const
 		mc += fc[d];
 	}
 	ctx->mean_count = mc / N;
+	ctx->max_fcount = *std::max_element(fc.begin(), fc.end());
 	ctx->n_ph = real;
 	CK(upload(ctx->ph, words.data(), words.size(), ctx->stream));
 	CK(upload(ctx->ph_off, off.data(), off.size(), ctx->stream));
@@ -670,6 +672,10 @@ extern "C" int dfg_calc_beta(dfg_ctx *ctx, double start, int need_scaling) {
 // ---------------------------------------------------------------------------
 // work buffers and the frame chunks
 // ---------------------------------------------------------------------------
+// Largest photon sum that the byte products' INT32 accumulators hold: 2^24
+// counts times a digit of at most 128 in magnitude.
+constexpr long long kHotMaxSum = 1LL << 24;
+
 static int build_chunks(dfg_ctx *ctx) {
 	const int N = ctx->N, P = ctx->P;
 	// per frame: pval and Pst of every orientation, plus its BF16 count row
@@ -701,8 +707,10 @@ static int build_chunks(dfg_ctx *ctx) {
 	// row Nc.
 	NEED(nc <= (long long)IDX_MASK, DFG_ERR_ARG, "frame chunk of %lld frames exceeds %u", nc, IDX_MASK);
 	const uint8_t *mk = ctx->h_mask.data();
-	std::vector<long long> c1(P + 1), cm(P + 1);
+	std::vector<long long> c1(P + 1), cm(P + 1), photons(P + 1);
 	std::vector<uint32_t> words;
+	ctx->h_pix_entries.assign((size_t)P, 0);
+	ctx->h_pix_big.assign((size_t)P, 0);
 	for (int k = 0; k < n_chunks; ++k) {
 		Chunk &ch = ctx->chunks[k];
 		ch.d0 = (int)(k * nc);
@@ -710,6 +718,7 @@ static int build_chunks(dfg_ctx *ctx) {
 		const uint32_t pad = (uint32_t)ch.nc;
 		std::fill(c1.begin(), c1.end(), 0);
 		std::fill(cm.begin(), cm.end(), 0);
+		std::fill(photons.begin(), photons.end(), 0);
 		auto each = [&](auto fn) {
 			for (int dl = 0; dl < ch.nc; ++dl) {
 				int d = ch.d0 + dl;
@@ -730,6 +739,9 @@ static int build_chunks(dfg_ctx *ctx) {
 				c1[p]++;
 			else
 				cm[p] += (c + MAX_COUNT - 1) / MAX_COUNT;
+			photons[p] += c;
+			if (c > 255)
+				ctx->h_pix_big[p] = 1;
 		});
 		std::vector<long long> off(P + 1, 0), midv(P, 0), f1(P), fm(P);
 		long long real = 0;
@@ -740,6 +752,9 @@ static int build_chunks(dfg_ctx *ctx) {
 			fm[p] = midv[p];
 			off[p + 1] = off[p] + a + b;
 			real += c1[p] + cm[p];
+			ctx->h_pix_entries[p] += c1[p] + cm[p];
+			if (photons[p] >= kHotMaxSum)
+				ctx->h_pix_big[p] = 1;
 		}
 		words.assign((size_t)off[P], pad);
 		each([&](int p, int dl, long long c) {
@@ -768,9 +783,13 @@ static int build_chunks(dfg_ctx *ctx) {
 		CK(cudaStreamSynchronize(ctx->stream));
 	}
 	ctx->chunks_R = ctx->R;
+	ctx->layout++;
 	ctx->chunks_dense = (ctx->dense_active ? 1 : 0) | (ctx->m_dense_active ? 2 : 0);
 	return DFG_OK;
 }
+
+// Frame ranges of the psum_r partial sums.
+static int psum_splits(const dfg_ctx *ctx) { return std::max(1, std::min(64, ctx->chunk_frames / 2048)); }
 
 static int ensure_buffers(dfg_ctx *ctx) {
 	NEED(ctx->P > 0, DFG_ERR_STATE, "detector not set");
@@ -820,8 +839,7 @@ static int ensure_buffers(dfg_ctx *ctx) {
 	CK(ctx->tmax.ensure((size_t)ctx->RT * ctx->chunk_frames));
 	CK(ctx->targ.ensure((size_t)ctx->RT * ctx->chunk_frames));
 	CK(ctx->tlive.ensure((size_t)ctx->RT * (ctx->chunk_frames + 1)));
-	const int nsplit = std::max(1, std::min(64, ctx->chunk_frames / 2048));
-	CK(ctx->psum_part.ensure((size_t)nsplit * ctx->R_pad));
+	CK(ctx->psum_part.ensure((size_t)psum_splits(ctx) * ctx->R_pad));
 	return DFG_OK;
 }
 
@@ -1161,6 +1179,221 @@ static void dense_release(dfg_ctx *ctx) {
 	std::fill(ctx->map_src, ctx->map_src + 6, nullptr);
 }
 
+// ---------------------------------------------------------------------------
+// hot pixels (emc_hot.cuh)
+// ---------------------------------------------------------------------------
+// Tensor map of a row-major byte matrix [rows][pitch] read in boxes of 128
+// columns x 256 rows with the 128-byte swizzle (rows past the end read zero).
+static int encode_byte_map(dfg_ctx *ctx, CUtensorMap *map, const void *base, long long rows, long long pitch) {
+	auto fn = tensor_map_encoder();
+	NEED(fn != nullptr, DFG_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+	cuuint64_t dims[2] = {(cuuint64_t)pitch, (cuuint64_t)rows};
+	cuuint64_t strides[1] = {(cuuint64_t)pitch};
+	cuuint32_t box[2] = {(cuuint32_t)HK, (cuuint32_t)HM};
+	cuuint32_t estr[2] = {1, 1};
+	const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
+	                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+	                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+	NEED(r == CUDA_SUCCESS, DFG_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+	return DFG_OK;
+}
+
+// A pixel is hot when at least this share of the frames has photons on it. A
+// gathered photon word costs its row through the L2 path, a product column costs
+// the tensor pipe the same for every frame: iteration ms at thresholds 0.006 /
+// 0.012 / 0.02 / 0.04: production geometry (50100 orientations, 60000 frames)
+// 468 / 449 / 469 / 539 against 583 without products; 95^3, 17220 x 40000:
+// 27.1 / 26.2 / 26.8 / 29.1 against 55.9; 125^3 near the solution, 10860 x
+// 30000: 22.5 / 22.1 / 22.9 / 26.5 against 57.3; 1500 photons, 6300 x 15000:
+// 8.5 / 8.5 / 8.6 / 9.5 against 39.6.
+constexpr double kHotOccupancy = 0.012;
+
+// Chooses the hot pixels of the current chunk layout and lays out what depends
+// on the frames alone: the count matrices of every chunk and the photon lists
+// without them. hot_n = 0 leaves everything to the gathers.
+static int hot_choose(dfg_ctx *ctx) {
+	const int N = ctx->N, P = ctx->P;
+	cudaStream_t st = ctx->stream;
+	ctx->hot_n = 0;
+	ctx->hot_layout = ctx->layout;
+	ctx->phc.release();
+	for (Chunk &ch : ctx->chunks) {
+		ch.by_frame.release();
+		ch.by_pixel.release();
+		ch.pix_cold.release();
+	}
+	if (TILE != 128 || ctx->chunk_frames < HM || ctx->max_fcount >= kHotMaxSum)
+		return DFG_OK;
+	std::vector<int> cand;
+	for (int p = 0; p < P; ++p)
+		if (ctx->h_mask[p] == 0 && !ctx->h_pix_big[p] && ctx->h_pix_entries[p] > 0)
+			cand.push_back(p);
+	std::stable_sort(cand.begin(), cand.end(),
+	                 [&](int a, int b) { return ctx->h_pix_entries[a] > ctx->h_pix_entries[b]; });
+	long long m = 0;
+	while (m < (long long)cand.size() && (double)ctx->h_pix_entries[cand[m]] >= kHotOccupancy * N)
+		++m;
+	const int n = (int)std::min<long long>((m + HK / 2) / HK * HK, (long long)cand.size());
+	if (n < HK)
+		return DFG_OK;
+	cand.resize(n);
+	const int pitch = (n + HK - 1) / HK * HK;
+	std::vector<uint8_t> is_hot((size_t)P, 0);
+	for (int p : cand)
+		is_hot[p] = 1;
+	CK(upload(ctx->hot_pix, cand.data(), cand.size(), st));
+	CK(upload(ctx->is_hot, is_hot.data(), is_hot.size(), st));
+	// a failure to allocate leaves the gathers in charge
+	auto fits = [](cudaError_t e) {
+		if (e == cudaErrorMemoryAllocation)
+			cudaGetLastError();
+		return e;
+	};
+	bool room = true;
+	for (Chunk &ch : ctx->chunks) {
+		ch.k_pitch = (ch.nc + HK - 1) / HK * HK;
+		cudaError_t e = fits(ch.by_frame.ensure((size_t)ch.nc * pitch));
+		if (e == cudaSuccess)
+			e = fits(ch.by_pixel.ensure((size_t)n * ch.k_pitch));
+		if (e == cudaErrorMemoryAllocation) {
+			room = false;
+			break;
+		}
+		CK(e);
+		CK(cudaMemsetAsync(ch.by_frame.p, 0, (size_t)ch.nc * pitch, st));
+		CK(cudaMemsetAsync(ch.by_pixel.p, 0, (size_t)n * ch.k_pitch, st));
+		hot_counts_kernel<<<blocks_for((long long)n * 32, 256), 256, 0, st>>>(
+		    ch.cs.p, ch.cs_off.p, ch.cs_mid.p, ctx->hot_pix.p, n, pitch, ch.nc, ch.k_pitch, ch.by_frame.p,
+		    ch.by_pixel.p);
+		CKL("hot_counts_kernel");
+		if (int rc = encode_byte_map(ctx, &ch.map_frame, ch.by_frame.p, ch.nc, pitch))
+			return rc;
+		if (int rc = encode_byte_map(ctx, &ch.map_pixel, ch.by_pixel.p, n, ch.k_pitch))
+			return rc;
+		std::vector<int> pix((size_t)ch.npix), rest;
+		if (ch.npix > 0)
+			CK(cudaMemcpyAsync(pix.data(), ch.pix.p, pix.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+		CK(cudaStreamSynchronize(st));
+		for (int p : pix)
+			if (!is_hot[p])
+				rest.push_back(p);
+		ch.npix_cold = (int)rest.size();
+		CK(upload(ch.pix_cold, rest.data(), rest.size(), st));
+		CK(cudaStreamSynchronize(st));
+	}
+	// the E-step's lists without the hot pixels
+	DevBuf<int2> cnt;
+	std::vector<int2> h((size_t)N);
+	std::vector<long long> off((size_t)N + 1, 0), mid((size_t)N);
+	if (room) {
+		CK(cnt.ensure((size_t)N));
+		cold_count_kernel<<<blocks_for((long long)N * 32, 256), 256, 0, st>>>(ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p,
+		                                                                      N, P, ctx->is_hot.p, cnt.p);
+		CKL("cold_count_kernel");
+		CK(cudaMemcpyAsync(h.data(), cnt.p, (size_t)N * sizeof(int2), cudaMemcpyDeviceToHost, st));
+		CK(cudaStreamSynchronize(st));
+		for (int d = 0; d < N; ++d) {
+			mid[d] = off[d] + (h[d].x + 7) / 8 * 8;
+			off[d + 1] = mid[d] + (h[d].y + 7) / 8 * 8;
+		}
+		const cudaError_t e = fits(ctx->phc.ensure((size_t)off[N]));
+		if (e != cudaErrorMemoryAllocation)
+			CK(e);
+		else
+			room = false;
+	}
+	if (!room) {
+		for (Chunk &ch : ctx->chunks) {
+			ch.by_frame.release();
+			ch.by_pixel.release();
+			ch.pix_cold.release();
+		}
+		return DFG_OK;
+	}
+	CK(upload(ctx->phc_off, off.data(), off.size(), st));
+	CK(upload(ctx->phc_mid, mid.data(), mid.size(), st));
+	cold_write_kernel<<<blocks_for((long long)N * 32, 256), 256, 0, st>>>(ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p, N,
+	                                                                      P, ctx->is_hot.p, ctx->phc_off.p,
+	                                                                      ctx->phc_mid.p, ctx->phc.p);
+	CKL("cold_write_kernel");
+	CK(cudaStreamSynchronize(st));
+	ctx->hot_n = n;
+	ctx->hot_pitch = pitch;
+	return DFG_OK;
+}
+
+// The products' buffers for this iteration: the log-slices' digits, and the
+// probabilities' digits over the chunk's log-likelihoods (dead by the M-step;
+// half their size).
+static int hot_prepare(dfg_ctx *ctx) {
+	if (ctx->hot_layout != ctx->layout)
+		if (int rc = hot_choose(ctx))
+			return rc;
+	if (ctx->hot_n == 0)
+		return DFG_OK;
+	const long long rows = (long long)ctx->RT * 2 * 4 * HO;
+	const cudaError_t e = ctx->wdig.ensure((size_t)rows * ctx->hot_pitch);
+	if (e == cudaErrorMemoryAllocation) {
+		cudaGetLastError();
+		ctx->hot_n = 0;
+		return DFG_OK;
+	}
+	CK(e);
+	CK(ctx->hot_special.ensure((size_t)ctx->RT));
+	CK(ctx->rowmax.ensure((size_t)ctx->R_pad));
+	CK(ctx->rowmax_part.ensure((size_t)psum_splits(ctx) * ctx->R_pad));
+	CK(ctx->derr.ensure(1));
+	CK(cudaMemsetAsync(ctx->derr.p, 0, sizeof(int), ctx->stream));
+	if (int rc = encode_byte_map(ctx, &ctx->map_wdig, ctx->wdig.p, rows, ctx->hot_pitch))
+		return rc;
+	for (Chunk &ch : ctx->chunks)
+		if (int rc = encode_byte_map(ctx, &ch.map_pdig, ctx->pval.p, rows, ch.k_pitch))
+			return rc;
+	CK(cudaFuncSetAttribute(hot_product_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, HSMEM_BYTES));
+	CK(cudaFuncSetAttribute(hot_product_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HSMEM_BYTES));
+	ctx->hot_active = true;
+	return DFG_OK;
+}
+
+static unsigned hot_grid(const dfg_ctx *ctx, long long tiles) {
+	return (unsigned)std::min<long long>(tiles, ctx->num_sms);
+}
+
+// The log-slices' digits (once per iteration, after the slices).
+static int launch_hot_digits(dfg_ctx *ctx) {
+	cudaStream_t st = ctx->stream;
+	CK(cudaMemsetAsync(ctx->hot_special.p, 0, (size_t)ctx->RT * sizeof(int), st));
+	hot_digits_kernel<false><<<dim3(ctx->hot_pitch / HK, ctx->RT * 2), 256, 0, st>>>(
+	    ctx->logW.p, (size_t)(ctx->P + 1) * TILE, ctx->hot_pix.p, ctx->hot_n, ctx->hot_pitch, nullptr, ctx->wdig.p,
+	    ctx->hot_special.p);
+	CKL("hot_digits_kernel");
+	return DFG_OK;
+}
+
+static int launch_hot_estep(dfg_ctx *ctx, const Chunk &ch) {
+	const int OT = ctx->RT * 2, FT = (ch.nc + HM - 1) / HM;
+	hot_product_kernel<false><<<hot_grid(ctx, (long long)OT * FT), HTHREADS, HSMEM_BYTES, ctx->stream>>>(
+	    ch.map_frame, ctx->map_wdig, ctx->hot_pitch / HK, OT, FT, ch.nc, HotOut{ctx->pval.p, nullptr, nullptr, nullptr, 0, 0},
+	    ctx->derr.p, ctx->dense_wait_cycles, ctx->dense_withhold);
+	CKL("hot_product_kernel");
+	return DFG_OK;
+}
+
+static int launch_hot_mstep(dfg_ctx *ctx, const Chunk &ch) {
+	cudaStream_t st = ctx->stream;
+	int8_t *dig = reinterpret_cast<int8_t *>(ctx->pval.p);
+	hot_digits_kernel<true><<<dim3(ch.k_pitch / HK, ctx->RT * 2), 256, 0, st>>>(
+	    ctx->Pst.p, (size_t)(ch.nc + 1) * TILE, nullptr, ch.nc, ch.k_pitch, ctx->rowmax.p, dig, nullptr);
+	CKL("hot_digits_kernel");
+	const int OT = ctx->RT * 2, FT = (ctx->hot_n + HM - 1) / HM;
+	hot_product_kernel<true><<<hot_grid(ctx, (long long)OT * FT), HTHREADS, HSMEM_BYTES, st>>>(
+	    ch.map_pixel, ch.map_pdig, ch.k_pitch / HK, OT, FT, ctx->hot_n,
+	    HotOut{nullptr, ctx->T.p, ctx->hot_pix.p, ctx->rowmax.p, ctx->P, ch.d0 == 0 ? 1 : 0}, ctx->derr.p,
+	    ctx->dense_wait_cycles, ctx->dense_withhold);
+	CKL("hot_product_kernel");
+	return DFG_OK;
+}
+
 static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par);
 static bool pair_mode(const dfg_ctx *ctx);
 static int ensure_pair_buffers(dfg_ctx *ctx, const dfg_iter_params *par);
@@ -1223,6 +1456,7 @@ static int max_prepare(dfg_ctx *ctx, const dfg_iter_params *par) {
 		return DFG_ERR_ARG;
 	NEED(par->beta_period > 0, DFG_ERR_ARG, "beta_period must be > 0");
 	CK(cudaSetDevice(ctx->device));
+	ctx->hot_active = false;
 	if (pair_mode(ctx))
 		return pair_prepare(ctx, par);
 	if (blocked_wanted(ctx))
@@ -1251,6 +1485,11 @@ static int max_prepare(dfg_ctx *ctx, const dfg_iter_params *par) {
 		return rc;
 	if (ctx->dense_active || ctx->m_dense_active)
 		if (int rc = dense_prepare_counts(ctx))
+			return rc;
+	// the plain search's sparse forms leave the hot pixels to the products
+	if (!ctx->refine && !ctx->mstep_skip && !(ctx->with_bg && par->need_scaling) &&
+	    (ctx->tuning || !(ctx->dense_active && ctx->m_dense_active)))
+		if (int rc = hot_prepare(ctx))
 			return rc;
 	cudaStream_t st = ctx->stream;
 	if (ctx->refine && !ctx->h_watch.empty()) {  // chunk-local indices of the watched frames
@@ -1376,13 +1615,19 @@ static int launch_mstep(dfg_ctx *ctx, const Chunk &ch, bool dense) {
 		CKL("mstep_dense_kernel");
 		return DFG_OK;
 	}
-	if (ch.npix > 0) {
-		const long long warps = (long long)RT * ch.npix;
+	const bool hot = ctx->hot_active;
+	if (hot)
+		if (int rc = launch_hot_mstep(ctx, ch))
+			return rc;
+	const int npix = hot ? ch.npix_cold : ch.npix;
+	const int *pix = hot ? ch.pix_cold.p : ch.pix.p;
+	if (npix > 0) {
+		const long long warps = (long long)RT * npix;
 		const int minb = ctx->tuning ? ctx->tune_mstep_minb
 		                             : (ctx->mstep_minb > 0 ? ctx->mstep_minb : ctx->tuned_mstep_minb);
 #define DFG_MSTEP(SK, MB)                                                                                     \
 	mstep_kernel<SK, MB><<<blocks_for(warps, 8), 256, 0, st>>>(ctx->Pst.p, Nc, ch.cs.p, ch.cs_off.p,           \
-	                                                           ch.cs_mid.p, ch.pix.p, ch.npix, P, RT, ctx->T.p,  \
+	                                                           ch.cs_mid.p, pix, npix, P, RT, ctx->T.p,          \
 	                                                           ctx->tlive.p)
 		if (tile_skipping(ctx))
 			DFG_MSTEP(true, MSTEP_MINB);
@@ -1422,18 +1667,31 @@ static int launch_estep(dfg_ctx *ctx, const Chunk &ch, int use_scale, bool bg, c
 	// blocks per SM: the autotuner's choice (or the option), else the default
 	const int minb = ctx->tuning ? ctx->tune_estep_minb : (ctx->estep_minb > 0 ? ctx->estep_minb
 	                                                                           : ctx->tuned_estep_minb);
-#define DFG_ESTEP(REF, MB)                                                                                    \
-	estep_kernel<REF, MB><<<blocks_for(warps, 8), 256, 0, st>>>(                                              \
-	    ctx->logW.p, ctx->u.p, ctx->logw.p, R, ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p, ctx->scale.p,          \
-	    ctx->blacklist.p, ch.d0, Nc, use_scale, ctx->scalars.p, P, RT, ctx->pval.p, ctx->tmax.p, ctx->targ.p, rm)
+	const bool hot = ctx->hot_active && rm.qmap == nullptr;
+	const uint32_t *ph = hot ? ctx->phc.p : ctx->ph.p;
+	const long long *off = hot ? ctx->phc_off.p : ctx->ph_off.p, *mid = hot ? ctx->phc_mid.p : ctx->ph_mid.p;
+	const HotLists full{ctx->hot_special.p, ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p};
+	if (hot)
+		if (int rc = launch_hot_estep(ctx, ch))
+			return rc;
+#define DFG_ESTEP(REF, MB, HOT)                                                                               \
+	estep_kernel<REF, MB, HOT><<<blocks_for(warps, 8), 256, 0, st>>>(                                         \
+	    ctx->logW.p, ctx->u.p, ctx->logw.p, R, ph, off, mid, ctx->scale.p, ctx->blacklist.p, ch.d0, Nc,        \
+	    use_scale, ctx->scalars.p, P, RT, ctx->pval.p, ctx->tmax.p, ctx->targ.p, rm, 0, full)
 	if (rm.qmap != nullptr)
-		DFG_ESTEP(true, ESTEP_MINB);
+		DFG_ESTEP(true, ESTEP_MINB, false);
+	else if (hot && minb == 2)
+		DFG_ESTEP(false, 2, true);
+	else if (hot && minb == 4)
+		DFG_ESTEP(false, 4, true);
+	else if (hot)
+		DFG_ESTEP(false, ESTEP_MINB, true);
 	else if (minb == 2)
-		DFG_ESTEP(false, 2);
+		DFG_ESTEP(false, 2, false);
 	else if (minb == 4)
-		DFG_ESTEP(false, 4);
+		DFG_ESTEP(false, 4, false);
 	else
-		DFG_ESTEP(false, ESTEP_MINB);
+		DFG_ESTEP(false, ESTEP_MINB, false);
 #undef DFG_ESTEP
 	CKL("estep_kernel");
 	return DFG_OK;
@@ -1469,6 +1727,22 @@ static int launch_norm(dfg_ctx *ctx, const Chunk &ch, int psum_d_on, bool bg) {
 	}
 #undef DFG_NORM
 	CKL("norm_kernel");
+	return DFG_OK;
+}
+
+// psum_r of one chunk (calc_psum_r, max_update.c:108-116), added to psum_r, and
+// each orientation's largest probability for the hot pixels' products.
+static int launch_psum(dfg_ctx *ctx, const Chunk &ch, int need_scaling) {
+	cudaStream_t st = ctx->stream;
+	const int nsplit = psum_splits(ctx), fps = (ch.nc + nsplit - 1) / nsplit;
+	float *const part_max = ctx->hot_active ? ctx->rowmax_part.p : nullptr;
+	psum_r_kernel<<<dim3(ctx->RT, nsplit), 256, 0, st>>>(ctx->Pst.p, ch.nc, ch.d0, fps, ctx->scale.p, need_scaling,
+	                                                     ctx->psum_part.p, ctx->R_pad,
+	                                                     tile_skipping(ctx) ? ctx->tlive.p : nullptr, part_max);
+	CKL("psum_r_kernel");
+	psum_r_reduce_kernel<<<blocks_for(ctx->R_pad, 256), 256, 0, st>>>(ctx->psum_part.p, nsplit, ctx->R, ctx->R_pad,
+	                                                                  ctx->psum_r.p, part_max, ctx->rowmax.p);
+	CKL("psum_r_reduce_kernel");
 	return DFG_OK;
 }
 
@@ -1927,8 +2201,7 @@ static int blocked_prepare(dfg_ctx *ctx, const dfg_iter_params *par) {
 	CK(ctx->tmax.ensure((size_t)ctx->RT * ctx->chunk_frames));
 	CK(ctx->targ.ensure((size_t)ctx->RT * ctx->chunk_frames));
 	CK(ctx->tlive.ensure((size_t)ctx->RT * (ctx->chunk_frames + 1)));
-	const int nsplit = std::max(1, std::min(64, ctx->chunk_frames / 2048));
-	CK(ctx->psum_part.ensure((size_t)nsplit * ctx->R_pad));
+	CK(ctx->psum_part.ensure((size_t)psum_splits(ctx) * ctx->R_pad));
 	return prepare_weight_cache(ctx);
 }
 
@@ -1986,7 +2259,6 @@ static int max_enqueue_blocked(dfg_ctx *ctx, const dfg_iter_params *par) {
 	ctx->have_prob = false;
 	// pass 1
 	for (Chunk &ch : ctx->chunks) {
-		const int Nc = ch.nc;
 		for (int t0 = 0; t0 < RT; t0 += BT) {
 			const int nt = std::min(BT, RT - t0);
 			phase_begin(ctx, PH_SLICE);
@@ -2006,14 +2278,8 @@ static int max_enqueue_blocked(dfg_ctx *ctx, const dfg_iter_params *par) {
 			if (int rc = collect_prob(ctx, ch))
 				return rc;
 		phase_begin(ctx, PH_PSUM);
-		const int nsplit = std::max(1, std::min(64, ctx->chunk_frames / 2048));
-		const int fps = (Nc + nsplit - 1) / nsplit;
-		psum_r_kernel<<<dim3(RT, nsplit), 256, 0, st>>>(ctx->Pst.p, Nc, ch.d0, fps, ctx->scale.p, par->need_scaling,
-		                                                ctx->psum_part.p, R_pad,
-		                                                tile_skipping(ctx) ? ctx->tlive.p : nullptr);
-		CKL("psum_r_kernel");
-		psum_r_reduce_kernel<<<blocks_for(R, 256), 256, 0, st>>>(ctx->psum_part.p, nsplit, R, R_pad, ctx->psum_r.p);
-		CKL("psum_r_reduce_kernel");
+		if (int rc = launch_psum(ctx, ch, par->need_scaling))
+			return rc;
 		phase_end(ctx, PH_PSUM, 2);
 	}
 	weight_pattern_kernel<<<1, 1024, 0, st>>>(ctx->psum_r.p, R, ctx->wpattern.p, ctx->wflags.p);
@@ -2113,7 +2379,10 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 		    (__nv_bfloat16 *)ctx->Alo.p);
 		CKL("split_logw_kernel");
 	}
-	phase_end(ctx, PH_SLICE, ctx->dense_active ? 4 : 3);
+	if (ctx->hot_active)
+		if (int rc = launch_hot_digits(ctx))
+			return rc;
+	phase_end(ctx, PH_SLICE, 3 + (ctx->dense_active ? 1 : 0) + (ctx->hot_active ? 1 : 0));
 
 	CK(cudaMemsetAsync(ctx->T.p, 0, (size_t)RT * P * TILE * sizeof(float), st));
 	CK(cudaMemsetAsync(ctx->psum_r.p, 0, (size_t)R_pad * sizeof(double), st));
@@ -2151,16 +2420,10 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 		// psum_r (calc_psum_r, max_update.c:108-116)
 		phase_begin(ctx, PH_PSUM);
 		{
-			const int nsplit = std::max(1, std::min(64, ctx->chunk_frames / 2048));
-			const int fps = (Nc + nsplit - 1) / nsplit;
-			psum_r_kernel<<<dim3(RT, nsplit), 256, 0, st>>>(ctx->Pst.p, Nc, ch.d0, fps, ctx->scale.p,
-			                                                par->need_scaling, ctx->psum_part.p, R_pad,
-			                                                tile_skipping(ctx) ? ctx->tlive.p : nullptr);
-			CKL("psum_r_kernel");
-			psum_r_reduce_kernel<<<blocks_for(R, 256), 256, 0, st>>>(ctx->psum_part.p, nsplit, R, R_pad,
-			                                                          ctx->psum_r.p);
-			CKL("psum_r_reduce_kernel");
+			if (int rc = launch_psum(ctx, ch, par->need_scaling))
+				return rc;
 			if (bg) {
+				const int nsplit = psum_splits(ctx), fps = (Nc + nsplit - 1) / nsplit;
 				scalemax_kernel<<<dim3(RT, nsplit), 256, 0, st>>>(ctx->Pd.p, Nc, ch.d0, fps, ctx->scale.p,
 				                                                  ctx->smax_part.p, R_pad);
 				CKL("scalemax_kernel");
@@ -2295,8 +2558,11 @@ static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par) {
 		CKL("rescale_kernel");
 		logw_kernel<<<blocks_for(ctx->R, 256), 256, 0, st>>>(ctx->quats.p, ctx->M, ctx->R, ctx->logw.p);
 		CKL("logw_kernel");
-		rc = timed([&] { return launch_estep(ctx, ctx->chunks[0], use_scale, bg, rm, false); }, rep[4]);
+		if (ctx->hot_active)
+			rc = launch_hot_digits(ctx);
 	}
+	if (rc == DFG_OK)
+		rc = timed([&] { return launch_estep(ctx, ctx->chunks[0], use_scale, bg, rm, false); }, rep[4]);
 	const Chunk &c0 = ctx->chunks[0];
 	if (rc == DFG_OK && dense_ok) {
 		split_logw_kernel<<<dim3(ctx->K_pad / DK, ctx->RT), 256, 0, st>>>(
@@ -2317,6 +2583,8 @@ static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par) {
 	const int psum_d_on = par->need_scaling && par->update_scale;
 	if (rc == DFG_OK)
 		rc = launch_norm(ctx, c0, psum_d_on, bg);
+	if (rc == DFG_OK && ctx->hot_active)
+		rc = launch_psum(ctx, c0, par->need_scaling);
 	if (rc == DFG_OK && !bg)
 		rc = timed([&] { return launch_mstep(ctx, c0, false); }, rep[8]);
 	if (rc == DFG_OK && dense_ok)
@@ -2351,11 +2619,11 @@ static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par) {
 				m_minb = cand[i];
 		ctx->tune_mstep_minb = MSTEP_MINB;
 	}
-	if (rc == DFG_OK && dense_ok) {
+	if (rc == DFG_OK && (dense_ok || ctx->hot_active)) {
 		int derr = 0;
 		CK(cudaMemcpy(&derr, ctx->derr.p, sizeof(int), cudaMemcpyDeviceToHost));
 		if (derr)
-			rc = ctx->fail(DFG_ERR_CUDA, "autotune: a dense kernel gave up");
+			rc = ctx->fail(DFG_ERR_CUDA, "autotune: a product kernel gave up");
 	}
 	if (e0)
 		cudaEventDestroy(e0);
@@ -2417,11 +2685,11 @@ extern "C" int dfg_maximize(dfg_ctx *ctx, const dfg_iter_params *par, double *av
 	double h[3];
 	int derr = 0;
 	CK(cudaMemcpyAsync(h, ctx->scalars.p, 3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-	if (ctx->dense_active || ctx->m_dense_active)
+	if (ctx->dense_active || ctx->m_dense_active || ctx->hot_active)
 		CK(cudaMemcpyAsync(&derr, ctx->derr.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
 	CK(cudaStreamSynchronize(ctx->stream));
 	phase_collect(ctx);
-	NEED(derr == 0, DFG_ERR_CUDA, "dense E-step / M-step: a pipeline wait gave up (results invalid)");
+	NEED(derr == 0, DFG_ERR_CUDA, "E-step / M-step products: a pipeline wait gave up (results invalid)");
 	max_finish(ctx, h);
 	if (avg_likelihood)
 		*avg_likelihood = ctx->avg_ll;
@@ -2800,11 +3068,11 @@ static int iteration_finish(dfg_ctx *ctx, const dfg_iter_params *par, double *ou
 	double h[6];
 	int derr = 0;
 	CK(cudaMemcpyAsync(h, ctx->scalars.p, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
-	if (ctx->dense_active || ctx->m_dense_active)
+	if (ctx->dense_active || ctx->m_dense_active || ctx->hot_active)
 		CK(cudaMemcpyAsync(&derr, ctx->derr.p, sizeof(int), cudaMemcpyDeviceToHost, st));
 	CK(cudaStreamSynchronize(st));
 	phase_collect(ctx);
-	NEED(derr == 0, DFG_ERR_CUDA, "dense E-step / M-step: a pipeline wait gave up (results invalid)");
+	NEED(derr == 0, DFG_ERR_CUDA, "E-step / M-step products: a pipeline wait gave up (results invalid)");
 	max_finish(ctx, h);
 	ctx->rms = std::sqrt(h[3] / ctx->M / (double)ctx->V);
 	double mean = 1.;
@@ -3161,11 +3429,11 @@ extern "C" int dfg_group_maximize(dfg_group *g, const dfg_iter_params *par, doub
 		dfg_ctx *c = g->m[k];
 		int derr = 0;
 		GCK(cudaMemcpyAsync(&h[3 * k], c->scalars.p, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-		if (c->dense_active || c->m_dense_active)
+		if (c->dense_active || c->m_dense_active || c->hot_active)
 			GCK(cudaMemcpyAsync(&derr, c->derr.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
 		GCK(cudaStreamSynchronize(c->stream));
 		phase_collect(c);
-		GNEED(derr == 0, DFG_ERR_CUDA, "detector %d: dense E-step / M-step: a pipeline wait gave up", (int)k);
+		GNEED(derr == 0, DFG_ERR_CUDA, "detector %d: E-step / M-step products: a pipeline wait gave up", (int)k);
 		max_finish(c, &h[3 * k]);
 		sum_mi += h[3 * k + 1];
 		sum_ll += h[3 * k + 2];

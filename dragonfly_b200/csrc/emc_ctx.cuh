@@ -96,6 +96,13 @@ struct Chunk {
 	DevBuf<int> pix;           // pixels with non-empty lists, longest first
 	int npix = 0;
 	long long entries = 0;
+	// hot pixels (emc_hot.cuh): counts as bytes [nc][hot_pitch] and
+	// [hot_n][k_pitch] (k_pitch = nc rounded up to 128), their tensor maps and
+	// that of the chunk's probability digits, and the pixels left to the gathers
+	DevBuf<uint8_t> by_frame, by_pixel;
+	DevBuf<int> pix_cold;
+	int npix_cold = 0, k_pitch = 0;
+	CUtensorMap map_frame, map_pixel, map_pdig;
 };
 
 }  // namespace dfg
@@ -220,6 +227,24 @@ struct dfg_ctx {
 	int K = 0, K_pad = 0, dense_P = -1, cnt_rows = 0;
 	int max_count0 = -1;  // largest count on a mask < 2 pixel; -1 = not known
 	DevBuf<int> kpix, pcol, derr;
+	// hot pixels: the pixels (mask 0) that enough frames share for the integer
+	// products of emc_hot.cuh. hot_n of them (hot_pix), hot_pitch = hot_n rounded
+	// up to 128; the E-step's photon lists without them (phc ...); the
+	// log-slices' digits; per tile whether its log-slices do not fit the digits;
+	// each orientation's largest probability in the chunk. layout counts the
+	// chunk layouts built, hot_layout is the one the hot set was made for
+	int hot_n = 0, hot_pitch = 0, layout = 0, hot_layout = -1;
+	bool hot_active = false;   // this iteration's plain path takes the products
+	std::vector<long long> h_pix_entries;  // [P] photon words over all chunks
+	std::vector<uint8_t> h_pix_big;        // [P] counts that the byte products cannot hold
+	DevBuf<int> hot_pix, hot_special;
+	DevBuf<uint8_t> is_hot;
+	DevBuf<uint32_t> phc;
+	DevBuf<long long> phc_off, phc_mid;
+	DevBuf<int8_t> wdig;
+	DevBuf<float> rowmax, rowmax_part;
+	CUtensorMap map_wdig;
+	int max_fcount = 0;        // most photons of a frame
 	// failure-detection test hooks of the dense kernels: the clock cycles
 	// after which a pipeline wait gives up, and a stage whose copies are never
 	// issued (-1: none)

@@ -276,13 +276,22 @@ __device__ __forceinline__ void refine_skip_tile(double *__restrict__ tmax, int 
 	}
 }
 
-template <bool REFINE, int MINB = ESTEP_MINB>
+// HOT: the photons of the hot pixels are already in pval as FP64 sums
+// (emc_hot.cuh), the lists hold the others; a tile marked special gathers all of
+// its photons (full) instead.
+struct HotLists {
+	const int *special;          // [RT]
+	const uint32_t *ph;          // every photon's lists
+	const long long *off, *mid;
+};
+
+template <bool REFINE, int MINB = ESTEP_MINB, bool HOT = false>
 __global__ void __launch_bounds__(256, MINB) estep_kernel(
     const float *__restrict__ logW, const double *__restrict__ u, const double *__restrict__ logw, int R,
     const uint32_t *__restrict__ ph, const long long *__restrict__ ph_off, const long long *__restrict__ ph_mid,
     const double *__restrict__ scale, const uint8_t *__restrict__ blacklist, int d0, int Nc, int use_scale,
     const double *__restrict__ scalars, int P, int RT, double *__restrict__ pval, double *__restrict__ tmax,
-    int *__restrict__ targ, RefineMask rm, int t0 = 0) {
+    int *__restrict__ targ, RefineMask rm, int t0 = 0, HotLists full = {}) {
 	// RT tiles from tile t0 (orientation blocks: logW holds tiles t0 ..)
 	const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const int lane = threadIdx.x & 31;
@@ -301,6 +310,15 @@ __global__ void __launch_bounds__(256, MINB) estep_kernel(
 		}
 	}
 	const float *L = logW + (size_t)rl * (P + 1) * TILE + lane * LW;
+	bool add_hot = HOT;
+	if constexpr (HOT) {
+		if (full.special[rt]) {
+			ph = full.ph;
+			ph_off = full.off;
+			ph_mid = full.mid;
+			add_hot = false;
+		}
+	}
 	const long long beg = ph_off[d], mid = ph_mid[d], end = ph_off[d + 1];
 	// segments start at multiples of 8 words: two 16-byte loads, identical for
 	// every lane (broadcast), bring 8 photon words
@@ -351,7 +369,13 @@ __global__ void __launch_bounds__(256, MINB) estep_kernel(
 				kahan_add_count(s[q % ECH][k], c[q % ECH][k], e[q] >> IDX_BITS, v[q][k]);
 	}
 	const double sd = use_scale ? scale[d] : scalars[0];
-	double acc[LW];
+	double acc[LW], hot[LW];
+	if constexpr (HOT) {
+		const double *h = pval + ((size_t)rt * Nc + dl) * TILE + lane * LW;
+#pragma unroll
+		for (int k = 0; k < LW; ++k)
+			hot[k] = add_hot ? h[k] : 0.;
+	}
 	// tile maximum and its lowest orientation index (strict > in ascending r,
 	// as the running maximum of max_prob.c:199-202)
 	double m = MAX_EXP_START;
@@ -364,6 +388,8 @@ __global__ void __launch_bounds__(256, MINB) estep_kernel(
 			double ph_sum = kahan_value(s[0][k], c[0][k]);
 			if (ECH == 2)
 				ph_sum = dadd(ph_sum, kahan_value(s[ECH - 1][k], c[ECH - 1][k]));
+			if (HOT)
+				ph_sum = dadd(ph_sum, hot[k]);
 			acc[k] = dadd(dsub(logw[r], dmul(u[r], sd)), ph_sum);
 			if (REFINE && !(live >> k & 1u))
 				acc[k] = -INFINITY;
@@ -848,17 +874,24 @@ __global__ void __launch_bounds__(256, DFG_NORM_MINB) norm_kernel(
 
 // psum_r partials: sum over a frame range of |Pst| * (phi_d or 1)
 // (max_update.c:108-116). Grid (RT, splits), 8 warps per block; fixed order.
+// part_max (may be null): the largest Pst of each orientation in the range, the
+// unit of the M-step's fixed-point products (emc_hot.cuh).
 __global__ void __launch_bounds__(256) psum_r_kernel(const float *__restrict__ Pst, int Nc, int d0,
                                                       int frames_per_split, const double *__restrict__ scale,
                                                       int need_scaling, double *__restrict__ part, int R_pad,
-                                                      const uint8_t *__restrict__ tlive) {
+                                                      const uint8_t *__restrict__ tlive,
+                                                      float *__restrict__ part_max) {
 	__shared__ double s[8][TILE];
+	__shared__ float s_m[8][TILE];
 	const int rt = blockIdx.x, split = blockIdx.y, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	const int beg = split * frames_per_split, end = min(Nc, beg + frames_per_split);
 	double acc[LW];
+	float top[LW];
 #pragma unroll
-	for (int k = 0; k < LW; ++k)
+	for (int k = 0; k < LW; ++k) {
 		acc[k] = 0.;
+		top[k] = 0.f;
+	}
 	const float *p = Pst + (size_t)rt * (Nc + 1) * TILE + lane * LW;
 	const uint8_t *live = tlive ? tlive + (size_t)rt * (Nc + 1) : nullptr;
 	for (int dl = beg + w; dl < end; dl += 8) {
@@ -868,25 +901,41 @@ __global__ void __launch_bounds__(256) psum_r_kernel(const float *__restrict__ P
 		ld_row(p + (size_t)dl * TILE, v);
 		const double f = need_scaling ? scale[d0 + dl] : 1.;
 #pragma unroll
-		for (int k = 0; k < LW; ++k)
+		for (int k = 0; k < LW; ++k) {
 			acc[k] += need_scaling ? fabs((double)v[k]) * f : fabs((double)v[k]);
+			top[k] = fmaxf(top[k], v[k]);
+		}
 	}
 #pragma unroll
-	for (int k = 0; k < LW; ++k)
+	for (int k = 0; k < LW; ++k) {
 		s[w][lane * LW + k] = acc[k];
+		s_m[w][lane * LW + k] = top[k];
+	}
 	__syncthreads();
 	for (int j = threadIdx.x; j < TILE; j += blockDim.x) {
 		double t = 0.;
+		float m = 0.f;
 #pragma unroll
-		for (int k = 0; k < 8; ++k)
+		for (int k = 0; k < 8; ++k) {
 			t += s[k][j];
+			m = fmaxf(m, s_m[k][j]);
+		}
 		part[(size_t)split * R_pad + rt * TILE + j] = t;
+		if (part_max != nullptr)
+			part_max[(size_t)split * R_pad + rt * TILE + j] = m;
 	}
 }
 
 __global__ void psum_r_reduce_kernel(const double *__restrict__ part, int nsplit, int R, int R_pad,
-                                     double *__restrict__ psum_r) {
+                                     double *__restrict__ psum_r, const float *__restrict__ part_max,
+                                     float *__restrict__ rowmax) {
 	int r = blockIdx.x * blockDim.x + threadIdx.x;
+	if (part_max != nullptr && r < R_pad) {
+		float m = 0.f;
+		for (int k = 0; k < nsplit; ++k)
+			m = fmaxf(m, part_max[(size_t)k * R_pad + r]);
+		rowmax[r] = m;
+	}
 	if (r >= R)
 		return;
 	double s = 0.;

@@ -1,0 +1,85 @@
+"""The hot pixels' integer products (csrc/emc_hot.cuh) against the FP64 oracle
+and against the gathers alone, at the edges of their tiles.
+
+The plain search leaves the pixels that many frames share to the products;
+option tile_skip keeps every photon in the gathers. Both add the same FP32
+log-slices (|log W| < 40 here); the gathers' compensated sums round each added
+value to 2^-24 of it, the products add exactly.
+"""
+import numpy as np
+import pytest
+
+from common import GPUEngine, compare_iteration
+from oracle.oracle import EMCProblem, OracleEngine
+from dragonfly_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(frames, div, side, photons, zeros=False, big=False):
+    d = synth.small_problem(seed=frames + div, det_side=side, size=side + 3, qmax=side / 2., n_atoms=60,
+                            atom_radius=4., num_div=div, n_frames=frames, mean_count=photons, hole_radius=2.)
+    model = d["model_start"] * photons / (d["mask"] == 0).sum() * 2.
+    if zeros:   # log 0 inside the detector: some tiles gather all of their photons
+        c = model.shape[1] // 2
+        model[:, c + 5:c + 8, c:c + 3, c:c + 3] = 0.
+    count = d["count_multi"].copy()
+    if big:     # counts past a byte keep their pixels out of the products
+        count[::97] = 300
+        count[5] = 1200
+    return EMCProblem(d["qvals"], d["corr"], d["mask"], d["ones"], d["multi"], d["place_ones"], d["place_multi"],
+                      count, d["quats"], model, need_scaling=1, update_scale=1, beta=0.1)
+
+
+def _photons(prob):
+    n = prob.ones.astype(np.int64).copy()
+    np.add.at(n, np.repeat(np.arange(prob.num_data), prob.multi), prob.count_multi)
+    return n
+
+
+@pytest.mark.parametrize("frames,div,side,photons,zeros,big,budget", [
+    (256, 1, 24, 150., False, False, 0.),    # one row tile exactly, under half an orientation tile
+    (257, 2, 24, 200., False, False, 0.),    # one frame past it
+    (300, 2, 40, 100., False, False, 0.),    # some pixels left to the gathers
+    (800, 2, 24, 120., False, False, 2.0),   # chunks of 267 frames: tomograms added over three
+    (511, 1, 24, 200., True, False, 0.),     # tiles with log 0
+    (400, 2, 24, 250., False, True, 0.),     # counts past a byte
+])
+def test_products_match_oracle_and_gathers(oracle_built, frames, div, side, photons, zeros, big, budget):
+    prob = _problem(frames, div, side, photons, zeros, big)
+    hot = GPUEngine(prob, pair_budget_mb=budget)
+    plain = GPUEngine(prob, pair_budget_mb=budget, tile_skip=1)
+    orc = OracleEngine(prob)
+    a, b, c = hot.run_iteration(1), orc.run_iteration(1), plain.run_iteration(1)
+    assert hot.ctx.workload()["launches"] > plain.ctx.workload()["launches"]   # the products ran
+    if budget:
+        assert hot.ctx.workload()["chunks"] == 3
+    compare_iteration(a, b, prob, 1, model_before=prob.model1)
+    np.testing.assert_array_equal(a["rmax"], c["rmax"])
+    assert np.all(np.abs(a["likelihood"] - c["likelihood"]) <= 2. ** -24 * 40. * _photons(prob))
+    model_before, scale_before = orc.model1(), orc.scale.copy()
+    compare_iteration(hot.run_iteration(2), orc.run_iteration(2), prob, 2, model_before=model_before,
+                      scale_before=scale_before)
+    hot.close()
+    plain.close()
+
+
+def test_product_wait_gives_up_and_the_context_recovers(oracle_built):
+    """A stage whose copies are withheld (test hook): its waits run out, the
+    kernels return, the call reports the error, and the next call succeeds."""
+    from dragonfly_b200._lib import DFG_ERR_CUDA, DFGError
+    prob = _problem(257, 2, 24, 200.)
+    gpu = GPUEngine(prob)
+    c = gpu.ctx
+    par = c.params(1, 1, 1, 0, 1., 100, 1.)
+    c.set_option("dense_wait_cycles", 2e7)
+    c.set_option("dense_withhold_stage", 1)
+    with pytest.raises(DFGError) as e:
+        c.maximize(par)
+    assert e.value.code == DFG_ERR_CUDA and "gave up" in str(e.value)
+    c.set_option("dense_withhold_stage", -1)
+    c.set_option("dense_wait_cycles", 2e9)
+    c.set_scale(np.ones(prob.num_data))   # the failed call's scale update is invalid with its other results
+    a = gpu.run_iteration(1)
+    compare_iteration(a, OracleEngine(prob).run_iteration(1), prob, 1, model_before=prob.model1)
+    gpu.close()
