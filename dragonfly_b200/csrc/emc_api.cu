@@ -788,6 +788,31 @@ static int build_chunks(dfg_ctx *ctx) {
 	return DFG_OK;
 }
 
+// The corner quads take four times the model; past kQuadMaxBytes (or without
+// the memory) the slices gather voxels instead.
+constexpr size_t kQuadMaxBytes = (size_t)8 << 30;
+
+static int ensure_quads(dfg_ctx *ctx) {
+	const size_t n = (size_t)ctx->M * ctx->V;
+	ctx->use_quads = n * sizeof(double4) <= kQuadMaxBytes;
+	if (!ctx->use_quads) {
+		ctx->quads.release();
+		return DFG_OK;
+	}
+	const cudaError_t e = ctx->quads.ensure(n);
+	if (e == cudaErrorMemoryAllocation) {
+		cudaGetLastError();
+		ctx->use_quads = false;
+		return DFG_OK;
+	}
+	CK(e);
+	return DFG_OK;
+}
+
+static SliceModel slice_model(const dfg_ctx *ctx) {
+	return SliceModel{ctx->use_quads ? ctx->quads.p : nullptr, ctx->model1.p};
+}
+
 // Frame ranges of the psum_r partial sums.
 static int psum_splits(const dfg_ctx *ctx) { return std::max(1, std::min(64, ctx->chunk_frames / 2048)); }
 
@@ -814,6 +839,8 @@ static int ensure_buffers(dfg_ctx *ctx) {
 	CK(ctx->logw.ensure((size_t)ctx->R_pad));
 	CK(ctx->psum_r.ensure((size_t)ctx->R_pad));
 	CK(ctx->scalars.ensure(8));
+	if (int rc = ensure_quads(ctx))
+		return rc;
 	CK(ctx->red_part.ensure(std::max<size_t>(blocks_for((long long)ctx->M * ctx->V, 256), 1024)));
 	const size_t N = (size_t)ctx->N;
 	CK(ctx->rmax.ensure(N));
@@ -1526,49 +1553,61 @@ static bool graphable(const dfg_ctx *ctx, const dfg_iter_params *par) {
 	return !ctx->keep_prob && !(ctx->with_bg && par->need_scaling && par->update_scale);
 }
 
-// Orientations per slice block: the option, else whole tiles when they give
-// every SM two blocks, else the largest block that does (16 at least).
+// Orientations per slice block: the option or the tuner's choice, else 8, so
+// that small sets fill the SMs (a block walks every pixel), and 32 once there
+// are eight such blocks per SM, where the shorter row segments of 8 cost a little.
+// Slice phase in ms at 8 / 16 / 32 / 64 / 128 orientations per block: 420 x 2304
+// pixels 0.082 / 0.131 / 0.219 / 0.402 / 0.789; 3240 x 4096 0.24 / 0.31 / 0.39 /
+// 0.73 / 1.40; 17220 x 9025 2.15 / 2.22 / 2.25 / 2.36 / 3.26; 50100 x 66820 42.8 /
+// 43.8 / 41.6 / 44.5 / 46.6. With the sums in the storing threads and eight
+// 8-byte gathers per sample those sizes took 0.163, 0.35, 2.8 and 56.
 static int slice_block_for(const dfg_ctx *ctx) {
 	int ob = (ctx->autotune && ctx->tuned && !ctx->tuning) ? ctx->tuned_ob : ctx->slice_block;
-	if (ob == 0) {
-		ob = 16;
-		for (int c : {TILE, 64, 32})
-			if (c <= TILE && ctx->R_pad / c >= 2 * ctx->num_sms) {
-				ob = c;
-				break;
-			}
-	}
+	if (ob == 0)
+		ob = ctx->R_pad / 32 >= 8 * ctx->num_sms ? 32 : 8;
 	return ob;
+}
+
+// The model's corner quads, read by every slice kernel of this iteration.
+static int launch_quads(dfg_ctx *ctx) {
+	const long long n = (long long)ctx->M * ctx->V;
+	if (!ctx->use_quads)
+		return DFG_OK;
+	quad_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(ctx->model1.p, n, ctx->S, ctx->quads.p);
+	CKL("quad_kernel");
+	return DFG_OK;
 }
 
 // Slices of every orientation with ob orientations per block: log W tiles (or
 // W in FP64 into Wd) and u_r.
 static int launch_slices(dfg_ctx *ctx, int ob, double *Wd) {
 	cudaStream_t st = ctx->stream;
-	const int M = ctx->M, R = ctx->R, RT = ctx->RT, P = ctx->P;
+	const int M = ctx->M, R = ctx->R, P = ctx->P;
 	const long long S = ctx->S, V = ctx->V;
 	const int nb = ctx->R_pad / ob;
 	// orientation parameters: quaternions (3-D) or (cos, sin) of the angles (2-D)
 	const double *geo = ctx->model_type == MT_2D ? ctx->cs2d.p : ctx->quats.p;
+	const int two_d = ctx->model_type == MT_2D;
 #define DFG_SLICE(OBV, G)                                                                                     \
-	slice_u_kernel<double, OBV, G><<<nb, 256, 0, st>>>(geo, M, R, ctx->qvals.p, ctx->corr.p, ctx->mask.p, P,     \
-	                                                   ctx->model1.p, S, V, ctx->logW.p, ctx->u.p, Wd)
-#define DFG_SLICE_ALL(G)                                                                                      \
-	if (ob == TILE)                                                                                           \
-		slice_u_tile_kernel<double, G><<<RT, 256, 0, st>>>(geo, M, R, ctx->qvals.p, ctx->corr.p, ctx->mask.p, P, \
-		                                                   ctx->model1.p, S, V, ctx->logW.p, ctx->u.p, Wd);     \
-	else if (ob == 64)                                                                                        \
-		DFG_SLICE(TILE >= 64 ? 64 : 16, G);                                                                   \
-	else if (ob == 32)                                                                                        \
-		DFG_SLICE(32, G);                                                                                     \
+	slice_u_kernel<OBV, G><<<nb, SLICE_THREADS, 0, st>>>(geo, M, R, ctx->qvals.p, ctx->corr.p, ctx->mask.p, P,    \
+	                                                     slice_model(ctx), S, V, ctx->logW.p, ctx->u.p, Wd)
+#define DFG_SLICE_ANY(OBV)                                                                                    \
+	if (two_d)                                                                                                \
+		DFG_SLICE(OBV, MT_2D);                                                                                \
 	else                                                                                                      \
-		DFG_SLICE(16, G)
-	if (ctx->model_type == MT_2D) {
-		DFG_SLICE_ALL(MT_2D);
+		DFG_SLICE(OBV, MT_3D)
+	if (ob == TILE) {
+		DFG_SLICE_ANY(TILE);
+	} else if (ob == 64) {
+		DFG_SLICE_ANY(TILE >= 64 ? 64 : TILE);
+	} else if (ob == 32) {
+		DFG_SLICE_ANY(32);
+	} else if (ob == 16) {
+		DFG_SLICE_ANY(16);
 	} else {
-		DFG_SLICE_ALL(MT_3D);
+		DFG_SLICE_ANY(8);
 	}
-#undef DFG_SLICE_ALL
+#undef DFG_SLICE_ANY
 #undef DFG_SLICE
 	CKL("slice_u_kernel");
 	return DFG_OK;
@@ -1943,6 +1982,8 @@ static int ensure_pair_buffers(dfg_ctx *ctx, const dfg_iter_params *par) {
 	CK(ctx->psum_r.ensure((size_t)ctx->R_pad));
 	CK(ctx->wsign.ensure((size_t)ctx->R_pad));
 	CK(ctx->scalars.ensure(8));
+	if (int rc = ensure_quads(ctx))
+		return rc;
 	CK(ctx->red_part.ensure(std::max<size_t>(blocks_for((long long)ctx->M * ctx->V, 256), 1024)));
 	CK(ctx->rmax.ensure(N));
 	CK(ctx->num_prob.ensure(N));
@@ -1992,21 +2033,21 @@ static int launch_slices_block(dfg_ctx *ctx, int ob, int t0, int nt) {
 	                     TILE * sizeof(float), nt, st));
 	const int nb = nt * TILE / ob;
 	const double *q = ctx->quats.p + 5 * (size_t)r0;
+#define DFG_SLICE(OBV)                                                                                        \
+	slice_u_kernel<OBV, MT_3D><<<nb, SLICE_THREADS, 0, st>>>(q, 1, Rb, ctx->qvals.p, ctx->corr.p, ctx->mask.p, P, \
+	                                                         slice_model(ctx), S, V, ctx->blk.p, ctx->u.p + r0,  \
+	                                                         nullptr)
 	if (ob == TILE)
-		slice_u_tile_kernel<double, MT_3D><<<nt, 256, 0, st>>>(q, 1, Rb, ctx->qvals.p, ctx->corr.p, ctx->mask.p, P,
-		                                                       ctx->model1.p, S, V, ctx->blk.p, ctx->u.p + r0, nullptr);
+		DFG_SLICE(TILE);
 	else if (ob == 64)
-		slice_u_kernel<double, TILE >= 64 ? 64 : 16, MT_3D><<<nb, 256, 0, st>>>(
-		    q, 1, Rb, ctx->qvals.p, ctx->corr.p, ctx->mask.p, P, ctx->model1.p, S, V, ctx->blk.p, ctx->u.p + r0,
-		    nullptr);
+		DFG_SLICE(TILE >= 64 ? 64 : TILE);
 	else if (ob == 32)
-		slice_u_kernel<double, 32, MT_3D><<<nb, 256, 0, st>>>(q, 1, Rb, ctx->qvals.p, ctx->corr.p, ctx->mask.p, P,
-		                                                      ctx->model1.p, S, V, ctx->blk.p, ctx->u.p + r0,
-		                                                      nullptr);
+		DFG_SLICE(32);
+	else if (ob == 16)
+		DFG_SLICE(16);
 	else
-		slice_u_kernel<double, 16, MT_3D><<<nb, 256, 0, st>>>(q, 1, Rb, ctx->qvals.p, ctx->corr.p, ctx->mask.p, P,
-		                                                      ctx->model1.p, S, V, ctx->blk.p, ctx->u.p + r0,
-		                                                      nullptr);
+		DFG_SLICE(8);
+#undef DFG_SLICE
 	CKL("slice_u_kernel");
 	return DFG_OK;
 }
@@ -2029,6 +2070,8 @@ static int max_enqueue_pairs(dfg_ctx *ctx, const dfg_iter_params *par) {
 		                                                 ctx->beta.p);
 		CKL("beta_kernel");
 	}
+	if (int rc = launch_quads(ctx))
+		return rc;
 	for (int t0 = 0; t0 < RT; t0 += BT) {
 		const int nt = std::min(BT, RT - t0);
 		phase_begin(ctx, PH_SLICE);
@@ -2093,13 +2136,13 @@ static int max_enqueue_pairs(dfg_ctx *ctx, const dfg_iter_params *par) {
 		phase_begin(ctx, PH_MERGE);
 		merge_kernel<MT_3D, true><<<dim3(nblk, nt), 256, 0, st>>>(
 		    ctx->blk.p, ctx->psum_r.p + r0, ctx->quats.p + 5 * (size_t)r0, 1, Rb, ctx->qvals.p, ctx->corr.p,
-		    ctx->mask.p, P, S, V, (double *)ctx->accum.p, ctx->wflags.p, 0, ctx->wsign.p + r0);
+		    ctx->mask.p, P, S, V, (long long)M * V, (double *)ctx->accum.p, ctx->wflags.p, 0, ctx->wsign.p + r0);
 		CKL("merge_kernel");
 		phase_end(ctx, PH_MERGE, 1);
 	}
 	phase_begin(ctx, PH_UPDATE);
 	unpack_accum_kernel<<<blocks_for((long long)M * V, 256), 256, 0, st>>>(
-	    ctx->accum.p, (long long)M * V, ctx->model2.p, ctx->weight.p, ctx->weight_cache.p, ctx->wflags.p);
+	    (const double *)ctx->accum.p, (long long)M * V, ctx->model2.p, ctx->weight.p, ctx->weight_cache.p, ctx->wflags.p);
 	CKL("unpack_accum_kernel");
 	frame_totals_kernel<<<1, 1024, 0, st>>>(ctx->info.p, ctx->likelihood.p, ctx->blacklist.p, N,
 	                                        ctx->scalars.p + 1);
@@ -2161,6 +2204,8 @@ static int blocked_prepare(dfg_ctx *ctx, const dfg_iter_params *par) {
 	CK(ctx->logw.ensure((size_t)ctx->R_pad));
 	CK(ctx->psum_r.ensure((size_t)ctx->R_pad));
 	CK(ctx->scalars.ensure(8));
+	if (int rc = ensure_quads(ctx))
+		return rc;
 	CK(ctx->red_part.ensure(std::max<size_t>(blocks_for((long long)ctx->M * ctx->V, 256), 1024)));
 	CK(ctx->rmax.ensure(N));
 	CK(ctx->num_prob.ensure(N));
@@ -2239,6 +2284,8 @@ static int max_enqueue_blocked(dfg_ctx *ctx, const dfg_iter_params *par) {
 		CKL("beta_kernel");
 	}
 	phase_begin(ctx, PH_SLICE);
+	if (int rc = launch_quads(ctx))
+		return rc;
 	for (int t0 = 0; t0 < RT; t0 += BT)
 		if (int rc = launch_slices_block(ctx, ob, t0, std::min(BT, RT - t0)))
 			return rc;
@@ -2246,7 +2293,7 @@ static int max_enqueue_blocked(dfg_ctx *ctx, const dfg_iter_params *par) {
 	CKL("rescale_kernel");
 	logw_kernel<<<blocks_for(R, 256), 256, 0, st>>>(ctx->quats.p, M, R, ctx->logw.p);
 	CKL("logw_kernel");
-	phase_end(ctx, PH_SLICE, (RT + BT - 1) / BT + 2);
+	phase_end(ctx, PH_SLICE, (RT + BT - 1) / BT + 3);
 	CK(cudaMemsetAsync(ctx->psum_r.p, 0, (size_t)R_pad * sizeof(double), st));
 	CK(cudaMemsetAsync(ctx->accum.p, 0, (size_t)M * V * sizeof(double2), st));
 	const int use_scale = par->need_scaling && (par->iteration > 1 || par->known_scale);
@@ -2317,13 +2364,13 @@ static int max_enqueue_blocked(dfg_ctx *ctx, const dfg_iter_params *par) {
 		merge_kernel<MT_3D><<<dim3(nblk, nt), 256, 0, st>>>(ctx->blkT.p, ctx->psum_r.p + r0,
 		                                                     ctx->quats.p + 5 * (size_t)r0, 1, Rb, ctx->qvals.p,
 		                                                     ctx->corr.p, ctx->mask.p, P, S, V,
-		                                                     (double *)ctx->accum.p, ctx->wflags.p, 0);
+		                                                     (long long)M * V, (double *)ctx->accum.p, ctx->wflags.p, 0);
 		CKL("merge_kernel");
 		phase_end(ctx, PH_MERGE, 1);
 	}
 	phase_begin(ctx, PH_UPDATE);
 	unpack_accum_kernel<<<blocks_for((long long)M * V, 256), 256, 0, st>>>(
-	    ctx->accum.p, (long long)M * V, ctx->model2.p, ctx->weight.p, ctx->weight_cache.p, ctx->wflags.p);
+	    (const double *)ctx->accum.p, (long long)M * V, ctx->model2.p, ctx->weight.p, ctx->weight_cache.p, ctx->wflags.p);
 	CKL("unpack_accum_kernel");
 	frame_totals_kernel<<<1, 1024, 0, st>>>(ctx->info.p, ctx->likelihood.p, ctx->blacklist.p, N,
 	                                        ctx->scalars.p + 1);
@@ -2367,6 +2414,8 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 
 	// slices, u_r, rescale (calculate_rescale, max_prob.c:3-64)
 	phase_begin(ctx, PH_SLICE);
+	if (int rc = launch_quads(ctx))
+		return rc;
 	if (int rc = launch_slices(ctx, slice_block_for(ctx), Wd))
 		return rc;
 	rescale_kernel<<<1, 256, 0, st>>>(ctx->u.p, ctx->quats.p, M, R, ctx->mean_count, ctx->scalars.p);
@@ -2382,7 +2431,7 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 	if (ctx->hot_active)
 		if (int rc = launch_hot_digits(ctx))
 			return rc;
-	phase_end(ctx, PH_SLICE, 3 + (ctx->dense_active ? 1 : 0) + (ctx->hot_active ? 1 : 0));
+	phase_end(ctx, PH_SLICE, 4 + (ctx->dense_active ? 1 : 0) + (ctx->hot_active ? 1 : 0));
 
 	CK(cudaMemsetAsync(ctx->T.p, 0, (size_t)RT * P * TILE * sizeof(float), st));
 	CK(cudaMemsetAsync(ctx->psum_r.p, 0, (size_t)R_pad * sizeof(double), st));
@@ -2460,18 +2509,18 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 	phase_begin(ctx, PH_MERGE);
 	if (two_d)
 		merge_kernel<MT_2D><<<dim3(nblk, RT), 256, 0, st>>>(ctx->T.p, ctx->psum_r.p, ctx->cs2d.p, M, R, ctx->qvals.p,
-		                                                     ctx->corr.p, ctx->mask.p, P, S, V, (double *)ctx->accum.p,
+		                                                     ctx->corr.p, ctx->mask.p, P, S, V, (long long)M * V, (double *)ctx->accum.p,
 		                                                     ctx->wflags.p, bg ? 1 : 0);
 	else
 		merge_kernel<MT_3D><<<dim3(nblk, RT), 256, 0, st>>>(ctx->T.p, ctx->psum_r.p, ctx->quats.p, M, R, ctx->qvals.p,
-		                                                     ctx->corr.p, ctx->mask.p, P, S, V, (double *)ctx->accum.p,
+		                                                     ctx->corr.p, ctx->mask.p, P, S, V, (long long)M * V, (double *)ctx->accum.p,
 		                                                     ctx->wflags.p, bg ? 1 : 0);
 	CKL("merge_kernel");
 	phase_end(ctx, PH_MERGE, 1);
 
 	phase_begin(ctx, PH_UPDATE);
 	unpack_accum_kernel<<<blocks_for((long long)M * V, 256), 256, 0, st>>>(
-	    ctx->accum.p, (long long)M * V, ctx->model2.p, ctx->weight.p, ctx->weight_cache.p, ctx->wflags.p);
+	    (const double *)ctx->accum.p, (long long)M * V, ctx->model2.p, ctx->weight.p, ctx->weight_cache.p, ctx->wflags.p);
 	CKL("unpack_accum_kernel");
 	// averages over good frames; the packaged Iterate never sets num_blacklist,
 	// so they divide by N (max_prob.c:373-374, iterate.pyx:35)
@@ -2542,6 +2591,8 @@ static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par) {
 	                                  : RefineMask{nullptr, nullptr, 0};
 	const int obs[4] = {128, 64, 32, 16};
 	int bi = -1;
+	if (rc == DFG_OK)
+		rc = launch_quads(ctx);
 	for (int i = 0; i < 4 && rc == DFG_OK; ++i) {
 		const int ob = obs[i];
 		if (ob > TILE || TILE % ob != 0)
@@ -3861,8 +3912,8 @@ extern "C" int dfg_set_option(dfg_ctx *ctx, const char *key, double value) {
 	}
 	if (!strcmp(key, "slice_block")) {
 		const int v = (int)value;
-		NEED(v == 0 || ((v == 16 || v == 32 || v == 64 || v == TILE) && v <= TILE), DFG_ERR_ARG,
-		     "slice_block must be 0 (automatic), 16, 32, 64 (at most %d) or %d", TILE, TILE);
+		NEED(v == 0 || v == 8 || ((v == 16 || v == 32 || v == 64 || v == TILE) && v <= TILE), DFG_ERR_ARG,
+		     "slice_block must be 0 (automatic), 8, 16, 32, 64 (at most %d) or %d", TILE, TILE);
 		ctx->slice_block = v;
 		return DFG_OK;
 	}

@@ -19,7 +19,7 @@
 //                                P > 1e-6 stored as +P, kept but <= 1e-6 as -P,
 //                                pruned 0; row Nc is all zero.
 //   T        [RT][P][TILE] float  photon tomograms sum_d P_dr * K_d[p].
-//   accum    [M*V] double2       (model2 sum, weight) merge accumulators.
+//   accum    [2][M*V] double      merge accumulators: model2 sums, then weights.
 // Photon lists: per frame (E-step) or per pixel (M-step) a segment of
 // count-1 photons followed by a segment of multi-photon words, each padded to
 // a multiple of 8 with words that point at the zero row. Count-1 words hold
@@ -88,18 +88,23 @@ struct Cell {
 	bool ok;
 };
 
+// Truncation toward zero for the bounds test and the fraction: 32-bit
+// conversions (a volume's side stays far below 2^31), which saturate past the
+// range and give 0 for NaN; NaN positions are out of bounds.
 __device__ __forceinline__ Cell locate(const double *rot, double qx, double qy, double qz, double center,
                                        long long S) {
 	Cell c;
-	double px = dadd(dadd(dadd(dmul(rot[0], qx), dmul(rot[1], qy)), dmul(rot[2], qz)), center);
-	double py = dadd(dadd(dadd(dmul(rot[3], qx), dmul(rot[4], qy)), dmul(rot[5], qz)), center);
-	double pz = dadd(dadd(dadd(dmul(rot[6], qx), dmul(rot[7], qy)), dmul(rot[8], qz)), center);
-	long long x = (long long)px, y = (long long)py, z = (long long)pz;
-	c.ok = !(x < 0 || x > S - 2 || y < 0 || y > S - 2 || z < 0 || z > S - 2);
+	const double px = dadd(dadd(dadd(dmul(rot[0], qx), dmul(rot[1], qy)), dmul(rot[2], qz)), center);
+	const double py = dadd(dadd(dadd(dmul(rot[3], qx), dmul(rot[4], qy)), dmul(rot[5], qz)), center);
+	const double pz = dadd(dadd(dadd(dmul(rot[6], qx), dmul(rot[7], qy)), dmul(rot[8], qz)), center);
+	const int x = __double2int_rz(px), y = __double2int_rz(py), z = __double2int_rz(pz);
+	const unsigned top = (unsigned)((int)S - 2);
+	const auto real = [](double v) { return (unsigned)(__double2hiint(v) & 0x7fffffff) <= 0x7ff00000u; };
+	c.ok = (unsigned)x <= top && (unsigned)y <= top && (unsigned)z <= top && real(px) && real(py) && real(pz);
 	c.fx = dsub(px, (double)x);
 	c.fy = dsub(py, (double)y);
 	c.fz = dsub(pz, (double)z);
-	c.i000 = c.ok ? (x * S + y) * S + z : 0;
+	c.i000 = c.ok ? (long long)(x * (int)S + y) * S + z : 0;
 	return c;
 }
 
@@ -239,6 +244,60 @@ __device__ __forceinline__ double geo_sample(const double *rot, double qx, doubl
 	}
 }
 
+// A model to take slices of: its corner quads (quad_kernel), or without them
+// (too large a copy) the voxels themselves.
+struct SliceModel {
+	const double4 *quads;
+	const double *voxels;
+};
+
+// The model at voxel v and at +1, +S, +S + 1 from it.
+__device__ __forceinline__ void ld_quad(const SliceModel &m, long long v, long long S, double (&x)[4]) {
+	if (m.quads != nullptr) {
+		asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+		    : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3])
+		    : "l"(m.quads + v));
+	} else {
+		x[0] = __ldg(m.voxels + v);
+		x[1] = __ldg(m.voxels + v + 1);
+		x[2] = __ldg(m.voxels + v + S);
+		x[3] = __ldg(m.voxels + v + S + 1);
+	}
+}
+
+// geo_sample of the model from voxel v0 on: the same terms in the same order.
+template <int GEO>
+__device__ __forceinline__ double quad_sample(const double *rot, double qx, double qy, double qz, double center,
+                                              long long S, const SliceModel &m, long long v0, double corr) {
+	double a[4], w[8];
+	if constexpr (GEO == MT_3D) {
+		const Cell c = locate(rot, qx, qy, qz, center, S);
+		if (!c.ok)
+			return DBL_MIN;
+		double b[4];
+		ld_quad(m, v0 + c.i000, S, a);
+		ld_quad(m, v0 + c.i000 + S * S, S, b);
+		corner_weights(c, w);
+		double v = dmul(w[0], a[0]);
+#pragma unroll
+		for (int k = 1; k < 8; ++k)
+			v = dadd(v, dmul(w[k], k < 4 ? a[k] : b[k - 4]));
+		return dmul(v, corr);
+	} else {
+		const Cell2 c = locate2d(rot, qx, qy, center, S);
+		if (!c.ok)
+			return DBL_MIN;
+		ld_quad(m, v0 + c.i00, S, a);
+		corner_weights2(c, w);
+		double v = dmul(w[0], a[0]);
+#pragma unroll
+		for (int k = 1; k < 4; ++k)
+			v = dadd(v, dmul(w[k], a[k]));
+		v = dmul(v, corr);
+		return v <= 0. ? DBL_MIN : v;
+	}
+}
+
 // Compensated FP32 summation (Kahan): the represented sum is s - comp, with
 // an error of order n u^2 sum|x| (u = 2^-24), i.e. far below FP32 rounding.
 // Intrinsics keep the compiler from simplifying (t - s) - y.
@@ -341,6 +400,18 @@ __device__ __forceinline__ void ld_row(const float *__restrict__ p, float (&v)[L
 		v[0] = x.x; v[1] = x.y;
 	} else {
 		v[0] = __ldg(p);
+	}
+}
+
+// Same, for rows read once: they leave L2 first.
+__device__ __forceinline__ void ld_row_stream(const float *__restrict__ p, float (&v)[LW]) {
+	if constexpr (LW == 4) {
+		const float4 x = __ldcs(reinterpret_cast<const float4 *>(p));
+		v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+	} else {
+#pragma unroll
+		for (int k = 0; k < LW; ++k)
+			v[k] = __ldcs(p + k);
 	}
 }
 

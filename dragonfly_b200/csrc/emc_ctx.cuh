@@ -148,6 +148,8 @@ struct dfg_ctx {
 	long long S = 0, V = 0;
 	DevBuf<double> model1, model2, weight;
 	DevBuf<double2> accum;
+	DevBuf<double4> quads;  // the model's corner quads (quad_kernel), remade every iteration
+	bool use_quads = false;
 	// inter_weight of the last merge and the psum_r > 0 pattern it was built
 	// for (the weights depend on nothing else once geometry is fixed); the
 	// pattern and the flags (accumulate weights, grid cached) live on the

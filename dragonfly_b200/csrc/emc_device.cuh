@@ -9,187 +9,133 @@ namespace dfg {
 // ---------------------------------------------------------------------------
 // (a) slice generation: logW[tile][p][j] = log(W_r[p]) and u_r, r = tile * TILE + j
 // ---------------------------------------------------------------------------
-// Block = one orientation tile; it walks every pixel in chunks of SB pixels,
-// in pixel order. Per chunk the 256 threads compute W for SB pixels x TILE
-// orientations into shared memory (thread (i = t % SB, g = t / SB) takes
-// pixel i of orientations g, g + 256/SB, ..., so a warp walks 32 neighbouring
-// pixels of one orientation); then thread j < TILE adds the chunk's mask-0
-// values of orientation j to u_j in pixel order, which keeps u_r
-// bit-identical to the reference's sequential sum (max_prob.c:32-38), while
-// the warps store log W as coalesced rows (max_prob.c:94-97); with Wd given
-// (background-aware path, max_prob.c:94) they store W itself in FP64 there.
-constexpr int SB = 32;
-
-template <typename MT, int GEO>
-__global__ void __launch_bounds__(256) slice_u_tile_kernel(
-    const double *__restrict__ quats, int M, int R, const double *__restrict__ qvals,
-    const double *__restrict__ corr, const uint8_t *__restrict__ mask, int P, const MT *__restrict__ model,
-    long long S, long long V, float *__restrict__ logW, double *__restrict__ u, double *__restrict__ Wd) {
-	__shared__ double s_rot[TILE][9];
-	__shared__ int s_mode[TILE];
-	__shared__ double s_w[SB][TILE + 1];
-	__shared__ double s_q[SB][4];
-	__shared__ int s_m[SB];
-	const int t = threadIdx.x, rt = blockIdx.x;
-	for (int j = t; j < TILE; j += blockDim.x) {
-		int r = rt * TILE + j;
-		int rr = r < R ? r : 0;
-		geo_setup<GEO>(quats, rr / M, s_rot[j]);
-		s_mode[j] = rr % M;
-	}
-	const double center = (double)(S / 2);
-	const int i = t % SB, g = t / SB, w = t >> 5, lane = t & 31;
-	double acc = 0.;
-	for (int p0 = 0; p0 < P; p0 += SB) {
-		if (t < SB) {
-			const int p = p0 + t;
-			if (p < P) {
-				s_q[t][0] = qvals[3 * (size_t)p];
-				s_q[t][1] = qvals[3 * (size_t)p + 1];
-				s_q[t][2] = qvals[3 * (size_t)p + 2];
-				s_q[t][3] = corr[p];
-				s_m[t] = mask[p];
-			} else {
-				s_m[t] = -1;
-			}
-		}
-		__syncthreads();
-		if (s_m[i] >= 0) {
-			const double qx = s_q[i][0], qy = s_q[i][1], qz = s_q[i][2], cr = s_q[i][3];
-#pragma unroll 2
-			for (int j = g; j < TILE; j += 256 / SB) {
-				if constexpr (GEO == MT_3D) {
-					Cell c = locate(s_rot[j], qx, qy, qz, center, S);
-					s_w[i][j] = interp(c, model + (size_t)s_mode[j] * V, S, cr);
-				} else {
-					s_w[i][j] = geo_sample<GEO>(s_rot[j], qx, qy, qz, center, S, model + (size_t)s_mode[j] * V, cr);
-				}
-			}
-		}
-		__syncthreads();
-		if (t < TILE) {
-#pragma unroll 8
-			for (int k = 0; k < SB; ++k)
-				if (s_m[k] == 0)
-					acc = dadd(acc, s_w[k][t]);
-		}
-		for (int row = w; row < SB; row += 8) {
-			const int pp = p0 + row;
-			if (pp < P) {
-				if (Wd != nullptr) {
-					double v[LW];
-#pragma unroll
-					for (int k = 0; k < LW; ++k)
-						v[k] = s_w[row][lane * LW + k];
-					st_row(Wd + ((size_t)rt * (P + 1) + pp) * TILE + lane * LW, v);
-				} else {
-					float v[LW];
-#pragma unroll
-					for (int k = 0; k < LW; ++k)
-						v[k] = (float)log(s_w[row][lane * LW + k]);
-					st_row(logW + ((size_t)rt * (P + 1) + pp) * TILE + lane * LW, v);
-				}
-			}
-		}
-		__syncthreads();
-	}
-	if (t < TILE && rt * TILE + t < R)
-		u[rt * TILE + t] = acc;
+// The model as corner quads: quad[v] holds the model at voxel v and at its
+// neighbours in the last two axes, (+0, +1, +S, +S + 1), zero past the end (no
+// cell reaches there). A trilinear sample then is two 32-byte loads instead of eight
+// of 8 bytes (a bilinear one a single load). The slices were bound by the L1
+// wavefronts of those gathers (88 % of the L1 rate, FP64 pipe 32 %): a warp's 32
+// neighbouring pixels touch as many lines with each load however narrow it is.
+__global__ void __launch_bounds__(256) quad_kernel(const double *__restrict__ model, long long n, long long S,
+                                                   double4 *__restrict__ quad) {
+	const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= n)
+		return;
+	auto at = [&](long long v) { return v < n ? __ldg(model + v) : 0.; };
+	quad[i] = make_double4(at(i), at(i + 1), at(i + S), at(i + S + 1));
 }
 
-// Block = OB consecutive orientations (OB divides TILE); it walks every pixel
-// in chunks of 4096 / OB pixels, in pixel order. Per chunk the 256 threads
-// compute W for the chunk's pixels x OB orientations into shared memory
-// (consecutive threads take consecutive pixels of one orientation, so a warp
-// reads neighbouring model voxels); then thread j < OB adds the chunk's
-// mask-0 values of its orientation to u in pixel order, which keeps u_r
-// bit-identical to the reference's sequential sum (max_prob.c:32-38), while
-// all threads store log W as coalesced row segments (max_prob.c:94-97). The
-// host uses it when whole tiles would give the SMs too few blocks.
-template <typename MT, int OB, int GEO>
-__global__ void __launch_bounds__(256) slice_u_kernel(
+// Block = OB consecutive orientations (OB divides TILE); it walks every pixel in
+// chunks of CB, in pixel order. Eight warps compute W of a chunk into shared
+// memory (consecutive threads take consecutive pixels of one orientation, so a
+// warp reads neighbouring voxels) and, after a barrier among themselves, store log W as
+// coalesced row segments (max_prob.c:94-97; with Wd given, for the
+// background-aware path, W itself in FP64). Meanwhile a ninth warp adds the
+// previous chunk's mask-0 values to u in pixel order -- one chain of additions
+// per orientation, which keeps u_r bit-identical to the reference's sequential
+// sum (max_prob.c:32-38) -- and fetches the next chunk's pixels (in the storing
+// threads the sums held the whole block up). Bound by the L1 path of the
+// gathers; times and block sizes at slice_block_for.
+template <int OB>
+struct SliceShape {
+	static constexpr int SAMPLES = OB >= 32 ? 2048 : 1024;  // per chunk
+	static constexpr int CB = SAMPLES / OB;                  // pixels per chunk
+};
+constexpr int SLICE_THREADS = 288;
+
+template <int OB, int GEO>
+__global__ void __launch_bounds__(SLICE_THREADS, 3) slice_u_kernel(
     const double *__restrict__ quats, int M, int R, const double *__restrict__ qvals,
-    const double *__restrict__ corr, const uint8_t *__restrict__ mask, int P, const MT *__restrict__ model,
+    const double *__restrict__ corr, const uint8_t *__restrict__ mask, int P, const SliceModel model,
     long long S, long long V, float *__restrict__ logW, double *__restrict__ u, double *__restrict__ Wd) {
-	static_assert(TILE % OB == 0 && OB % LW == 0, "orientation block must divide the tile");
-	constexpr int CB = 4096 / OB;  // pixels per chunk
+	static_assert(TILE % OB == 0, "orientation block must divide the tile");
+	constexpr int CB = SliceShape<OB>::CB;
 	static_assert(256 % CB == 0, "a thread keeps one pixel of the chunk");
-	constexpr int SEG = OB / LW;   // vector stores per row segment
+	constexpr int NU = OB >= 32 ? OB / 32 : 1;   // sums per lane of the ninth warp
 	__shared__ double s_rot[OB][9];
 	__shared__ int s_mode[OB];
-	__shared__ double s_w[CB][OB + 1];
-	__shared__ double s_q[CB][4];
-	__shared__ int s_m[CB];
-	const int t = threadIdx.x, r0 = blockIdx.x * OB, rt = r0 / TILE, jj0 = r0 % TILE;
+	__shared__ double s_w[2][CB][OB + 1];
+	__shared__ double s_q[3][CB][4];
+	__shared__ int s_m[3][CB];
+	const int t = threadIdx.x, lane = t & 31, r0 = blockIdx.x * OB, rt = r0 / TILE, jj0 = r0 % TILE;
+	const bool sums = t >= 256;
 	for (int j = t; j < OB; j += blockDim.x) {
 		const int r = r0 + j;
 		const int rr = r < R ? r : 0;
 		geo_setup<GEO>(quats, rr / M, s_rot[j]);
 		s_mode[j] = rr % M;
 	}
-	const double center = (double)(S / 2);
-	double acc = 0.;
-	for (int p0 = 0; p0 < P; p0 += CB) {
-		for (int k = t; k < CB; k += blockDim.x) {
-			const int p = p0 + k;
+	auto fetch = [&](int c) {
+		for (int k = lane; k < CB; k += 32) {
+			const int p = c * CB + k;
 			if (p < P) {
-				s_q[k][0] = qvals[3 * (size_t)p];
-				s_q[k][1] = qvals[3 * (size_t)p + 1];
-				s_q[k][2] = qvals[3 * (size_t)p + 2];
-				s_q[k][3] = corr[p];
-				s_m[k] = mask[p];
+				s_q[c % 3][k][0] = qvals[3 * (size_t)p];
+				s_q[c % 3][k][1] = qvals[3 * (size_t)p + 1];
+				s_q[c % 3][k][2] = qvals[3 * (size_t)p + 2];
+				s_q[c % 3][k][3] = corr[p];
+				s_m[c % 3][k] = mask[p];
 			} else {
-				s_m[k] = -1;
+				s_m[c % 3][k] = -1;
 			}
 		}
-		__syncthreads();
-		{
-			// 256 is a multiple of CB: thread t keeps pixel t % CB in registers
-			// and takes orientations t / CB, t / CB + 256 / CB, ...
-			const int i = t % CB;
-			if (s_m[i] >= 0) {
-				const double qx = s_q[i][0], qy = s_q[i][1], qz = s_q[i][2], cr = s_q[i][3];
-#pragma unroll 2
-				for (int j = t / CB; j < OB; j += 256 / CB) {
-					if constexpr (GEO == MT_3D) {
-						Cell c = locate(s_rot[j], qx, qy, qz, center, S);
-						s_w[i][j] = interp(c, model + (size_t)s_mode[j] * V, S, cr);
-					} else {
-						s_w[i][j] =
-						    geo_sample<GEO>(s_rot[j], qx, qy, qz, center, S, model + (size_t)s_mode[j] * V, cr);
-					}
-				}
-			}
-		}
-		__syncthreads();
-		if (t < OB) {
+	};
+	if (sums)
+		fetch(0);
+	__syncthreads();
+	const double center = (double)(S / 2);
+	const int nc = (P + CB - 1) / CB;
+	double acc[NU];
+#pragma unroll
+	for (int k = 0; k < NU; ++k)
+		acc[k] = 0.;
+	for (int c = 0; c <= nc; ++c) {
+		if (sums) {
+			if (c + 1 < nc)
+				fetch(c + 1);
+			if (c > 0 && lane < OB) {
+				const double(*w)[OB + 1] = s_w[(c - 1) & 1];
+				const int *m = s_m[(c - 1) % 3];
 #pragma unroll 8
-			for (int k = 0; k < CB; ++k)
-				if (s_m[k] == 0)
-					acc = dadd(acc, s_w[k][t]);
-		}
-		for (int idx = t; idx < CB * SEG; idx += blockDim.x) {
-			const int row = idx / SEG, seg = idx % SEG, pp = p0 + row;
-			if (pp < P) {
-				if (Wd != nullptr) {
-					double v[LW];
+				for (int k = 0; k < CB; ++k)
+					if (m[k] == 0) {
 #pragma unroll
-					for (int k = 0; k < LW; ++k)
-						v[k] = s_w[row][seg * LW + k];
-					st_row(Wd + ((size_t)rt * (P + 1) + pp) * TILE + jj0 + seg * LW, v);
-				} else {
-					float v[LW];
-#pragma unroll
-					for (int k = 0; k < LW; ++k)
-						v[k] = (float)log(s_w[row][seg * LW + k]);
-					st_row(logW + ((size_t)rt * (P + 1) + pp) * TILE + jj0 + seg * LW, v);
-				}
+						for (int h = 0; h < NU; ++h)
+							acc[h] = dadd(acc[h], w[k][lane + 32 * h]);
+					}
+			}
+		} else if (c < nc) {
+			double(*w)[OB + 1] = s_w[c & 1];
+			const int i = t % CB;
+			if (s_m[c % 3][i] >= 0) {
+				const double *q = s_q[c % 3][i];
+				const double qx = q[0], qy = q[1], qz = q[2], cr = q[3];
+#pragma unroll 2
+				for (int j = t / CB; j < OB; j += 256 / CB)
+					w[i][j] = quad_sample<GEO>(s_rot[j], qx, qy, qz, center, S, model, (long long)s_mode[j] * V, cr);
+			}
+			asm volatile("bar.sync 1, 256;" ::: "memory");
+			const size_t row0 = (size_t)rt * (P + 1) + (size_t)c * CB;
+			const int rows = min(CB, P - c * CB);
+#pragma unroll 2
+			for (int idx = t; idx < rows * OB; idx += 256) {
+				const int row = idx / OB, col = idx % OB;
+				const size_t at = (row0 + row) * TILE + jj0 + col;
+				const double v = w[row][col];
+				if (Wd != nullptr)
+					Wd[at] = v;
+				else
+					logW[at] = (float)log(v);
 			}
 		}
 		__syncthreads();
 	}
-	if (t < OB && r0 + t < R)
-		u[r0 + t] = acc;
+	if (sums && lane < OB) {
+#pragma unroll
+		for (int h = 0; h < NU; ++h) {
+			const int r = r0 + lane + 32 * h;
+			if (r < R)
+				u[r] = acc[h];
+		}
+	}
 }
 
 // log w_r per orientation, so that no pair evaluates a logarithm of its
@@ -1115,57 +1061,63 @@ __global__ void __launch_bounds__(256, MINB) mstep_kernel(const float *__restric
 // ---------------------------------------------------------------------------
 // (e2) merge: slice_merge3d of tomo_r / psum_r for every r with psum_r > 0
 // ---------------------------------------------------------------------------
-// Block = orientation tile x PB pixels (same thread layout as slice_log_kernel).
-// The tile's tomogram rows are staged through shared memory; each
-// (pixel, orientation) with mask <= 1 and in bounds adds (f * w, f) to its 8
-// corners (model.c:171-244, max_update.c:33-36). The accumulators are FP64
-// (model, weight) pairs, interleaved so both atomics of a corner hit one
-// 32-byte sector: FP32 sums of thousands of contributions per voxel would
-// carry ~1e-6 relative error into the next iteration's likelihoods.
-// The weight sum depends only on which orientations have psum_r > 0; when
-// that set is the one of a cached weight grid, with_weight is 0 and only the
-// model sums are accumulated. With views_final the tomograms already are the
-// views (background-aware update) and are not divided by psum_r.
-// INCR (pair lists): zero tomogram values add nothing and are skipped, and
-// the weights are a change to the cached grid: wsign[r] = +1 / -1 adds /
-// subtracts orientation r's weights (its psum_r > 0 state changed, or +1 for
-// every orientation with psum_r > 0 when no grid is cached), 0 adds none.
-// The full merge's scatter with warp aggregation: the 32 lanes of a warp hold
-// 32 consecutive pixels of one orientation (j = g + 4 k is the same for the
-// warp), and neighbouring pixels often fall in the same trilinear cell.
-// Lanes whose cells coincide (__match_any_sync on the cell index) add their
-// corner contributions in registers, in lane order, and the group's lowest
-// lane issues one atomic per corner for the group.
+// Block = orientation tile x PB pixels. The tile's tomogram rows are staged
+// through shared memory; each (pixel, orientation) with mask <= 1 and in bounds
+// adds (f * w, f) to its 8 corners (model.c:171-244, max_update.c:33-36). The
+// accumulators are FP64: FP32 sums of thousands of contributions per voxel
+// would carry ~1e-6 relative error into the next iteration's likelihoods. They are
+// two planes of n = M V sums, model then weights: the weight sum depends only
+// on which orientations have psum_r > 0, so when that set is the one of a cached
+// weight grid with_weight is 0 and the model plane alone is touched, and a
+// zero tomogram value adds nothing. With views_final the tomograms already are
+// the views (background-aware update) and are not divided by psum_r.
+// INCR (pair lists): the weights are a change to the cached grid: wsign[r] = +1
+// / -1 adds / subtracts orientation r's weights (its psum_r > 0 state changed,
+// or +1 for every orientation with psum_r > 0 when no grid is cached), 0 adds none.
+//
+// The kernel is bound by the L2's atomic units: 190e9 32-byte sectors a second
+// while the grid fits L2 (33e9 when it does not: at 201^3 one plane is 65 MB,
+// two interleaved were 130), with up to two doubles of a sector at no extra cost. So the
+// full merge sends as few sectors as it can:
+// * the 32 lanes of a warp hold 32 consecutive pixels of one orientation (j =
+//   g + 4 k is the same for the warp); lanes whose trilinear cells coincide
+//   (__match_any_sync on the cell index) add their corner contributions in
+//   registers, in lane order, and the group's lowest lane goes on for the group;
+// * neighbouring lanes then trade halves of their corner pairs, so that one
+//   atomic instruction carries both ends of a pair (consecutive doubles, one
+//   sector in three of four cases) in neighbouring lanes.
+// Near the solution most tomogram values are zero: 10860 x 15625 pixels 4.69 ->
+// 2.01 ms, 10860 x 8281 refined 2.59 -> 1.31; all non-zero: 17220 x 9025 4.49 ->
+// 3.98, 50100 x 66820 84 (bound by issue: geometry and group sums).
 template <int GEO>
 __device__ __forceinline__ void merge_aggregated(const float (*s_tile)[TILE + 1], const double *s_ps,
                                                  const double (*s_rot)[9], const int *s_mode, int i, int g, int p,
                                                  int P, const double *__restrict__ qvals,
                                                  const double *__restrict__ corr, const uint8_t *__restrict__ mask,
-                                                 long long S, long long V, double *__restrict__ accum,
+                                                 long long S, long long V, long long n, double *__restrict__ accum,
                                                  int with_weight, int views_final) {
 	const int lane = threadIdx.x & 31;
-	const bool pix = p < P && mask[p] <= 1;
+	const bool pix = p < P && mask[p] <= 1, odd = lane & 1;
 	const int pp = pix ? p : 0;
 	const double qx = qvals[3 * (size_t)pp], qy = qvals[3 * (size_t)pp + 1], qz = qvals[3 * (size_t)pp + 2];
-	const double cr = corr[pp];
+	const double icr = 1. / corr[pp];
 	const double center = (double)(S / 2);
 	constexpr int NC = GEO == MT_3D ? 8 : 4;  // corners
-	// corner q's offset from the cell's first voxel (corner_offsets order)
-	auto off = [S](int q) -> long long {
-		if constexpr (GEO == MT_3D)
-			return (long long)(q & 1) + ((q >> 1) & 1) * S + (long long)(q >> 2) * S * S;
-		else
-			return (long long)(q & 1) + (long long)(q >> 1) * S;
+	// corner pair h's offset from the cell's first voxel (corner_offsets order:
+	// corners 2 h and 2 h + 1 are consecutive)
+	auto off = [S](int h) -> long long {
+		return GEO == MT_3D ? (long long)(h & 1) * S + (long long)(h >> 1) * S * S : (long long)h * S;
 	};
 	for (int k = 0; k < TILE / 4; ++k) {
 		const int j = g + 4 * k;   // the same for every lane of the warp
-		const double ps = s_ps[j];
-		if (!(ps > 0.))
+		const double ips = s_ps[j];
+		if (!(ips > 0.))
 			continue;
+		const float tv = s_tile[i][j];
 		double fw[8];
 		long long base = -1;
 		bool ok = false;
-		if (pix) {
+		if (pix && (with_weight || tv != 0.f || isinf(icr))) {
 			if constexpr (GEO == MT_3D) {
 				Cell c = locate(s_rot[j], qx, qy, qz, center, S);
 				ok = c.ok;
@@ -1190,33 +1142,44 @@ __device__ __forceinline__ void merge_aggregated(const float (*s_tile)[TILE + 1]
 				fw[q] = 0.;
 			base = -1 - lane;    // a group of its own
 		}
-		const double wv = views_final ? (double)s_tile[i][j] / cr : ((double)s_tile[i][j] / ps) / cr;
+		const double wv = views_final ? (double)tv * icr : (double)tv * ips * icr;
 		const unsigned grp = __match_any_sync(FULL, base);
-		const int members = __popc(grp);
-		const int most = (int)__reduce_max_sync(FULL, (unsigned)members);
+		const int most = (int)__reduce_max_sync(FULL, (unsigned)__popc(grp));
 		const bool lead = ok && (__ffs(grp) - 1) == lane;
-		double *a = accum + 2 * ((size_t)s_mode[j] * V + (ok ? base : 0));
-		// model sums (slot 0), then with_weight the weights (slot 1): the
+		const long long pbase = __shfl_xor_sync(FULL, base, 1);
+		const bool plead = __shfl_xor_sync(FULL, (int)lead, 1) != 0;
+		// first the even lane's corners, then the odd one's
+		const bool on0 = odd ? plead : lead, on1 = odd ? lead : plead;
+		double *const mode0 = accum + (size_t)s_mode[j] * V + (odd ? 1 : 0);
+		// model sums (plane 0), then with_weight the weights (plane 1): the
 		// group's lanes in lane order, summed by the lowest lane
 		for (int h = 0; h < (with_weight ? 2 : 1); ++h) {
 			double v[8];
 #pragma unroll
-			for (int q = 0; q < NC; ++q)
+			for (int q = 0; q < NC; ++q) {
 				v[q] = h == 0 ? fw[q] * wv : fw[q];
+			}
+			unsigned rest = grp & (grp - 1u);   // the group without its lowest lane
 			for (int m = 1; m < most; ++m) {
 				// the group's m-th lane, or this lane when the group is smaller
-				const int src = m < members ? (int)__fns(grp, 0, m + 1) : lane;
+				const int src = rest ? __ffs(rest) - 1 : lane;
 #pragma unroll
 				for (int q = 0; q < NC; ++q) {
 					const double x = __shfl_sync(FULL, h == 0 ? fw[q] * wv : fw[q], src);
-					if (m < members)
+					if (rest)
 						v[q] += x;
 				}
+				rest &= rest - 1u;
 			}
-			if (lead) {
+			double *const a0 = mode0 + (odd ? pbase : base) + (size_t)h * n;
+			double *const a1 = mode0 + (odd ? base : pbase) + (size_t)h * n;
 #pragma unroll
-				for (int q = 0; q < NC; ++q)
-					atomicAdd(a + 2 * off(q) + h, v[q]);
+			for (int q = 0; q < NC; q += 2) {
+				const double x = __shfl_xor_sync(FULL, odd ? v[q] : v[q + 1], 1);
+				if (on0)
+					atomicAdd(a0 + off(q / 2), odd ? x : v[q]);
+				if (on1)
+					atomicAdd(a1 + off(q / 2), odd ? v[q + 1] : x);
 			}
 		}
 	}
@@ -1229,7 +1192,7 @@ __global__ void __launch_bounds__(256, 3) merge_kernel(const float *__restrict__
                                                      const double *__restrict__ qvals,
                                                      const double *__restrict__ corr,
                                                      const uint8_t *__restrict__ mask, int P, long long S,
-                                                     long long V, double *__restrict__ accum,
+                                                     long long V, long long n, double *__restrict__ accum,
                                                      const int *__restrict__ weight_flag,
                                                      int views_final, const signed char *__restrict__ wsign = nullptr) {
 	__shared__ double s_rot[TILE][9];
@@ -1244,7 +1207,8 @@ __global__ void __launch_bounds__(256, 3) merge_kernel(const float *__restrict__
 		int rr = r < R ? r : 0;
 		geo_setup<GEO>(quats, rr / M, s_rot[j]);
 		s_mode[j] = rr % M;
-		s_ps[j] = r < R ? psum_r[r] : 0.;
+		const double ps = r < R ? psum_r[r] : 0.;
+		s_ps[j] = ps > 0. ? fmax(fmin(1. / ps, DBL_MAX), DBL_MIN) : 0.;  // 0: not merged
 		if constexpr (INCR)
 			s_sg[j] = r < R ? wsign[r] : 0;
 	}
@@ -1254,7 +1218,7 @@ __global__ void __launch_bounds__(256, 3) merge_kernel(const float *__restrict__
 			int pp = p0 + row;
 			float v[LW];
 			if (pp < P) {
-				ld_row(T + ((size_t)rt * P + pp) * TILE + lane * LW, v);
+				ld_row_stream(T + ((size_t)rt * P + pp) * TILE + lane * LW, v);
 			} else {
 #pragma unroll
 				for (int k = 0; k < LW; ++k)
@@ -1268,14 +1232,14 @@ __global__ void __launch_bounds__(256, 3) merge_kernel(const float *__restrict__
 	__syncthreads();
 	const int i = t & (PB - 1), g = t >> 6, p = p0 + i;
 	if constexpr (!INCR) {
-		merge_aggregated<GEO>(s_tile, s_ps, s_rot, s_mode, i, g, p, P, qvals, corr, mask, S, V, accum,
+		merge_aggregated<GEO>(s_tile, s_ps, s_rot, s_mode, i, g, p, P, qvals, corr, mask, S, V, n, accum,
 		                      with_weight, views_final);
 		return;
 	}
 	if (p >= P || mask[p] > 1)
 		return;
 	const double qx = qvals[3 * (size_t)p], qy = qvals[3 * (size_t)p + 1], qz = qvals[3 * (size_t)p + 2];
-	const double cr = corr[p];
+	const double icr = 1. / corr[p];
 	const double center = (double)(S / 2);
 	constexpr int NC = GEO == MT_3D ? 8 : 4;  // corners
 	long long o[8];
@@ -1286,17 +1250,11 @@ __global__ void __launch_bounds__(256, 3) merge_kernel(const float *__restrict__
 	}
 	for (int k = 0; k < TILE / 4; ++k) {
 		const int j = g + 4 * k;
-		const double ps = s_ps[j];
-		bool model = ps > 0.;
-		int sg = 0;
-		if constexpr (INCR) {
-			sg = s_sg[j];
-			model = model && s_tile[i][j] != 0.f;
-			if (!model && sg == 0)
-				continue;
-		} else if (!model) {
+		const double ips = s_ps[j];
+		const bool model = ips > 0. && s_tile[i][j] != 0.f;
+		const int sg = INCR ? s_sg[j] : 0;
+		if (!model && sg == 0)
 			continue;
-		}
 		double fw[8];
 		long long base;
 		if constexpr (GEO == MT_3D) {
@@ -1312,32 +1270,17 @@ __global__ void __launch_bounds__(256, 3) merge_kernel(const float *__restrict__
 			corner_weights2(c, fw);
 			base = c.i00;
 		}
-		double *a = accum + 2 * ((size_t)s_mode[j] * V + base);
-		if constexpr (INCR) {
-			if (model) {
-				const double wv = ((double)s_tile[i][j] / ps) / cr;
-#pragma unroll
-				for (int q = 0; q < NC; ++q)
-					atomicAdd(a + 2 * o[q], fw[q] * wv);
-			}
-			if (sg != 0) {
-#pragma unroll
-				for (int q = 0; q < NC; ++q)
-					atomicAdd(a + 2 * o[q] + 1, sg > 0 ? fw[q] : -fw[q]);
-			}
-			continue;
-		}
-		const double wv = views_final ? (double)s_tile[i][j] / cr : ((double)s_tile[i][j] / ps) / cr;
-		if (with_weight) {
-#pragma unroll
-			for (int q = 0; q < NC; ++q) {
-				atomicAdd(a + 2 * o[q], fw[q] * wv);
-				atomicAdd(a + 2 * o[q] + 1, fw[q]);
-			}
-		} else {
+		double *a = accum + (size_t)s_mode[j] * V + base;
+		if (model) {
+			const double wv = (double)s_tile[i][j] * ips * icr;
 #pragma unroll
 			for (int q = 0; q < NC; ++q)
-				atomicAdd(a + 2 * o[q], fw[q] * wv);
+				atomicAdd(a + o[q], fw[q] * wv);
+		}
+		if (sg != 0) {
+#pragma unroll
+			for (int q = 0; q < NC; ++q)
+				atomicAdd(a + n + o[q], sg > 0 ? fw[q] : -fw[q]);
 		}
 	}
 }
@@ -1390,20 +1333,20 @@ __global__ void __launch_bounds__(1024) weight_sign_kernel(const double *__restr
 // model2 / inter_weight from the accumulators; the weights come from this
 // merge (flag 1), from weight_cache (flag 0) or from weight_cache plus this
 // merge's change (flag 2); weight_cache keeps the result.
-__global__ void unpack_accum_kernel(const double2 *__restrict__ accum, long long n, double *__restrict__ model2,
+__global__ void unpack_accum_kernel(const double *__restrict__ accum, long long n, double *__restrict__ model2,
                                     double *__restrict__ weight, double *__restrict__ weight_cache,
                                     const int *__restrict__ weight_flag) {
 	long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n)
 		return;
 	const int with_weight = *weight_flag;
-	double2 a = accum[i];
-	model2[i] = a.x;
+	model2[i] = accum[i];
 	if (with_weight == 1) {
-		weight[i] = a.y;
-		weight_cache[i] = a.y;
+		const double w = accum[n + i];
+		weight[i] = w;
+		weight_cache[i] = w;
 	} else if (with_weight == 2) {
-		const double w = weight_cache[i] + a.y;
+		const double w = weight_cache[i] + accum[n + i];
 		weight[i] = w;
 		weight_cache[i] = w;
 	} else {

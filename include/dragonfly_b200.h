@@ -448,7 +448,7 @@ DFG_API int dfg_save_emc(dfg_ctx *ctx, const char *path);
  * "keep_prob" (1: keep the sparse probability lists), "graph" (1: capture
  * iterations as CUDA graphs), "autotune" (1: time the kernel forms on the
  * inputs and keep the fastest), "estep_form" / "mstep_form" (0 sparse, 1
- * tensor-core products), "slice_block" (orientations per slice block, 0
+ * tensor-core products), "slice_block" (orientations per slice block: 8, 16, 32, 64 or 128; 0
  * automatic), "tile_skip" (skip dead (tile, frame) pairs without
  * refinement), "pair_lists" (1: restricted searches store only their live
  * (tile, frame) pairs, orientations in blocks), "block_budget_mb" (device
