@@ -1253,8 +1253,9 @@ static int hot_choose(dfg_ctx *ctx) {
 		ch.by_frame.release();
 		ch.by_pixel.release();
 		ch.pix_cold.release();
+		ch.csc.release();
 	}
-	if (TILE != 128 || ctx->chunk_frames < HM || ctx->max_fcount >= kHotMaxSum)
+	if (TILE != 128 || ctx->RT > 65535 || ctx->chunk_frames < HM || ctx->max_fcount >= kHotMaxSum)
 		return DFG_OK;
 	std::vector<int> cand;
 	for (int p = 0; p < P; ++p)
@@ -1313,42 +1314,73 @@ static int hot_choose(dfg_ctx *ctx) {
 		CK(upload(ch.pix_cold, rest.data(), rest.size(), st));
 		CK(cudaStreamSynchronize(st));
 	}
-	// the E-step's lists without the hot pixels
+	// the photon lists without the hot pixels: per frame, and per chunk and pixel
 	DevBuf<int2> cnt;
-	std::vector<int2> h((size_t)N);
-	std::vector<long long> off((size_t)N + 1, 0), mid((size_t)N);
-	if (room) {
-		CK(cnt.ensure((size_t)N));
-		cold_count_kernel<<<blocks_for((long long)N * 32, 256), 256, 0, st>>>(ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p,
-		                                                                      N, P, ctx->is_hot.p, cnt.p);
-		CKL("cold_count_kernel");
-		CK(cudaMemcpyAsync(h.data(), cnt.p, (size_t)N * sizeof(int2), cudaMemcpyDeviceToHost, st));
-		CK(cudaStreamSynchronize(st));
-		for (int d = 0; d < N; ++d) {
+	std::vector<int2> h;
+	std::vector<long long> off, mid;
+	auto lay_out = [&](int lists) {
+		off.assign((size_t)lists + 1, 0);
+		mid.assign((size_t)lists, 0);
+		for (int d = 0; d < lists; ++d) {
 			mid[d] = off[d] + (h[d].x + 7) / 8 * 8;
 			off[d + 1] = mid[d] + (h[d].y + 7) / 8 * 8;
 		}
+	};
+	if (room) {
+		CK(cnt.ensure((size_t)std::max(N, P)));
+		h.resize((size_t)N);
+		cold_count_kernel<false><<<blocks_for((long long)N * 32, 256), 256, 0, st>>>(
+		    ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p, N, (uint32_t)P, ctx->is_hot.p, cnt.p);
+		CKL("cold_count_kernel");
+		CK(cudaMemcpyAsync(h.data(), cnt.p, (size_t)N * sizeof(int2), cudaMemcpyDeviceToHost, st));
+		CK(cudaStreamSynchronize(st));
+		lay_out(N);
 		const cudaError_t e = fits(ctx->phc.ensure((size_t)off[N]));
-		if (e != cudaErrorMemoryAllocation)
+		room = e != cudaErrorMemoryAllocation;
+		if (room) {
 			CK(e);
-		else
-			room = false;
+			CK(upload(ctx->phc_off, off.data(), off.size(), st));
+			CK(upload(ctx->phc_mid, mid.data(), mid.size(), st));
+			cold_write_kernel<false><<<blocks_for((long long)N * 32, 256), 256, 0, st>>>(
+			    ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p, N, (uint32_t)P, (uint32_t)P, ctx->is_hot.p, ctx->phc_off.p,
+			    ctx->phc_mid.p, ctx->phc.p);
+			CKL("cold_write_kernel");
+			CK(cudaStreamSynchronize(st));
+		}
+	}
+	h.resize((size_t)P);
+	for (Chunk &ch : ctx->chunks) {
+		if (!room)
+			break;
+		cold_count_kernel<true><<<blocks_for((long long)P * 32, 256), 256, 0, st>>>(
+		    ch.cs.p, ch.cs_off.p, ch.cs_mid.p, P, (uint32_t)ch.nc, ctx->is_hot.p, cnt.p);
+		CKL("cold_count_kernel");
+		CK(cudaMemcpyAsync(h.data(), cnt.p, (size_t)P * sizeof(int2), cudaMemcpyDeviceToHost, st));
+		CK(cudaStreamSynchronize(st));
+		lay_out(P);
+		const cudaError_t e = fits(ch.csc.ensure((size_t)off[P]));
+		room = e != cudaErrorMemoryAllocation;
+		if (room) {
+			CK(e);
+			CK(upload(ch.csc_off, off.data(), off.size(), st));
+			CK(upload(ch.csc_mid, mid.data(), mid.size(), st));
+			cold_write_kernel<true><<<blocks_for((long long)P * 32, 256), 256, 0, st>>>(
+			    ch.cs.p, ch.cs_off.p, ch.cs_mid.p, P, (uint32_t)ch.nc, (uint32_t)ch.nc, ctx->is_hot.p, ch.csc_off.p,
+			    ch.csc_mid.p, ch.csc.p);
+			CKL("cold_write_kernel");
+			CK(cudaStreamSynchronize(st));
+		}
 	}
 	if (!room) {
+		ctx->phc.release();
 		for (Chunk &ch : ctx->chunks) {
 			ch.by_frame.release();
 			ch.by_pixel.release();
 			ch.pix_cold.release();
+			ch.csc.release();
 		}
 		return DFG_OK;
 	}
-	CK(upload(ctx->phc_off, off.data(), off.size(), st));
-	CK(upload(ctx->phc_mid, mid.data(), mid.size(), st));
-	cold_write_kernel<<<blocks_for((long long)N * 32, 256), 256, 0, st>>>(ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p, N,
-	                                                                      P, ctx->is_hot.p, ctx->phc_off.p,
-	                                                                      ctx->phc_mid.p, ctx->phc.p);
-	CKL("cold_write_kernel");
-	CK(cudaStreamSynchronize(st));
 	ctx->hot_n = n;
 	ctx->hot_pitch = pitch;
 	return DFG_OK;
@@ -1665,14 +1697,15 @@ static int launch_mstep(dfg_ctx *ctx, const Chunk &ch, bool dense) {
 			return rc;
 	const int npix = hot ? ch.npix_cold : ch.npix;
 	const int *pix = hot ? ch.pix_cold.p : ch.pix.p;
+	const uint32_t *cs = hot ? ch.csc.p : ch.cs.p;
+	const long long *cs_off = hot ? ch.csc_off.p : ch.cs_off.p, *cs_mid = hot ? ch.csc_mid.p : ch.cs_mid.p;
 	if (npix > 0) {
 		const long long warps = (long long)RT * npix;
 		const int minb = ctx->tuning ? ctx->tune_mstep_minb
 		                             : (ctx->mstep_minb > 0 ? ctx->mstep_minb : ctx->tuned_mstep_minb);
 #define DFG_MSTEP(SK, MB)                                                                                     \
-	mstep_kernel<SK, MB><<<blocks_for(warps, 8), 256, 0, st>>>(ctx->Pst.p, Nc, ch.cs.p, ch.cs_off.p,           \
-	                                                           ch.cs_mid.p, pix, npix, P, RT, ctx->T.p,          \
-	                                                           ctx->tlive.p)
+	mstep_kernel<SK, MB><<<blocks_for(warps, 8), 256, 0, st>>>(ctx->Pst.p, Nc, cs, cs_off, cs_mid, pix, npix, P,   \
+	                                                           RT, ctx->T.p, ctx->tlive.p)
 		if (tile_skipping(ctx))
 			DFG_MSTEP(true, MSTEP_MINB);
 		else if (minb == 3)
@@ -1711,31 +1744,36 @@ static int launch_estep(dfg_ctx *ctx, const Chunk &ch, int use_scale, bool bg, c
 	// blocks per SM: the autotuner's choice (or the option), else the default
 	const int minb = ctx->tuning ? ctx->tune_estep_minb : (ctx->estep_minb > 0 ? ctx->estep_minb
 	                                                                           : ctx->tuned_estep_minb);
-	const bool hot = ctx->hot_active && rm.qmap == nullptr;
-	const uint32_t *ph = hot ? ctx->phc.p : ctx->ph.p;
-	const long long *off = hot ? ctx->phc_off.p : ctx->ph_off.p, *mid = hot ? ctx->phc_mid.p : ctx->ph_mid.p;
-	const HotLists full{ctx->hot_special.p, ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p};
-	if (hot)
+	if (ctx->hot_active && rm.qmap == nullptr) {
 		if (int rc = launch_hot_estep(ctx, ch))
 			return rc;
-#define DFG_ESTEP(REF, MB, HOT)                                                                               \
-	estep_kernel<REF, MB, HOT><<<blocks_for(warps, 8), 256, 0, st>>>(                                         \
-	    ctx->logW.p, ctx->u.p, ctx->logw.p, R, ph, off, mid, ctx->scale.p, ctx->blacklist.p, ch.d0, Nc,        \
-	    use_scale, ctx->scalars.p, P, RT, ctx->pval.p, ctx->tmax.p, ctx->targ.p, rm, 0, full)
+		const HotLists full{ctx->hot_special.p, ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p};
+#define DFG_ECOLD(MB)                                                                                         \
+	estep_cold_kernel<MB><<<dim3(blocks_for(Nc, 8), RT), 256, 0, st>>>(                                       \
+	    ctx->logW.p, ctx->u.p, ctx->logw.p, R, ctx->phc.p, ctx->phc_off.p, ctx->phc_mid.p, ctx->scale.p,        \
+	    ctx->blacklist.p, ch.d0, Nc, use_scale, ctx->scalars.p, P, ctx->pval.p, ctx->tmax.p, ctx->targ.p, full)
+		if (minb == 2)
+			DFG_ECOLD(2);
+		else if (minb == 3)
+			DFG_ECOLD(3);
+		else
+			DFG_ECOLD(4);
+#undef DFG_ECOLD
+		CKL("estep_cold_kernel");
+		return DFG_OK;
+	}
+#define DFG_ESTEP(REF, MB)                                                                                    \
+	estep_kernel<REF, MB><<<blocks_for(warps, 8), 256, 0, st>>>(                                              \
+	    ctx->logW.p, ctx->u.p, ctx->logw.p, R, ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p, ctx->scale.p,          \
+	    ctx->blacklist.p, ch.d0, Nc, use_scale, ctx->scalars.p, P, RT, ctx->pval.p, ctx->tmax.p, ctx->targ.p, rm)
 	if (rm.qmap != nullptr)
-		DFG_ESTEP(true, ESTEP_MINB, false);
-	else if (hot && minb == 2)
-		DFG_ESTEP(false, 2, true);
-	else if (hot && minb == 4)
-		DFG_ESTEP(false, 4, true);
-	else if (hot)
-		DFG_ESTEP(false, ESTEP_MINB, true);
+		DFG_ESTEP(true, ESTEP_MINB);
 	else if (minb == 2)
-		DFG_ESTEP(false, 2, false);
+		DFG_ESTEP(false, 2);
 	else if (minb == 4)
-		DFG_ESTEP(false, 4, false);
+		DFG_ESTEP(false, 4);
 	else
-		DFG_ESTEP(false, ESTEP_MINB, false);
+		DFG_ESTEP(false, ESTEP_MINB);
 #undef DFG_ESTEP
 	CKL("estep_kernel");
 	return DFG_OK;

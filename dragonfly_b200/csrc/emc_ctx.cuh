@@ -101,6 +101,8 @@ struct Chunk {
 	// that of the chunk's probability digits, and the pixels left to the gathers
 	DevBuf<uint8_t> by_frame, by_pixel;
 	DevBuf<int> pix_cold;
+	DevBuf<uint32_t> csc;      // their frame lists
+	DevBuf<long long> csc_off, csc_mid;
 	int npix_cold = 0, k_pitch = 0;
 	CUtensorMap map_frame, map_pixel, map_pdig;
 };

@@ -222,22 +222,13 @@ __device__ __forceinline__ void refine_skip_tile(double *__restrict__ tmax, int 
 	}
 }
 
-// HOT: the photons of the hot pixels are already in pval as FP64 sums
-// (emc_hot.cuh), the lists hold the others; a tile marked special gathers all of
-// its photons (full) instead.
-struct HotLists {
-	const int *special;          // [RT]
-	const uint32_t *ph;          // every photon's lists
-	const long long *off, *mid;
-};
-
-template <bool REFINE, int MINB = ESTEP_MINB, bool HOT = false>
+template <bool REFINE, int MINB = ESTEP_MINB>
 __global__ void __launch_bounds__(256, MINB) estep_kernel(
     const float *__restrict__ logW, const double *__restrict__ u, const double *__restrict__ logw, int R,
     const uint32_t *__restrict__ ph, const long long *__restrict__ ph_off, const long long *__restrict__ ph_mid,
     const double *__restrict__ scale, const uint8_t *__restrict__ blacklist, int d0, int Nc, int use_scale,
     const double *__restrict__ scalars, int P, int RT, double *__restrict__ pval, double *__restrict__ tmax,
-    int *__restrict__ targ, RefineMask rm, int t0 = 0, HotLists full = {}) {
+    int *__restrict__ targ, RefineMask rm, int t0 = 0) {
 	// RT tiles from tile t0 (orientation blocks: logW holds tiles t0 ..)
 	const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const int lane = threadIdx.x & 31;
@@ -256,15 +247,6 @@ __global__ void __launch_bounds__(256, MINB) estep_kernel(
 		}
 	}
 	const float *L = logW + (size_t)rl * (P + 1) * TILE + lane * LW;
-	bool add_hot = HOT;
-	if constexpr (HOT) {
-		if (full.special[rt]) {
-			ph = full.ph;
-			ph_off = full.off;
-			ph_mid = full.mid;
-			add_hot = false;
-		}
-	}
 	const long long beg = ph_off[d], mid = ph_mid[d], end = ph_off[d + 1];
 	// segments start at multiples of 8 words: two 16-byte loads, identical for
 	// every lane (broadcast), bring 8 photon words
@@ -315,13 +297,7 @@ __global__ void __launch_bounds__(256, MINB) estep_kernel(
 				kahan_add_count(s[q % ECH][k], c[q % ECH][k], e[q] >> IDX_BITS, v[q][k]);
 	}
 	const double sd = use_scale ? scale[d] : scalars[0];
-	double acc[LW], hot[LW];
-	if constexpr (HOT) {
-		const double *h = pval + ((size_t)rt * Nc + dl) * TILE + lane * LW;
-#pragma unroll
-		for (int k = 0; k < LW; ++k)
-			hot[k] = add_hot ? h[k] : 0.;
-	}
+	double acc[LW];
 	// tile maximum and its lowest orientation index (strict > in ascending r,
 	// as the running maximum of max_prob.c:199-202)
 	double m = MAX_EXP_START;
@@ -334,8 +310,6 @@ __global__ void __launch_bounds__(256, MINB) estep_kernel(
 			double ph_sum = kahan_value(s[0][k], c[0][k]);
 			if (ECH == 2)
 				ph_sum = dadd(ph_sum, kahan_value(s[ECH - 1][k], c[ECH - 1][k]));
-			if (HOT)
-				ph_sum = dadd(ph_sum, hot[k]);
 			acc[k] = dadd(dsub(logw[r], dmul(u[r], sd)), ph_sum);
 			if (REFINE && !(live >> k & 1u))
 				acc[k] = -INFINITY;
@@ -350,6 +324,128 @@ __global__ void __launch_bounds__(256, MINB) estep_kernel(
 	for (int o = 16; o > 0; o >>= 1) {
 		double om = __shfl_xor_sync(FULL, m, o);
 		int oa = __shfl_xor_sync(FULL, am, o);
+		if (om > m || (om == m && oa >= 0 && (am < 0 || oa < am))) {
+			m = om;
+			am = oa;
+		}
+	}
+	if (lane == 0) {
+		tmax[(size_t)rt * Nc + dl] = m;
+		targ[(size_t)rt * Nc + dl] = am;
+	}
+}
+
+// The E-step's end where the hot pixels' photon sums are already in pval
+// (emc_hot.cuh): the other photons are gathered as in estep_kernel, and the
+// log-likelihood formed. A tile marked special gathers all of its photons (full)
+// instead. The lists are short (tens of rows), so what a warp spends outside
+// the rows counts: the grid gives tile and frame without a division, the frame's
+// partial sums and the orientations' constants come as one 32-byte load per lane,
+// and two orientations share each compensated addition (the kernel is bound by issue and
+// the L2 path about equally).
+struct HotLists {
+	const int *special;          // [RT]
+	const uint32_t *ph;          // every photon's lists
+	const long long *off, *mid;
+};
+
+template <int MINB>
+__global__ void __launch_bounds__(256, MINB) estep_cold_kernel(
+    const float *__restrict__ logW, const double *__restrict__ u, const double *__restrict__ logw, int R,
+    const uint32_t *__restrict__ ph, const long long *__restrict__ ph_off, const long long *__restrict__ ph_mid,
+    const double *__restrict__ scale, const uint8_t *__restrict__ blacklist, int d0, int Nc, int use_scale,
+    const double *__restrict__ scalars, int P, double *pval, double *__restrict__ tmax, int *__restrict__ targ,
+    HotLists full) {
+	static_assert(LW == 4, "the products need 128-orientation tiles");
+	const int rt = blockIdx.y, dl = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, d = d0 + dl;
+	if (dl >= Nc || blacklist[d])
+		return;
+	const bool special = full.special[rt] != 0;
+	if (special) {
+		ph = full.ph;
+		ph_off = full.off;
+		ph_mid = full.mid;
+	}
+	const long long beg = ph_off[d], mid = ph_mid[d], end = ph_off[d + 1];
+	const float *L = logW + (size_t)rt * (P + 1) * TILE + lane * LW;
+	double *const row = pval + ((size_t)rt * Nc + dl) * TILE + lane * LW;
+	const uint4 *w4 = reinterpret_cast<const uint4 *>(ph);
+	f32x2 s[NPAIR], c[NPAIR];
+#pragma unroll
+	for (int h = 0; h < NPAIR; ++h)
+		s[h] = c[h] = 0ull;
+	uint4 a = make_uint4(P, P, P, P), b = a;
+	if (beg < mid) {
+		a = __ldg(w4 + (beg >> 2));
+		b = __ldg(w4 + (beg >> 2) + 1);
+	}
+	for (long long j = beg; j < mid; j += 8) {
+		f32x2 v[8][NPAIR];
+		ld_pairs(L + a.x * TILE, v[0]);
+		ld_pairs(L + a.y * TILE, v[1]);
+		ld_pairs(L + a.z * TILE, v[2]);
+		ld_pairs(L + a.w * TILE, v[3]);
+		ld_pairs(L + b.x * TILE, v[4]);
+		ld_pairs(L + b.y * TILE, v[5]);
+		ld_pairs(L + b.z * TILE, v[6]);
+		ld_pairs(L + b.w * TILE, v[7]);
+		if (j + 8 < mid) {
+			a = __ldg(w4 + ((j + 8) >> 2));
+			b = __ldg(w4 + ((j + 8) >> 2) + 1);
+		}
+#pragma unroll
+		for (int q = 0; q < 8; ++q)
+#pragma unroll
+			for (int h = 0; h < NPAIR; ++h)
+				kahan_add2(s[h], c[h], v[q][h]);
+	}
+	for (long long j = mid; j < end; j += 8) {
+		const uint4 x = __ldg(w4 + (j >> 2)), y = __ldg(w4 + (j >> 2) + 1);
+		const uint32_t e[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+		f32x2 v[8][NPAIR];
+#pragma unroll
+		for (int q = 0; q < 8; ++q)
+			ld_pairs(L + (e[q] & IDX_MASK) * TILE, v[q]);
+#pragma unroll
+		for (int q = 0; q < 8; ++q)
+#pragma unroll
+			for (int h = 0; h < NPAIR; ++h)
+				kahan_add_count2(s[h], c[h], e[q] >> IDX_BITS, v[q][h]);
+	}
+	double hot[LW], ur[LW], lw[LW], acc[LW];
+	asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+	             : "=d"(hot[0]), "=d"(hot[1]), "=d"(hot[2]), "=d"(hot[3])
+	             : "l"(row));
+	const int r0 = rt * TILE + lane * LW;
+	ld_row32(u + r0, ur);
+	ld_row32(logw + r0, lw);
+	const double sd = use_scale ? scale[d] : scalars[0];
+	double m = MAX_EXP_START;
+	int am = -1;
+#pragma unroll
+	for (int k = 0; k < LW; ++k) {
+		float slo, shi, clo, chi;
+		f2_unpack(s[k / 2], slo, shi);
+		f2_unpack(c[k / 2], clo, chi);
+		double sum = k & 1 ? kahan_value(shi, chi) : kahan_value(slo, clo);
+		if (!special)
+			sum = dadd(sum, hot[k]);
+		acc[k] = 0.;
+		if (r0 + k < R) {
+			acc[k] = dadd(dsub(lw[k], dmul(ur[k], sd)), sum);
+			if (acc[k] > m) {
+				m = acc[k];
+				am = r0 + k;
+			}
+		}
+	}
+	asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(row), "d"(acc[0]), "d"(acc[1]), "d"(acc[2]),
+	             "d"(acc[3])
+	             : "memory");
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) {
+		const double om = __shfl_xor_sync(FULL, m, o);
+		const int oa = __shfl_xor_sync(FULL, am, o);
 		if (om > m || (om == m && oa >= 0 && (am < 0 || oa < am))) {
 			m = om;
 			am = oa;

@@ -424,58 +424,84 @@ __global__ void __launch_bounds__(256) hot_counts_kernel(const uint32_t *__restr
 	}
 }
 
-// The E-step's photon lists without the hot pixels, in two passes: the words
-// that stay in each frame's two segments (counts), then the lists, each
-// segment padded to 8 words with the zero row. One warp per frame.
-__device__ __forceinline__ bool cold_word(uint32_t w, bool multi, int P, const uint8_t *__restrict__ is_hot) {
-	const uint32_t p = multi ? (w & IDX_MASK) : w;
-	return p < (uint32_t)P && !is_hot[p];
+// The photon lists without the hot pixels, in two passes: the words of each
+// list's two segments (counts), then the lists, each segment padded to 8 words
+// with `pad`. A count of up to COLD_REPEAT becomes that many count-1 words: the
+// few such photons of a cold pixel would take a segment of their own, padded to 8
+// rows. One warp per list. BY_LIST false: lists of pixels per frame (E-step), hot
+// words dropped; true: lists of frames per pixel (M-step), hot lists dropped.
+// Words naming `limit` or above are padding.
+constexpr uint32_t COLD_REPEAT = 4;
+
+// (count-1 words, counted words) that word w of a list contributes
+template <bool BY_LIST>
+__device__ __forceinline__ int2 cold_words(uint32_t w, bool multi, uint32_t limit, const uint8_t *__restrict__ is_hot) {
+	const uint32_t idx = multi ? (w & IDX_MASK) : w, c = multi ? (w >> IDX_BITS) : 1u;
+	if (idx >= limit || (!BY_LIST && is_hot[idx]))
+		return make_int2(0, 0);
+	return c <= COLD_REPEAT ? make_int2((int)c, 0) : make_int2(0, 1);
 }
 
-__global__ void __launch_bounds__(256) cold_count_kernel(const uint32_t *__restrict__ ph,
+template <bool BY_LIST>
+__global__ void __launch_bounds__(256) cold_count_kernel(const uint32_t *__restrict__ words,
                                                          const long long *__restrict__ off,
-                                                         const long long *__restrict__ mid, int N, int P,
-                                                         const uint8_t *__restrict__ is_hot, int2 *__restrict__ n) {
+                                                         const long long *__restrict__ mid, int n, uint32_t limit,
+                                                         const uint8_t *__restrict__ is_hot, int2 *__restrict__ out) {
 	const int d = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-	if (d >= N)
+	if (d >= n)
 		return;
 	int a = 0, b = 0;
-	for (long long j = off[d] + lane; j < mid[d]; j += 32)
-		a += cold_word(ph[j], false, P, is_hot);
-	for (long long j = mid[d] + lane; j < off[d + 1]; j += 32)
-		b += cold_word(ph[j], true, P, is_hot);
+	if (!BY_LIST || !is_hot[d])
+		for (long long j = off[d] + lane; j < off[d + 1]; j += 32) {
+			const int2 k = cold_words<BY_LIST>(words[j], j >= mid[d], limit, is_hot);
+			a += k.x;
+			b += k.y;
+		}
 	a = __reduce_add_sync(FULL, a);
 	b = __reduce_add_sync(FULL, b);
 	if (lane == 0)
-		n[d] = make_int2(a, b);
+		out[d] = make_int2(a, b);
 }
 
-__global__ void __launch_bounds__(256) cold_write_kernel(const uint32_t *__restrict__ ph,
+__device__ __forceinline__ int warp_prefix(int x, int lane) {  // inclusive
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const int y = __shfl_up_sync(FULL, x, o);
+		if (lane >= o)
+			x += y;
+	}
+	return x;
+}
+
+template <bool BY_LIST>
+__global__ void __launch_bounds__(256) cold_write_kernel(const uint32_t *__restrict__ words,
                                                          const long long *__restrict__ off,
-                                                         const long long *__restrict__ mid, int N, int P,
-                                                         const uint8_t *__restrict__ is_hot,
+                                                         const long long *__restrict__ mid, int n, uint32_t limit,
+                                                         uint32_t pad, const uint8_t *__restrict__ is_hot,
                                                          const long long *__restrict__ coff,
                                                          const long long *__restrict__ cmid,
                                                          uint32_t *__restrict__ out) {
 	const int d = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-	if (d >= N)
+	if (d >= n || coff[d + 1] == coff[d])
 		return;
-	for (int seg = 0; seg < 2; ++seg) {
-		const long long b = seg ? mid[d] : off[d], e = seg ? off[d + 1] : mid[d];
-		long long at = seg ? cmid[d] : coff[d];
-		const long long stop = seg ? coff[d + 1] : cmid[d];
-		for (long long j0 = b; j0 < e; j0 += 32) {
-			const long long j = j0 + lane;
-			const uint32_t w = j < e ? ph[j] : (uint32_t)P;
-			const bool keep = j < e && cold_word(w, seg != 0, P, is_hot);
-			const unsigned m = __ballot_sync(FULL, keep);
-			if (keep)
-				out[at + __popc(m & ((1u << lane) - 1u))] = w;
-			at += __popc(m);
-		}
-		for (long long j = at + lane; j < stop; j += 32)
-			out[j] = (uint32_t)P;
+	long long at1 = coff[d], atm = cmid[d];
+	for (long long j0 = off[d]; j0 < off[d + 1]; j0 += 32) {
+		const long long j = j0 + lane;
+		const bool multi = j >= mid[d];
+		const uint32_t w = j < off[d + 1] ? words[j] : 0u;
+		const int2 k = j < off[d + 1] ? cold_words<BY_LIST>(w, multi, limit, is_hot) : make_int2(0, 0);
+		const int p1 = warp_prefix(k.x, lane), pm = warp_prefix(k.y, lane);
+		for (int c = 0; c < k.x; ++c)
+			out[at1 + p1 - k.x + c] = multi ? (w & IDX_MASK) : w;
+		if (k.y)
+			out[atm + pm - 1] = w;
+		at1 += __shfl_sync(FULL, p1, 31);
+		atm += __shfl_sync(FULL, pm, 31);
 	}
+	for (long long j = at1 + lane; j < cmid[d]; j += 32)
+		out[j] = pad;
+	for (long long j = atm + lane; j < coff[d + 1]; j += 32)
+		out[j] = pad;
 }
 
 }  // namespace dfg
