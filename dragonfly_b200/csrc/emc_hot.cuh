@@ -78,21 +78,18 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 	asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-// 16 TMEM columns of this thread's lane, without waiting for them.
-__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
-	asm volatile(
-	    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-	    "%14, %15}, [%16];"
-	    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-	      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-	    : "r"(taddr));
+// 8 TMEM columns of this thread's lane, without waiting for them.
+__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t (&r)[8]) {
+	asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+	             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+	             : "r"(taddr));
 }
-// Orders the uses of r after the wait for the loads into it.
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&a)[16], uint32_t (&b)[16], uint32_t (&c)[16],
-                                             uint32_t (&d)[16]) {
+// Orders the uses of the loaded columns after the wait for them.
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&a)[8], uint32_t (&b)[8], uint32_t (&c)[8],
+                                             uint32_t (&d)[8]) {
 	asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-	for (int k = 0; k < 16; ++k)
+	for (int k = 0; k < 8; ++k)
 		asm volatile("" : "+r"(a[k]), "+r"(b[k]), "+r"(c[k]), "+r"(d[k]));
 }
 
@@ -264,25 +261,32 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 				tp = out.T + ((size_t)rt * out.P + (valid ? out.pix[row] : 0)) * TILE + j0;
 			else
 				pv = out.pval + ((size_t)rt * nrows + (valid ? row : 0)) * TILE + j0;
-#pragma unroll 1
-			for (int c = 0; c < HO / 16; ++c) {
-				uint32_t d0[16], d1[16], d2[16], d3[16];
-				tmem_ld16_issue(base + c * 16, d0);
-				tmem_ld16_issue(base + HO + c * 16, d1);
-				tmem_ld16_issue(base + 2 * HO + c * 16, d2);
-				tmem_ld16_issue(base + 3 * HO + c * 16, d3);
-				tmem_ld_wait(d0, d1, d2, d3);
-				if (c == HO / 16 - 1) {  // the accumulator may be overwritten from here on
-					tc_fence_before();
-					__syncwarp();
-					if (lane == 0)
-						mbar_arrive(tempty);
-				}
-				if (MSTEP && valid) {
-					const float *rm = out.rmax + (size_t)rt * TILE + j0 + c * 16;
+			// all sums into registers first, so that the next tile's products
+			// run while this one's results are stored (the stores alone take about
+			// 10000 cycles a tile, as long as the products over 1250 pixels)
+			double v[HO];
 #pragma unroll
-					for (int k = 0; k < 16; k += 4) {
-						float4 *dst = reinterpret_cast<float4 *>(tp + c * 16 + k);
+			for (int c = 0; c < HO / 8; ++c) {
+				uint32_t d0[8], d1[8], d2[8], d3[8];
+				tmem_ld8_issue(base + c * 8, d0);
+				tmem_ld8_issue(base + HO + c * 8, d1);
+				tmem_ld8_issue(base + 2 * HO + c * 8, d2);
+				tmem_ld8_issue(base + 3 * HO + c * 8, d3);
+				tmem_ld_wait(d0, d1, d2, d3);
+#pragma unroll
+				for (int k = 0; k < 8; ++k)
+					v[c * 8 + k] = join_digits(d0[k], d1[k], d2[k], d3[k]);
+			}
+			tc_fence_before();
+			__syncwarp();
+			if (lane == 0)
+				mbar_arrive(tempty);
+			if (valid) {
+				if constexpr (MSTEP) {
+					const float *rm = out.rmax + (size_t)rt * TILE + j0;
+#pragma unroll
+					for (int k = 0; k < HO; k += 4) {
+						float4 *dst = reinterpret_cast<float4 *>(tp + k);
 						const float4 r4 = __ldg(reinterpret_cast<const float4 *>(rm + k));
 						const float rr[4] = {r4.x, r4.y, r4.z, r4.w};
 						float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -291,26 +295,19 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 						float o[4] = {o4.x, o4.y, o4.z, o4.w};
 #pragma unroll
 						for (int e = 0; e < 4; ++e)
-							o[e] = (float)((double)o[e] + join_digits(d0[k + e], d1[k + e], d2[k + e], d3[k + e]) *
-							                                  ((double)rr[e] * (1. / HP_STEPS)));
+							o[e] = (float)((double)o[e] + v[k + e] * ((double)rr[e] * (1. / HP_STEPS)));
 						*dst = make_float4(o[0], o[1], o[2], o[3]);
 					}
-				}
-				if (!MSTEP && valid) {
+				} else {
 #pragma unroll
-					for (int k = 0; k < 16; k += 4) {
-						double v[4];
-#pragma unroll
-						for (int e = 0; e < 4; ++e)
-							v[e] = join_digits(d0[k + e], d1[k + e], d2[k + e], d3[k + e]) * (1. / HE_SCALE);
-						// 32 bytes per lane: a whole sector in one store
-						asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(pv + c * 16 + k), "d"(v[0]),
-						             "d"(v[1]), "d"(v[2]), "d"(v[3])
+					for (int k = 0; k < HO; k += 4)  // 32 bytes per lane: a whole sector in one store
+						asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(pv + k),
+						             "d"(v[k] * (1. / HE_SCALE)), "d"(v[k + 1] * (1. / HE_SCALE)),
+						             "d"(v[k + 2] * (1. / HE_SCALE)), "d"(v[k + 3] * (1. / HE_SCALE))
 						             : "memory");
-					}
 				}
-				__syncwarp();
 			}
+			__syncwarp();
 		}
 	}
 	tc_fence_before();
