@@ -1833,6 +1833,29 @@ static int launch_psum(dfg_ctx *ctx, const Chunk &ch, int need_scaling) {
 	return DFG_OK;
 }
 
+// Merge of the tiles [t0, t0 + nt), whose tomograms are T's tiles 0 ..
+static int launch_merge(dfg_ctx *ctx, const float *T, int t0, int nt, int views_final) {
+	const int r0 = t0 * TILE, Rb = std::min(ctx->R - r0, nt * TILE);
+	const bool two_d = ctx->model_type == MT_2D;
+	const double *geo = two_d ? ctx->cs2d.p : ctx->quats.p + 5 * (size_t)r0;
+	const unsigned nb = blocks_for(ctx->P, 32 * ML) * (unsigned)(nt * (TILE / MO));
+#define DFG_MERGE(G)                                                                                          \
+	do {                                                                                                      \
+		CK(cudaFuncSetAttribute(merge_runs_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,               \
+		                        (int)sizeof(MergeShared)));                                                   \
+		merge_runs_kernel<G><<<nb, 256, sizeof(MergeShared), ctx->stream>>>(                                   \
+		    T, ctx->psum_r.p + r0, geo, ctx->M, Rb, ctx->qvals.p, ctx->corr.p, ctx->mask.p, ctx->P, ctx->S,        \
+		    ctx->V, (long long)ctx->M * ctx->V, (double *)ctx->accum.p, ctx->wflags.p, views_final);            \
+	} while (0)
+	if (two_d)
+		DFG_MERGE(MT_2D);
+	else
+		DFG_MERGE(MT_3D);
+#undef DFG_MERGE
+	CKL("merge_runs_kernel");
+	return DFG_OK;
+}
+
 // Captured probability mass of the watched frames that lie in this chunk
 // (their chunk-local indices were uploaded by max_prepare).
 static int launch_watch(dfg_ctx *ctx, const Chunk &ch) {
@@ -2182,10 +2205,10 @@ static int max_enqueue_pairs(dfg_ctx *ctx, const dfg_iter_params *par) {
 		}
 		phase_end(ctx, PH_MSTEP, nq > 0 ? 1 : 0);
 		phase_begin(ctx, PH_MERGE);
-		merge_kernel<MT_3D, true><<<dim3(nblk, nt), 256, 0, st>>>(
-		    ctx->blk.p, ctx->psum_r.p + r0, ctx->quats.p + 5 * (size_t)r0, 1, Rb, ctx->qvals.p, ctx->corr.p,
-		    ctx->mask.p, P, S, V, (long long)M * V, (double *)ctx->accum.p, ctx->wflags.p, 0, ctx->wsign.p + r0);
-		CKL("merge_kernel");
+		merge_change_kernel<<<dim3(nblk, nt), 256, 0, st>>>(
+		    ctx->blk.p, ctx->psum_r.p + r0, ctx->quats.p + 5 * (size_t)r0, Rb, ctx->qvals.p, ctx->corr.p, ctx->mask.p,
+		    P, S, (long long)M * V, (double *)ctx->accum.p, ctx->wsign.p + r0);
+		CKL("merge_change_kernel");
 		phase_end(ctx, PH_MERGE, 1);
 	}
 	phase_begin(ctx, PH_UPDATE);
@@ -2321,8 +2344,8 @@ static int launch_estep_block(dfg_ctx *ctx, const Chunk &ch, int t0, int nt, int
 static int max_enqueue_blocked(dfg_ctx *ctx, const dfg_iter_params *par) {
 	cudaStream_t st = ctx->stream;
 	const int N = ctx->N, P = ctx->P, M = ctx->M, R = ctx->R, RT = ctx->RT, R_pad = ctx->R_pad;
-	const long long S = ctx->S, V = ctx->V;
-	const int nblk = (P + PB - 1) / PB, BT = ctx->blk_tiles;
+	const long long V = ctx->V;
+	const int BT = ctx->blk_tiles;
 	const int ob = slice_block_for(ctx);
 	{
 		double factor = std::pow(par->beta_jump, (double)((par->iteration - 1) / par->beta_period));
@@ -2409,11 +2432,8 @@ static int max_enqueue_blocked(dfg_ctx *ctx, const dfg_iter_params *par) {
 			phase_end(ctx, PH_MSTEP, ch.npix > 0 ? 1 : 0);
 		}
 		phase_begin(ctx, PH_MERGE);
-		merge_kernel<MT_3D><<<dim3(nblk, nt), 256, 0, st>>>(ctx->blkT.p, ctx->psum_r.p + r0,
-		                                                     ctx->quats.p + 5 * (size_t)r0, 1, Rb, ctx->qvals.p,
-		                                                     ctx->corr.p, ctx->mask.p, P, S, V,
-		                                                     (long long)M * V, (double *)ctx->accum.p, ctx->wflags.p, 0);
-		CKL("merge_kernel");
+		if (int rc = launch_merge(ctx, ctx->blkT.p, t0, nt, 0))
+			return rc;
 		phase_end(ctx, PH_MERGE, 1);
 	}
 	phase_begin(ctx, PH_UPDATE);
@@ -2443,11 +2463,9 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 		return max_enqueue_blocked(ctx, par);
 	cudaStream_t st = ctx->stream;
 	const int N = ctx->N, P = ctx->P, M = ctx->M, R = ctx->R, RT = ctx->RT, R_pad = ctx->R_pad;
-	const long long S = ctx->S, V = ctx->V;
-	const int nblk = (P + PB - 1) / PB;
+	const long long V = ctx->V;
 	const bool bg = ctx->with_bg && par->need_scaling;
 	double *const Wd = bg ? ctx->Wd.p : nullptr;  // FP64 slices for the background path
-	const bool two_d = ctx->model_type == MT_2D;
 	const RefineMask rm = ctx->refine ? RefineMask{ctx->qmap.p, ctx->rel_bits.p, ctx->rwords}
 	                                  : RefineMask{nullptr, nullptr, 0};
 
@@ -2555,15 +2573,8 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 	weight_pattern_kernel<<<1, 1024, 0, st>>>(ctx->psum_r.p, R, ctx->wpattern.p, ctx->wflags.p);
 	CKL("weight_pattern_kernel");
 	phase_begin(ctx, PH_MERGE);
-	if (two_d)
-		merge_kernel<MT_2D><<<dim3(nblk, RT), 256, 0, st>>>(ctx->T.p, ctx->psum_r.p, ctx->cs2d.p, M, R, ctx->qvals.p,
-		                                                     ctx->corr.p, ctx->mask.p, P, S, V, (long long)M * V, (double *)ctx->accum.p,
-		                                                     ctx->wflags.p, bg ? 1 : 0);
-	else
-		merge_kernel<MT_3D><<<dim3(nblk, RT), 256, 0, st>>>(ctx->T.p, ctx->psum_r.p, ctx->quats.p, M, R, ctx->qvals.p,
-		                                                     ctx->corr.p, ctx->mask.p, P, S, V, (long long)M * V, (double *)ctx->accum.p,
-		                                                     ctx->wflags.p, bg ? 1 : 0);
-	CKL("merge_kernel");
+	if (int rc = launch_merge(ctx, ctx->T.p, 0, RT, bg ? 1 : 0))
+		return rc;
 	phase_end(ctx, PH_MERGE, 1);
 
 	phase_begin(ctx, PH_UPDATE);

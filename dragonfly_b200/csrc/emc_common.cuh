@@ -92,7 +92,7 @@ struct Cell {
 // conversions (a volume's side stays far below 2^31), which saturate past the
 // range and give 0 for NaN; NaN positions are out of bounds.
 __device__ __forceinline__ Cell locate(const double *rot, double qx, double qy, double qz, double center,
-                                       long long S) {
+                                       long long S, int (&xyz)[3]) {
 	Cell c;
 	const double px = dadd(dadd(dadd(dmul(rot[0], qx), dmul(rot[1], qy)), dmul(rot[2], qz)), center);
 	const double py = dadd(dadd(dadd(dmul(rot[3], qx), dmul(rot[4], qy)), dmul(rot[5], qz)), center);
@@ -105,7 +105,16 @@ __device__ __forceinline__ Cell locate(const double *rot, double qx, double qy, 
 	c.fy = dsub(py, (double)y);
 	c.fz = dsub(pz, (double)z);
 	c.i000 = c.ok ? (long long)(x * (int)S + y) * S + z : 0;
+	xyz[0] = x;
+	xyz[1] = y;
+	xyz[2] = z;
 	return c;
+}
+
+__device__ __forceinline__ Cell locate(const double *rot, double qx, double qy, double qz, double center,
+                                       long long S) {
+	int xyz[3];
+	return locate(rot, qx, qy, qz, center, S, xyz);
 }
 
 // The 8 corner weights in the reference's order (000, 001, 010, 011, 100, ...).

@@ -1178,169 +1178,288 @@ __global__ void __launch_bounds__(256, MINB) mstep_kernel(const float *__restric
 // ---------------------------------------------------------------------------
 // (e2) merge: slice_merge3d of tomo_r / psum_r for every r with psum_r > 0
 // ---------------------------------------------------------------------------
-// Block = orientation tile x PB pixels. The tile's tomogram rows are staged
-// through shared memory; each (pixel, orientation) with mask <= 1 and in bounds
-// adds (f * w, f) to its 8 corners (model.c:171-244, max_update.c:33-36). The
-// accumulators are FP64: FP32 sums of thousands of contributions per voxel
-// would carry ~1e-6 relative error into the next iteration's likelihoods. They are
-// two planes of n = M V sums, model then weights: the weight sum depends only
-// on which orientations have psum_r > 0, so when that set is the one of a cached
-// weight grid with_weight is 0 and the model plane alone is touched, and a
-// zero tomogram value adds nothing. With views_final the tomograms already are
-// the views (background-aware update) and are not divided by psum_r.
-// INCR (pair lists): the weights are a change to the cached grid: wsign[r] = +1
-// / -1 adds / subtracts orientation r's weights (its psum_r > 0 state changed,
-// or +1 for every orientation with psum_r > 0 when no grid is cached), 0 adds none.
+// Every (pixel, orientation) with mask <= 1 and in bounds adds (f * w, f) to the
+// corners of its cell (model.c:171-244, max_update.c:33-36). The accumulators are
+// FP64: FP32 sums of thousands of contributions per voxel would carry ~1e-6
+// relative error into the next iteration's likelihoods. They are two planes of n
+// = M V sums, model then weights: the weight sum depends only on which
+// orientations have psum_r > 0, so when that set is the one of a cached weight
+// grid with_weight is 0 and the model plane alone is touched, and a zero
+// tomogram value adds nothing. With views_final the tomograms already are the
+// views (background-aware update) and are not divided by psum_r.
 //
-// The kernel is bound by the L2's atomic units: 190e9 32-byte sectors a second
-// while the grid fits L2 (33e9 when it does not: at 201^3 one plane is 65 MB,
-// two interleaved were 130), with up to two doubles of a sector at no extra cost. So the
-// full merge sends as few sectors as it can:
-// * the 32 lanes of a warp hold 32 consecutive pixels of one orientation (j =
-//   g + 4 k is the same for the warp); lanes whose trilinear cells coincide
-//   (__match_any_sync on the cell index) add their corner contributions in
-//   registers, in lane order, and the group's lowest lane goes on for the group;
-// * neighbouring lanes then trade halves of their corner pairs, so that one
-//   atomic instruction carries both ends of a pair (consecutive doubles, one
-//   sector in three of four cases) in neighbouring lanes.
-// Near the solution most tomogram values are zero: 10860 x 15625 pixels 4.69 ->
-// 2.01 ms, 10860 x 8281 refined 2.59 -> 1.31; all non-zero: 17220 x 9025 4.49 ->
-// 3.98, 50100 x 66820 84 (bound by issue: geometry and group sums).
+// The L2's atomic units take 190e9 additions a second on a grid that fits L2
+// (33e9 on one that does not: at 201^3 one plane is 65 MB, two interleaved were
+// 130), so the kernel sends as few as it can. A lane walks a run of ML
+// neighbouring pixels and keeps the corner sums of the cell that it is in: pixels
+// in the same cell add to them in registers, and on a step into the next
+// cell across a face only the face left behind goes to memory, the other one
+// becomes the new cell's. All 32 runs of a warp belong to one orientation and walk
+// about the same way, so the corners are numbered along that way (bit 0 behind, 1
+// ahead) and a step across one face is the same code for every lane; any other
+// move (a gap, an edge of the detector) writes the whole cell out. Before, the
+// lanes of a warp held 32 neighbouring pixels and summed equal cells by shuffles:
+// the kernel was bound by those (L1 wavefronts 85 %).
+// Block = 32 runs of ML pixels x 32 orientations, their tomogram values staged
+// through shared memory; rows in run order so that neither side has bank conflicts.
+// Runs of 8: the last cell of a run is written out whole, twice as often as with
+// runs of 16, but three blocks of warps fit an SM (two with 16: 50100 x
+// 66820 61.0 against 52.2 ms). Each pair of corners is one sector for the atomic
+// units: see send.
+// Merge in ms before / now: 50100 x 66820 84 / 52, 17220 x 9025 4.0 / 2.5, 6300 x
+// 11817 1.93 / 1.19, 3240 x 4096 0.36 / 0.23, near the solution 10860 x 15625 2.0 /
+// 1.5; without the pairs 62, 3.4, 1.6, 0.31 and 1.7.
+constexpr int MO = 32;  // orientations per block
+constexpr int ML = 8;   // pixels per run
+
+struct MergeShared {
+	float t[ML * 32][MO + 1];
+	double q[4][ML][32];   // qx, qy, qz, 1 / corr
+	double rot[MO][9];
+	double ips[MO];        // 1 / psum_r, 0 where it is not positive
+	int mode[MO];
+	unsigned use[ML];      // per step: the lanes whose pixel is merged
+};
+
+// Cell and fractions of a pixel's position, and whether the cell is inside.
 template <int GEO>
-__device__ __forceinline__ void merge_aggregated(const float (*s_tile)[TILE + 1], const double *s_ps,
-                                                 const double (*s_rot)[9], const int *s_mode, int i, int g, int p,
-                                                 int P, const double *__restrict__ qvals,
-                                                 const double *__restrict__ corr, const uint8_t *__restrict__ mask,
-                                                 long long S, long long V, long long n, double *__restrict__ accum,
-                                                 int with_weight, int views_final) {
-	const int lane = threadIdx.x & 31;
-	const bool pix = p < P && mask[p] <= 1, odd = lane & 1;
-	const int pp = pix ? p : 0;
-	const double qx = qvals[3 * (size_t)pp], qy = qvals[3 * (size_t)pp + 1], qz = qvals[3 * (size_t)pp + 2];
-	const double icr = 1. / corr[pp];
-	const double center = (double)(S / 2);
-	constexpr int NC = GEO == MT_3D ? 8 : 4;  // corners
-	// corner pair h's offset from the cell's first voxel (corner_offsets order:
-	// corners 2 h and 2 h + 1 are consecutive)
-	auto off = [S](int h) -> long long {
-		return GEO == MT_3D ? (long long)(h & 1) * S + (long long)(h >> 1) * S * S : (long long)h * S;
-	};
-	for (int k = 0; k < TILE / 4; ++k) {
-		const int j = g + 4 * k;   // the same for every lane of the warp
-		const double ips = s_ps[j];
-		if (!(ips > 0.))
-			continue;
-		const float tv = s_tile[i][j];
-		double fw[8];
-		long long base = -1;
-		bool ok = false;
-		if (pix && (with_weight || tv != 0.f || isinf(icr))) {
-			if constexpr (GEO == MT_3D) {
-				Cell c = locate(s_rot[j], qx, qy, qz, center, S);
-				ok = c.ok;
-				if (ok) {
-					corner_weights(c, fw);
-					base = c.i000;
-				}
-			} else {
-				Cell2 c = locate2d(s_rot[j], qx, qy, center, S);
-				ok = c.ok;
-				if (ok) {
-					corner_weights2(c, fw);
-					base = c.i00;
-				}
-			}
-		}
-		if (!__any_sync(FULL, ok))
-			continue;
-		if (!ok) {
-#pragma unroll
-			for (int q = 0; q < NC; ++q)
-				fw[q] = 0.;
-			base = -1 - lane;    // a group of its own
-		}
-		const double wv = views_final ? (double)tv * icr : (double)tv * ips * icr;
-		const unsigned grp = __match_any_sync(FULL, base);
-		const int most = (int)__reduce_max_sync(FULL, (unsigned)__popc(grp));
-		const bool lead = ok && (__ffs(grp) - 1) == lane;
-		const long long pbase = __shfl_xor_sync(FULL, base, 1);
-		const bool plead = __shfl_xor_sync(FULL, (int)lead, 1) != 0;
-		// first the even lane's corners, then the odd one's
-		const bool on0 = odd ? plead : lead, on1 = odd ? lead : plead;
-		double *const mode0 = accum + (size_t)s_mode[j] * V + (odd ? 1 : 0);
-		// model sums (plane 0), then with_weight the weights (plane 1): the
-		// group's lanes in lane order, summed by the lowest lane
-		for (int h = 0; h < (with_weight ? 2 : 1); ++h) {
-			double v[8];
-#pragma unroll
-			for (int q = 0; q < NC; ++q) {
-				v[q] = h == 0 ? fw[q] * wv : fw[q];
-			}
-			unsigned rest = grp & (grp - 1u);   // the group without its lowest lane
-			for (int m = 1; m < most; ++m) {
-				// the group's m-th lane, or this lane when the group is smaller
-				const int src = rest ? __ffs(rest) - 1 : lane;
-#pragma unroll
-				for (int q = 0; q < NC; ++q) {
-					const double x = __shfl_sync(FULL, h == 0 ? fw[q] * wv : fw[q], src);
-					if (rest)
-						v[q] += x;
-				}
-				rest &= rest - 1u;
-			}
-			double *const a0 = mode0 + (odd ? pbase : base) + (size_t)h * n;
-			double *const a1 = mode0 + (odd ? base : pbase) + (size_t)h * n;
-#pragma unroll
-			for (int q = 0; q < NC; q += 2) {
-				const double x = __shfl_xor_sync(FULL, odd ? v[q] : v[q + 1], 1);
-				if (on0)
-					atomicAdd(a0 + off(q / 2), odd ? x : v[q]);
-				if (on1)
-					atomicAdd(a1 + off(q / 2), odd ? v[q + 1] : x);
-			}
-		}
+__device__ __forceinline__ bool locate_axes(const double *rot, double qx, double qy, double qz, double center, int S,
+                                            int (&c)[3], double (&f)[3]) {
+	if constexpr (GEO == MT_3D) {
+		const Cell k = locate(rot, qx, qy, qz, center, S, c);
+		f[0] = k.fx;
+		f[1] = k.fy;
+		f[2] = k.fz;
+		return k.ok;
+	} else {
+		const Cell2 k = locate2d(rot, qx, qy, center, S);
+		c[0] = (int)(k.i00 / S);
+		c[1] = (int)(k.i00 - (long long)c[0] * S);
+		f[0] = k.fx;
+		f[1] = k.fy;
+		return k.ok;
 	}
 }
 
-template <int GEO, bool INCR = false>
-__global__ void __launch_bounds__(256, 3) merge_kernel(const float *__restrict__ T,
-                                                     const double *__restrict__ psum_r,
-                                                     const double *__restrict__ quats, int M, int R,
-                                                     const double *__restrict__ qvals,
-                                                     const double *__restrict__ corr,
-                                                     const uint8_t *__restrict__ mask, int P, long long S,
-                                                     long long V, long long n, double *__restrict__ accum,
-                                                     const int *__restrict__ weight_flag,
-                                                     int views_final, const signed char *__restrict__ wsign = nullptr) {
+template <int GEO>
+__global__ void __launch_bounds__(256, 3) merge_runs_kernel(
+    const float *__restrict__ T, const double *__restrict__ psum_r, const double *__restrict__ quats, int M, int R,
+    const double *__restrict__ qvals, const double *__restrict__ corr, const uint8_t *__restrict__ mask, int P,
+    long long S, long long V, long long n, double *__restrict__ accum, const int *__restrict__ weight_flag,
+    int views_final) {
+	constexpr int NA = GEO == MT_3D ? 3 : 2, NC = 1 << NA;  // axes, corners
+	extern __shared__ __align__(16) unsigned char merge_smem[];
+	MergeShared &sh = *reinterpret_cast<MergeShared *>(merge_smem);
+	const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+	// grid: pixel chunks fastest, then the orientation blocks
+	const int chunks = (P + 32 * ML - 1) / (32 * ML), ob = blockIdx.x / chunks;
+	const int p0 = (blockIdx.x - ob * chunks) * (32 * ML), rt = ob / (TILE / MO), j0 = ob % (TILE / MO) * MO;
+	const int with_weight = *weight_flag, Si = (int)S;
+	if (t < MO) {
+		const int r = rt * TILE + j0 + t;
+		const int rr = r < R ? r : 0;
+		geo_setup<GEO>(quats, rr / M, sh.rot[t]);
+		sh.mode[t] = rr % M;
+		const double ps = r < R ? psum_r[r] : 0.;
+		sh.ips[t] = ps > 0. ? fmax(fmin(1. / ps, DBL_MAX), DBL_MIN) : 0.;
+	}
+	// pixel p0 + l * ML + s is step s of lane l's run: row s * 32 + l
+	for (int i = w; i < 32 * ML; i += 8) {
+		const int p = p0 + i, row = i % ML * 32 + i / ML;
+		sh.t[row][lane] = p < P ? __ldcs(T + ((size_t)rt * P + p) * TILE + j0 + lane) : 0.f;
+	}
+	for (int s = w; s < ML; s += 8) {
+		const int p = p0 + lane * ML + s;
+		const bool use = p < P && mask[p] <= 1;
+		sh.q[0][s][lane] = use ? qvals[3 * (size_t)p] : 0.;
+		sh.q[1][s][lane] = use ? qvals[3 * (size_t)p + 1] : 0.;
+		sh.q[2][s][lane] = use ? qvals[3 * (size_t)p + 2] : 0.;
+		sh.q[3][s][lane] = use ? 1. / corr[p] : 0.;
+		const unsigned u = __ballot_sync(FULL, use);
+		if (lane == 0)
+			sh.use[s] = u;
+	}
+	__syncthreads();
+	const double center = (double)(S / 2);
+	const int stride[3] = {GEO == MT_3D ? Si * Si : Si, GEO == MT_3D ? Si : 1, 1};
+	const bool odd = lane & 1;
+	for (int h = 0; h < (with_weight ? 2 : 1); ++h)
+		for (int j = w; j < MO; j += 8) {
+			const double ips = sh.ips[j];
+			if (!(ips > 0.))
+				continue;
+			const double *rot = sh.rot[j];
+			// the way of the warp's runs: the signs of one lane's first step (a
+			// wrong guess costs whole cells, nothing else)
+			bool back[NA];
+			int off[NC];   // corner q from corner 0, the one behind on every axis
+			{
+				const unsigned both = sh.use[0] & sh.use[1];
+				const int l0 = both ? __ffs(both) - 1 : 0;
+				double d[3];
+#pragma unroll
+				for (int k = 0; k < 3; ++k)
+					d[k] = sh.q[k][1][l0] - sh.q[k][0][l0];
+#pragma unroll
+				for (int q = 0; q < NC; ++q)
+					off[q] = 0;
+#pragma unroll
+				for (int a = 0; a < NA; ++a) {
+					const double m = GEO == MT_3D ? rot[3 * a] * d[0] + rot[3 * a + 1] * d[1] + rot[3 * a + 2] * d[2]
+					                              : (a == 0 ? rot[0] * d[0] - rot[1] * d[1] : rot[1] * d[0] + rot[0] * d[1]);
+					back[a] = m < 0.;
+#pragma unroll
+					for (int q = 0; q < NC; ++q)
+						if (q >> (NA - 1 - a) & 1)
+							off[q] += back[a] ? -stride[a] : stride[a];
+				}
+			}
+			double *const grid = accum + (size_t)h * n + (size_t)sh.mode[j] * V;
+			uint32_t at = 0;      // corner 0 of the lane's cell (a volume has fewer than 2^32 voxels)
+			int cell[NA];
+			bool open = false;    // the lane holds a cell
+			double v[NC];
+#pragma unroll
+			for (int a = 0; a < NA; ++a)
+				cell[a] = 0;
+#pragma unroll
+			for (int q = 0; q < NC; ++q)
+				v[q] = 0.;
+			// Adds the corners in the lane's bit set `out`. Corners q and q | 1 are
+			// consecutive doubles: neighbouring lanes trade one of the two, so that each
+			// of two instructions carries both of one lane in neighbouring lanes.
+			auto send = [&](unsigned out) {
+				const unsigned theirs = __shfl_xor_sync(FULL, out, 1);
+				const uint32_t their_at = __shfl_xor_sync(FULL, at, 1);
+				const unsigned first = odd ? theirs : out, second = odd ? out : theirs;  // even lane's, odd lane's
+				const uint32_t at1 = odd ? their_at : at, at2 = odd ? at : their_at;
+#pragma unroll
+				for (int q = 0; q < NC; q += 2) {
+					const double got = __shfl_xor_sync(FULL, odd ? v[q] : v[q | 1], 1);
+					const int mine = odd ? q | 1 : q;          // the corner of either cell that this lane adds
+					const uint32_t o = (uint32_t)(odd ? off[q | 1] : off[q]);
+					if (first >> mine & 1u)
+						atomicAdd(grid + (uint32_t)(at1 + o), odd ? got : v[q]);
+					if (second >> mine & 1u)
+						atomicAdd(grid + (uint32_t)(at2 + o), odd ? v[q | 1] : got);
+				}
+			};
+#pragma unroll 1
+			for (int s = 0; s < ML; ++s) {
+				const float tv = sh.t[s * 32 + lane][j];
+				const double icr = sh.q[3][s][lane];
+				bool on = (sh.use[s] >> lane & 1u) && (h || tv != 0.f || isinf(icr));
+				if (!__any_sync(FULL, on))
+					continue;
+				int c[3];
+				double f[3];
+				const bool in = locate_axes<GEO>(rot, sh.q[0][s][lane], sh.q[1][s][lane], sh.q[2][s][lane], center, Si, c, f);
+				on = on && in;
+				// the move from the lane's cell, along the runs' way: the axes
+				// crossed into the next cell, or any other move
+				int far = 0;
+				unsigned cross = 0;
+#pragma unroll
+				for (int a = 0; a < NA; ++a) {
+					const int d = back[a] ? cell[a] - c[a] : c[a] - cell[a];
+					far |= d;
+					cross |= (unsigned)(d & 1) << (NA - 1 - a);
+				}
+				const bool whole = on && (!open || (far & ~1));
+				if (whole || !on)
+					cross = 0;
+				// corners left behind: q with a crossed axis where it is behind
+				constexpr unsigned long long LEFT = NA == 3 ? 0x7f3f5f0f77335500ull : 0x07030500ull;
+				const unsigned left = whole ? (open ? (1u << NC) - 1u : 0u) : (unsigned)(LEFT >> (8 * cross)) & 0xffu;
+				if (__any_sync(FULL, left != 0u))
+					send(left);
+				if (__any_sync(FULL, whole)) {
+					if (whole) {
+#pragma unroll
+						for (int q = 0; q < NC; ++q)
+							v[q] = 0.;
+						uint32_t x = 0;
+#pragma unroll
+						for (int a = 0; a < NA; ++a)
+							x += (uint32_t)(c[a] + (back[a] ? 1 : 0)) * (uint32_t)stride[a];
+						at = x;
+						open = true;
+					}
+				}
+#pragma unroll
+				for (int a = 0; a < NA; ++a) {
+					constexpr int top = NA - 1;
+					const int bit = 1 << (top - a);
+					if (cross & bit) {
+#pragma unroll
+						for (int q = 0; q < NC; ++q)
+							if (!(q & bit)) {
+								v[q] = v[q | bit];
+								v[q | bit] = 0.;
+							}
+						at += (uint32_t)off[bit];
+					}
+				}
+				if (on) {
+#pragma unroll
+					for (int a = 0; a < NA; ++a)
+						cell[a] = c[a];
+					const double wv = h ? 1. : (views_final ? (double)tv * icr : (double)tv * ips * icr);
+					double w0[NA], w1[NA];   // weight behind, ahead
+#pragma unroll
+					for (int a = 0; a < NA; ++a) {
+						const double g = dsub(1., f[a]);
+						w0[a] = back[a] ? f[a] : g;
+						w1[a] = back[a] ? g : f[a];
+					}
+					w0[0] *= wv;
+					w1[0] *= wv;
+#pragma unroll
+					for (int q = 0; q < NC; q += 2) {
+						double x = q >> (NA - 1) & 1 ? w1[0] : w0[0];
+						if (NA == 3)
+							x *= q >> 1 & 1 ? w1[1] : w0[1];
+						v[q] = fma(x, w0[NA - 1], v[q]);
+						v[q | 1] = fma(x, w1[NA - 1], v[q | 1]);
+					}
+				}
+			}
+			if (__any_sync(FULL, open))
+				send(open ? (1u << NC) - 1u : 0u);
+		}
+}
+
+// The merge of the pair lists (3-D): tomogram values are mostly zero and skipped,
+// and the weights are a change to the cached grid: wsign[r] = +1 / -1 adds /
+// subtracts orientation r's weights (its psum_r > 0 state changed, or +1 for every
+// orientation with psum_r > 0 when no grid is cached), 0 adds none. Block =
+// orientation tile x PB pixels, the tomogram rows staged through shared memory.
+__global__ void __launch_bounds__(256, 3) merge_change_kernel(
+    const float *__restrict__ T, const double *__restrict__ psum_r, const double *__restrict__ quats, int R,
+    const double *__restrict__ qvals, const double *__restrict__ corr, const uint8_t *__restrict__ mask, int P,
+    long long S, long long n, double *__restrict__ accum, const signed char *__restrict__ wsign) {
 	__shared__ double s_rot[TILE][9];
-	__shared__ int s_mode[TILE];
 	__shared__ double s_ps[TILE];
-	__shared__ signed char s_sg[INCR ? TILE : 1];
+	__shared__ signed char s_sg[TILE];
 	__shared__ float s_tile[PB][TILE + 1];
 	const int t = threadIdx.x, rt = blockIdx.y, p0 = blockIdx.x * PB;
-	const int with_weight = *weight_flag;
 	for (int j = t; j < TILE; j += blockDim.x) {
-		int r = rt * TILE + j;
-		int rr = r < R ? r : 0;
-		geo_setup<GEO>(quats, rr / M, s_rot[j]);
-		s_mode[j] = rr % M;
+		const int r = rt * TILE + j;
+		rot_from_quat(quats + 5 * (size_t)(r < R ? r : 0), s_rot[j]);
 		const double ps = r < R ? psum_r[r] : 0.;
 		s_ps[j] = ps > 0. ? fmax(fmin(1. / ps, DBL_MAX), DBL_MIN) : 0.;  // 0: not merged
-		if constexpr (INCR)
-			s_sg[j] = r < R ? wsign[r] : 0;
+		s_sg[j] = r < R ? wsign[r] : 0;
 	}
 	{
 		const int w = t >> 5, lane = t & 31;
 		for (int row = w; row < PB; row += 8) {
-			int pp = p0 + row;
+			const int pp = p0 + row;
 			float v[LW];
-			if (pp < P) {
-				ld_row_stream(T + ((size_t)rt * P + pp) * TILE + lane * LW, v);
-			} else {
 #pragma unroll
-				for (int k = 0; k < LW; ++k)
-					v[k] = 0.f;
-			}
+			for (int k = 0; k < LW; ++k)
+				v[k] = 0.f;
+			if (pp < P)
+				ld_row_stream(T + ((size_t)rt * P + pp) * TILE + lane * LW, v);
 #pragma unroll
 			for (int k = 0; k < LW; ++k)
 				s_tile[row][lane * LW + k] = v[k];
@@ -1348,55 +1467,34 @@ __global__ void __launch_bounds__(256, 3) merge_kernel(const float *__restrict__
 	}
 	__syncthreads();
 	const int i = t & (PB - 1), g = t >> 6, p = p0 + i;
-	if constexpr (!INCR) {
-		merge_aggregated<GEO>(s_tile, s_ps, s_rot, s_mode, i, g, p, P, qvals, corr, mask, S, V, n, accum,
-		                      with_weight, views_final);
-		return;
-	}
 	if (p >= P || mask[p] > 1)
 		return;
 	const double qx = qvals[3 * (size_t)p], qy = qvals[3 * (size_t)p + 1], qz = qvals[3 * (size_t)p + 2];
 	const double icr = 1. / corr[p];
 	const double center = (double)(S / 2);
-	constexpr int NC = GEO == MT_3D ? 8 : 4;  // corners
 	long long o[8];
-	if constexpr (GEO == MT_3D) {
-		corner_offsets(S, o);
-	} else {
-		o[0] = 0; o[1] = 1; o[2] = S; o[3] = S + 1;
-	}
+	corner_offsets(S, o);
 	for (int k = 0; k < TILE / 4; ++k) {
-		const int j = g + 4 * k;
+		const int j = g + 4 * k, sg = s_sg[j];
 		const double ips = s_ps[j];
 		const bool model = ips > 0. && s_tile[i][j] != 0.f;
-		const int sg = INCR ? s_sg[j] : 0;
 		if (!model && sg == 0)
 			continue;
+		const Cell c = locate(s_rot[j], qx, qy, qz, center, S);
+		if (!c.ok)
+			continue;
 		double fw[8];
-		long long base;
-		if constexpr (GEO == MT_3D) {
-			Cell c = locate(s_rot[j], qx, qy, qz, center, S);
-			if (!c.ok)
-				continue;
-			corner_weights(c, fw);
-			base = c.i000;
-		} else {
-			Cell2 c = locate2d(s_rot[j], qx, qy, center, S);
-			if (!c.ok)
-				continue;
-			corner_weights2(c, fw);
-			base = c.i00;
-		}
-		double *a = accum + (size_t)s_mode[j] * V + base;
+		corner_weights(c, fw);
+		double *a = accum + c.i000;
 		if (model) {
 			const double wv = (double)s_tile[i][j] * ips * icr;
 #pragma unroll
-			for (int q = 0; q < NC; ++q)
+			for (int q = 0; q < 8; ++q)
 				atomicAdd(a + o[q], fw[q] * wv);
 		}
 		if (sg != 0) {
 #pragma unroll
-			for (int q = 0; q < NC; ++q)
+			for (int q = 0; q < 8; ++q)
 				atomicAdd(a + n + o[q], sg > 0 ? fw[q] : -fw[q]);
 		}
 	}
