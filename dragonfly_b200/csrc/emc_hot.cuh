@@ -325,14 +325,17 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 // Balanced digits: x = sum_g d_g 256^g with -128 <= d_g <= 127. K past the last
 // pixel or frame is zero. A log-slice that the digits cannot hold (log 0, the
 // value outside the model, NaN) sets special[tile]: the E-step then gathers
-// that tile's photons all. Block = 128 reduction rows x 64 orientations,
+// that tile's photons all. live (true; may be null): [tile][Nc + 1] flags of
+// the rows that hold probabilities (tile skipping), the others count as zero.
+// Block = 128 reduction rows x 64 orientations,
 // transposed through shared memory; the rotation by 4 (k / 16) keeps the
 // column reads free of bank conflicts. Memory-bound: 4 bytes read, 4 written.
 template <bool MSTEP>
 __global__ void __launch_bounds__(256) hot_digits_kernel(const float *__restrict__ src, size_t tile_stride,
                                                          const int *__restrict__ pix, int nk, int k_pitch,
                                                          const float *__restrict__ rmax, int8_t *__restrict__ dig,
-                                                         int *__restrict__ special) {
+                                                         int *__restrict__ special,
+                                                         const uint8_t *__restrict__ live) {
 	__shared__ int s[HK][HO + 1];
 	__shared__ double s_scale[HO];
 	const int kb = blockIdx.x, ot = blockIdx.y, t = threadIdx.x;
@@ -347,7 +350,7 @@ __global__ void __launch_bounds__(256) hot_digits_kernel(const float *__restrict
 	for (int idx = t; idx < HK * (HO / 4); idx += 256) {
 		const int k = idx / (HO / 4), o = (idx % (HO / 4)) * 4, kg = kb * HK + k;
 		int v[4] = {0, 0, 0, 0};
-		if (kg < nk) {
+		if (kg < nk && (live == nullptr || live[(size_t)rt * (nk + 1) + kg])) {
 			const int row = MSTEP ? kg : pix[kg];
 			const float4 x4 = __ldg(reinterpret_cast<const float4 *>(src + (size_t)rt * tile_stride +
 			                                                          (size_t)row * TILE + j0 + o));

@@ -64,6 +64,39 @@ def test_products_match_oracle_and_gathers(oracle_built, frames, div, side, phot
     plain.close()
 
 
+@pytest.mark.parametrize("refined", [False, True])
+def test_tomograms_are_the_sums_over_the_kept_pairs(refined):
+    """T_r = sum_d P_dr c_d / psum_r from the FP64 probability lists. Refined: most
+    tiles are dead for a frame, and their probability rows (here those of a full
+    search before) are not written. FP32: P carries three roundings (exp, 1 / norm,
+    product), T one."""
+    prob = _problem(300, 2, 24, 200.)
+    R, n = prob.quats.shape[0], prob.num_data
+    cells = (np.arange(R) * 7 // R).astype(np.int32)         # consecutive orientations share a cell
+    lists = np.random.default_rng(3).integers(0, 7, (n, 1)).astype(np.int32)
+    lister, gpu = GPUEngine(prob, keep_prob=1), GPUEngine(prob)
+    par = gpu.ctx.params(1, 1, 0, 0, 1., 100, 1.)
+    gpu.ctx.maximize(par)
+    if refined:
+        for g in (lister, gpu):
+            g.ctx.set_refinement(7, cells, lists)
+    lister.ctx.maximize(par)
+    gpu.ctx.maximize(par)
+    off, place, p = lister.ctx.sparse_prob()
+    psum = lister.ctx.orientation_results()[1]
+    counts = np.zeros((n, prob.num_pix))
+    np.add.at(counts, (np.repeat(np.arange(n), prob.ones), prob.place_ones), 1.)
+    np.add.at(counts, (np.repeat(np.arange(n), prob.multi), prob.place_multi), prob.count_multi)
+    counts[:, prob.mask > 1] = 0.
+    P = np.zeros((R, n))
+    P[place, np.repeat(np.arange(n), np.diff(off))] = p
+    want = P @ counts
+    want[psum > 0] /= psum[psum > 0, None]
+    np.testing.assert_allclose(gpu.ctx.tomograms(0, R), want, rtol=4 * 2. ** -24, atol=1e-8 * want.max())
+    lister.close()
+    gpu.close()
+
+
 def test_product_wait_gives_up_and_the_context_recovers(oracle_built):
     """A stage whose copies are withheld (test hook): its waits run out, the
     kernels return, the call reports the error, and the next call succeeds."""
