@@ -372,6 +372,7 @@ static int finish_refinement(dfg_ctx *ctx, int num_coarse, const int *quat_mappi
 	ctx->rwords = (num_coarse + 31) / 32;
 	ctx->refine = true;
 	ctx->qmap_valid = false;
+	ctx->refine_live = -1.;
 	return DFG_OK;
 }
 
@@ -1244,6 +1245,7 @@ constexpr double kHotOccupancy = 0.012;
 // on the frames alone: the count matrices of every chunk and the photon lists
 // without them. hot_n = 0 leaves everything to the gathers.
 static bool tile_skipping(const dfg_ctx *ctx);
+static int prepare_qmap(dfg_ctx *ctx);
 
 static int hot_choose(dfg_ctx *ctx) {
 	const int N = ctx->N, P = ctx->P;
@@ -1272,6 +1274,9 @@ static int hot_choose(dfg_ctx *ctx) {
 	if (n < HK)
 		return DFG_OK;
 	cand.resize(n);
+	ctx->hot_words = 0.;
+	for (int p : cand)
+		ctx->hot_words += (double)ctx->h_pix_entries[p] / N;
 	const int pitch = (n + HK - 1) / HK * HK;
 	std::vector<uint8_t> is_hot((size_t)P, 0);
 	for (int p : cand)
@@ -1388,6 +1393,34 @@ static int hot_choose(dfg_ctx *ctx) {
 	return DFG_OK;
 }
 
+// A refined search takes the E-step's products too when they cost less than the
+// gathers they replace: they run over all (tile, frame) pairs, the gathers over
+// the share with an evaluated pair. A column of the products costs about as much
+// as 0.008 gathered words per frame (2.2e-15 s per orientation, frame and pixel
+// against 2.3e-13 to 3.5e-13 per word). 10860 x 12000, 140 words a frame: E-step ms
+// with products / gathers at shares 0.43, 0.30, 0.25 and 0.15: 1.31 / 2.77, 1.19 /
+// 2.12, 1.13 / 1.82, 1.02 / 1.27.
+constexpr double kHotColumnWords = 0.008;
+
+// The share of the (tile, frame) pairs that a refinement evaluates, counted once.
+static double refine_share(dfg_ctx *ctx) {
+	if (ctx->refine_live < 0.) {
+		DevBuf<unsigned long long> n;
+		unsigned long long h = 0;
+		if (prepare_qmap(ctx) != DFG_OK || n.ensure(1) != cudaSuccess ||
+		    cudaMemsetAsync(n.p, 0, sizeof(h), ctx->stream) != cudaSuccess)
+			return 0.;
+		refine_count_kernel<<<dim3((unsigned)std::min<long long>(blocks_for(ctx->N, 8), 64), ctx->RT), 256, 0, ctx->stream>>>(
+		    RefineMask{ctx->qmap.p, ctx->rel_bits.p, ctx->rwords}, ctx->N, ctx->RT, n.p);
+		ctx->launches++;
+		if (cudaMemcpyAsync(&h, n.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
+		    cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+			return 0.;
+		ctx->refine_live = (double)h / ((double)ctx->N * ctx->RT);
+	}
+	return ctx->refine_live;
+}
+
 // The products' buffers for this iteration: the log-slices' digits, and the
 // probabilities' digits over the chunk's log-likelihoods (dead by the M-step;
 // half their size).
@@ -1398,7 +1431,8 @@ static int hot_prepare(dfg_ctx *ctx) {
 	if (ctx->hot_n == 0)
 		return DFG_OK;
 	const long long rows = (long long)ctx->RT * 2 * 4 * HO;
-	if (!ctx->refine) {  // a restricted E-step gathers: most of its pairs are skipped
+	ctx->hot_estep = !ctx->refine || refine_share(ctx) * ctx->hot_words >= kHotColumnWords * ctx->hot_n;
+	if (ctx->hot_estep) {
 		const cudaError_t e = ctx->wdig.ensure((size_t)rows * ctx->hot_pitch);
 		if (e == cudaErrorMemoryAllocation) {
 			cudaGetLastError();
@@ -1525,7 +1559,7 @@ static int max_prepare(dfg_ctx *ctx, const dfg_iter_params *par) {
 		return DFG_ERR_ARG;
 	NEED(par->beta_period > 0, DFG_ERR_ARG, "beta_period must be > 0");
 	CK(cudaSetDevice(ctx->device));
-	ctx->hot_active = false;
+	ctx->hot_active = ctx->hot_estep = false;
 	if (pair_mode(ctx))
 		return pair_prepare(ctx, par);
 	if (blocked_wanted(ctx))
@@ -1751,20 +1785,23 @@ static int launch_estep(dfg_ctx *ctx, const Chunk &ch, int use_scale, bool bg, c
 	// blocks per SM: the autotuner's choice (or the option), else the default
 	const int minb = ctx->tuning ? ctx->tune_estep_minb : (ctx->estep_minb > 0 ? ctx->estep_minb
 	                                                                           : ctx->tuned_estep_minb);
-	if (ctx->hot_active && rm.qmap == nullptr) {
+	if (ctx->hot_estep) {
 		if (int rc = launch_hot_estep(ctx, ch))
 			return rc;
 		const HotLists full{ctx->hot_special.p, ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p};
-#define DFG_ECOLD(MB)                                                                                         \
-	estep_cold_kernel<MB><<<dim3(blocks_for(Nc, 8), RT), 256, 0, st>>>(                                       \
+#define DFG_ECOLD(REF, MB)                                                                                    \
+	estep_cold_kernel<REF, MB><<<dim3(blocks_for(Nc, 8), RT), 256, 0, st>>>(                                       \
 	    ctx->logW.p, ctx->u.p, ctx->logw.p, R, ctx->phc.p, ctx->phc_off.p, ctx->phc_mid.p, ctx->scale.p,        \
-	    ctx->blacklist.p, ch.d0, Nc, use_scale, ctx->scalars.p, P, ctx->pval.p, ctx->tmax.p, ctx->targ.p, full)
-		if (minb == 2)
-			DFG_ECOLD(2);
+	    ctx->blacklist.p, ch.d0, Nc, use_scale, ctx->scalars.p, P, ctx->pval.p, ctx->tmax.p, ctx->targ.p, full, \
+	    rm)
+		if (rm.qmap != nullptr)
+			DFG_ECOLD(true, 4);
+		else if (minb == 2)
+			DFG_ECOLD(false, 2);
 		else if (minb == 3)
-			DFG_ECOLD(3);
+			DFG_ECOLD(false, 3);
 		else
-			DFG_ECOLD(4);
+			DFG_ECOLD(false, 4);
 #undef DFG_ECOLD
 		CKL("estep_cold_kernel");
 		return DFG_OK;
@@ -2501,7 +2538,7 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 		    (__nv_bfloat16 *)ctx->Alo.p);
 		CKL("split_logw_kernel");
 	}
-	const bool hot_e = ctx->hot_active && !ctx->refine;
+	const bool hot_e = ctx->hot_active && ctx->hot_estep;
 	if (hot_e)
 		if (int rc = launch_hot_digits(ctx))
 			return rc;
@@ -2676,7 +2713,7 @@ static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par) {
 		CKL("rescale_kernel");
 		logw_kernel<<<blocks_for(ctx->R, 256), 256, 0, st>>>(ctx->quats.p, ctx->M, ctx->R, ctx->logw.p);
 		CKL("logw_kernel");
-		if (ctx->hot_active && !ctx->refine)
+		if (ctx->hot_estep)
 			rc = launch_hot_digits(ctx);
 	}
 	if (rc == DFG_OK)

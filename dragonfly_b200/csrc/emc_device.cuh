@@ -349,17 +349,38 @@ struct HotLists {
 	const long long *off, *mid;
 };
 
-template <int MINB>
+// Tiles with an evaluated pair under refinement, over all frames (the share of
+// the pairs that a gathering E-step would visit). One warp per (tile, frame) in
+// turn; out += live tiles.
+__global__ void __launch_bounds__(256) refine_count_kernel(RefineMask rm, int N, int RT,
+                                                           unsigned long long *__restrict__ out) {
+	const int rt = blockIdx.y, lane = threadIdx.x & 31;
+	unsigned live = 0;
+	for (int d = blockIdx.x * 8 + (threadIdx.x >> 5); d < N; d += gridDim.x * 8)
+		live += __any_sync(FULL, refine_live(rm, d, rt * TILE + lane * LW)) ? 1u : 0u;
+	if (lane == 0 && live)
+		atomicAdd(out, (unsigned long long)live);
+}
+
+template <bool REFINE, int MINB>
 __global__ void __launch_bounds__(256, MINB) estep_cold_kernel(
     const float *__restrict__ logW, const double *__restrict__ u, const double *__restrict__ logw, int R,
     const uint32_t *__restrict__ ph, const long long *__restrict__ ph_off, const long long *__restrict__ ph_mid,
     const double *__restrict__ scale, const uint8_t *__restrict__ blacklist, int d0, int Nc, int use_scale,
     const double *__restrict__ scalars, int P, double *pval, double *__restrict__ tmax, int *__restrict__ targ,
-    HotLists full) {
+    HotLists full, RefineMask rm) {
 	static_assert(LW == 4, "the products need 128-orientation tiles");
 	const int rt = blockIdx.y, dl = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, d = d0 + dl;
 	if (dl >= Nc || blacklist[d])
 		return;
+	unsigned live = (1u << LW) - 1u;
+	if constexpr (REFINE) {
+		live = refine_live(rm, d, rt * TILE + lane * LW);
+		if (!__any_sync(FULL, live)) {
+			refine_skip_tile(tmax, targ, rt, Nc, dl, lane);
+			return;
+		}
+	}
 	const bool special = full.special[rt] != 0;
 	if (special) {
 		ph = full.ph;
@@ -433,7 +454,9 @@ __global__ void __launch_bounds__(256, MINB) estep_cold_kernel(
 		acc[k] = 0.;
 		if (r0 + k < R) {
 			acc[k] = dadd(dsub(lw[k], dmul(ur[k], sd)), sum);
-			if (acc[k] > m) {
+			if (REFINE && !(live >> k & 1u)) {
+				acc[k] = -INFINITY;
+			} else if (acc[k] > m) {
 				m = acc[k];
 				am = r0 + k;
 			}

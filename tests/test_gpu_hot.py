@@ -64,25 +64,30 @@ def test_products_match_oracle_and_gathers(oracle_built, frames, div, side, phot
     plain.close()
 
 
-@pytest.mark.parametrize("refined", [False, True])
-def test_tomograms_are_the_sums_over_the_kept_pairs(refined):
-    """T_r = sum_d P_dr c_d / psum_r from the FP64 probability lists. Refined: most
-    tiles are dead for a frame, and their probability rows (here those of a full
-    search before) are not written. FP32: P carries three roundings (exp, 1 / norm,
-    product), T one."""
+@pytest.mark.parametrize("cells_per_frame", [0, 1, 6])
+def test_tomograms_are_the_sums_over_the_kept_pairs(cells_per_frame):
+    """T_r = sum_d P_dr c_d / psum_r from the FP64 probability lists: full search, and
+    refined with one cell of seven a frame (most tiles dead, their probability rows --
+    here those of a full search before -- not written) and with six (the E-step's
+    products too). FP32: P carries three roundings (exp, 1 / norm, product), T one."""
     prob = _problem(300, 2, 24, 200.)
     R, n = prob.quats.shape[0], prob.num_data
     cells = (np.arange(R) * 7 // R).astype(np.int32)         # consecutive orientations share a cell
-    lists = np.random.default_rng(3).integers(0, 7, (n, 1)).astype(np.int32)
+    rng = np.random.default_rng(3)
+    lists = np.array([rng.permutation(7)[:cells_per_frame] for _ in range(n)], np.int32)
     lister, gpu = GPUEngine(prob, keep_prob=1), GPUEngine(prob)
     par = gpu.ctx.params(1, 1, 0, 0, 1., 100, 1.)
     gpu.ctx.maximize(par)
-    if refined:
+    if cells_per_frame:
         for g in (lister, gpu):
             g.ctx.set_refinement(7, cells, lists)
     lister.ctx.maximize(par)
     gpu.ctx.maximize(par)
     off, place, p = lister.ctx.sparse_prob()
+    if cells_per_frame:
+        own = np.zeros((n, 7), bool)
+        np.put_along_axis(own, lists, True, 1)
+        assert np.all(own[np.repeat(np.arange(n), np.diff(off)), cells[place]])
     psum = lister.ctx.orientation_results()[1]
     counts = np.zeros((n, prob.num_pix))
     np.add.at(counts, (np.repeat(np.arange(n), prob.ones), prob.place_ones), 1.)
