@@ -12,9 +12,9 @@
 // operand becomes a 32-bit fixed-point number cut into four signed bytes, each
 // byte's product accumulates in an INT32 TMEM accumulator (exact below 2^24
 // counts per sum), and the epilogue puts the four sums together in FP64. The
-// FP32 log-slices are multiples of 2^-23 for |x| >= 1 (the error below that is
-// 2^-24), so the E-step's sum is the exact sum of the values that the
-// gathers add; the probabilities are taken relative to their orientation's
+// FP32 log-slices are multiples of 2^-26 from |x| = 1/8 on (below it they are
+// off by at most 2^-27), so the E-step's sum is the exact sum of the values that
+// the gathers add; the probabilities are taken relative to their orientation's
 // largest in the chunk (2e9 steps), 2.5e-10 of it, far below the FP32 rounding of
 // the tomogram they end in. The remaining (cold) photons are gathered as before.
 //
@@ -56,8 +56,8 @@ constexpr int HSTAGE_BYTES = HA_BYTES + HB_BYTES;  // 64 KB
 constexpr int HSMEM_BYTES = 1024 + HSTAGES * HSTAGE_BYTES + 128;
 constexpr int HTHREADS = 320;
 constexpr int HGROUP = 12;   // orientation tiles per rasterisation group: 12 x 12 resident tiles share operands in L2
-constexpr float HE_SCALE = 8388608.f;   // log-slices in steps of 2^-23
-constexpr float HE_LIMIT = 250.f;       // largest |log W| that the four digits hold
+constexpr float HE_SCALE = 67108864.f;  // log-slices in steps of 2^-26
+constexpr float HE_LIMIT = 31.f;        // largest |log W| that the four digits hold (W from 3.4e-14)
 constexpr double HP_STEPS = 2.0e9;      // steps of an orientation's largest probability (< 125 x 2^24)
 
 // Instruction descriptor of kind::i8: S32 accumulator (bits 4-5 = 2), A

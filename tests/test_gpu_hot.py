@@ -64,6 +64,24 @@ def test_products_match_oracle_and_gathers(oracle_built, frames, div, side, phot
     plain.close()
 
 
+def test_products_lose_no_precision_at_small_logarithms(oracle_built):
+    """A start model of about one photon per pixel, where log W is small and FP32
+    holds it finely: the digits must too. The gathers' compensated sums round once
+    more per photon, so the products' model is as close to the oracle's (its error
+    is a sum over few orientations here, hence the half)."""
+    d, shared = synth.two_detector_problem(seed=8, n_frames=(300, 200))
+    d = d[0]
+    prob = EMCProblem(d["qvals"], d["corr"], d["mask"], d["ones"], d["multi"], d["place_ones"], d["place_multi"],
+                      d["count_multi"], shared["quats"], shared["model_start"], need_scaling=1, update_scale=1, beta=0.5)
+    want = OracleEngine(prob).run_iteration(1)["model1"]
+    off = []
+    for skip in (0, 1):
+        gpu = GPUEngine(prob, tile_skip=skip)
+        off.append(np.linalg.norm(gpu.run_iteration(1)["model1"] - want))
+        gpu.close()
+    assert off[0] <= 1.5 * off[1]
+
+
 @pytest.mark.parametrize("cells_per_frame", [0, 1, 6])
 def test_tomograms_are_the_sums_over_the_kept_pairs(cells_per_frame):
     """T_r = sum_d P_dr c_d / psum_r from the FP64 probability lists: full search, and
