@@ -11,6 +11,7 @@
 
 #include <cudaTypedefs.h>
 
+#include <memory>
 #include <thread>
 
 #include "emc_ctx.cuh"
@@ -152,6 +153,10 @@ extern "C" int dfg_set_detector(dfg_ctx *ctx, int num_pix, const double *qvals, 
 // per host thread (ascending ranges for ascending thread numbers).
 template <typename F>
 static void parallel_ranges(long long n, int threads, F fn) {
+	if (threads <= 1) {
+		fn(0, 0LL, n);
+		return;
+	}
 	std::vector<std::thread> pool;
 	for (int k = 0; k < threads; ++k) {
 		const long long b = n * k / threads, e = n * (k + 1) / threads;
@@ -716,8 +721,6 @@ static int build_chunks(dfg_ctx *ctx) {
 	// row Nc.
 	NEED(nc <= (long long)IDX_MASK, DFG_ERR_ARG, "frame chunk of %lld frames exceeds %u", nc, IDX_MASK);
 	const uint8_t *mk = ctx->h_mask.data();
-	std::vector<long long> c1(P + 1), cm(P + 1), photons(P + 1);
-	std::vector<uint32_t> words;
 	ctx->h_pix_entries.assign((size_t)P, 0);
 	ctx->h_pix_big.assign((size_t)P, 0);
 	for (int k = 0; k < n_chunks; ++k) {
@@ -725,58 +728,93 @@ static int build_chunks(dfg_ctx *ctx) {
 		ch.d0 = (int)(k * nc);
 		ch.nc = (int)std::min<long long>(nc, N - ch.d0);
 		const uint32_t pad = (uint32_t)ch.nc;
-		std::fill(c1.begin(), c1.end(), 0);
-		std::fill(cm.begin(), cm.end(), 0);
-		std::fill(photons.begin(), photons.end(), 0);
-		auto each = [&](auto fn) {
-			for (int dl = 0; dl < ch.nc; ++dl) {
-				int d = ch.d0 + dl;
+		// contiguous frame ranges, one per host thread (at least a million words
+		// each): every range counts its words per pixel and fills them in from its
+		// own cursors, so the lists keep the frames' order
+		const int d1 = ch.d0 + ch.nc;
+		const long long given = ctx->h_ones_off[d1] - ctx->h_ones_off[ch.d0] + ctx->h_multi_off[d1] -
+		                        ctx->h_multi_off[ch.d0];
+		const int nth = (int)std::max<long long>(
+		    1, std::min<long long>({16, (long long)std::thread::hardware_concurrency(), given >> 20, ch.nc}));
+		auto each = [&](long long b, long long e, auto fn) {
+			for (int dl = (int)b; dl < (int)e; ++dl) {
+				const int d = ch.d0 + dl;
 				for (long long i = ctx->h_ones_off[d]; i < ctx->h_ones_off[d + 1]; ++i) {
-					int p = ctx->h_place_ones[i];
+					const int p = ctx->h_place_ones[i];
 					if (mk[p] < 2)
 						fn(p, dl, 1LL);
 				}
 				for (long long i = ctx->h_multi_off[d]; i < ctx->h_multi_off[d + 1]; ++i) {
-					int p = ctx->h_place_multi[i];
+					const int p = ctx->h_place_multi[i];
 					if (mk[p] < 2)
 						fn(p, dl, (long long)ctx->h_count_multi[i]);
 				}
 			}
 		};
-		each([&](int p, int, long long c) {
-			if (c == 1)
-				c1[p]++;
-			else
-				cm[p] += (c + MAX_COUNT - 1) / MAX_COUNT;
-			photons[p] += c;
-			if (c > 255)
-				ctx->h_pix_big[p] = 1;
+		// per range and pixel: count-1 words, counted words, photons, counts past
+		// a byte; then the cursors of the two segments
+		std::vector<long long> c1((size_t)nth * P, 0), cm((size_t)nth * P, 0), photons((size_t)nth * P, 0);
+		std::vector<uint8_t> big((size_t)nth * P, 0);
+		parallel_ranges(ch.nc, nth, [&](int th, long long b, long long e) {
+			long long *t1 = c1.data() + (size_t)th * P, *tm = cm.data() + (size_t)th * P;
+			long long *tp = photons.data() + (size_t)th * P;
+			uint8_t *tb = big.data() + (size_t)th * P;
+			each(b, e, [&](int p, int, long long c) {
+				if (c == 1)
+					t1[p]++;
+				else
+					tm[p] += (c + MAX_COUNT - 1) / MAX_COUNT;
+				tp[p] += c;
+				if (c > 255)
+					tb[p] = 1;
+			});
 		});
-		std::vector<long long> off(P + 1, 0), midv(P, 0), f1(P), fm(P);
+		std::vector<long long> off(P + 1, 0), midv(P, 0), end1(P), endm(P);
 		long long real = 0;
 		for (int p = 0; p < P; ++p) {
-			const long long a = (c1[p] + 7) / 8 * 8, b = (cm[p] + 7) / 8 * 8;
-			f1[p] = off[p];
-			midv[p] = off[p] + a;
-			fm[p] = midv[p];
-			off[p + 1] = off[p] + a + b;
-			real += c1[p] + cm[p];
-			ctx->h_pix_entries[p] += c1[p] + cm[p];
-			if (photons[p] >= kHotMaxSum)
+			long long n1 = 0, nm = 0, ph = 0;
+			for (int th = 0; th < nth; ++th) {
+				n1 += c1[(size_t)th * P + p];
+				nm += cm[(size_t)th * P + p];
+				ph += photons[(size_t)th * P + p];
+				ctx->h_pix_big[p] |= big[(size_t)th * P + p];
+			}
+			midv[p] = off[p] + (n1 + 7) / 8 * 8;
+			off[p + 1] = midv[p] + (nm + 7) / 8 * 8;
+			end1[p] = off[p] + n1;
+			endm[p] = midv[p] + nm;
+			long long f1 = off[p], fm = midv[p];
+			for (int th = 0; th < nth; ++th) {
+				const long long a = c1[(size_t)th * P + p], b = cm[(size_t)th * P + p];
+				c1[(size_t)th * P + p] = f1;
+				cm[(size_t)th * P + p] = fm;
+				f1 += a;
+				fm += b;
+			}
+			real += n1 + nm;
+			ctx->h_pix_entries[p] += n1 + nm;
+			if (ph >= kHotMaxSum)
 				ctx->h_pix_big[p] = 1;
 		}
-		words.assign((size_t)off[P], pad);
-		each([&](int p, int dl, long long c) {
-			if (c == 1) {
-				words[(size_t)f1[p]++] = (uint32_t)dl;
-				return;
-			}
-			while (c > 0) {
-				uint32_t cc = (uint32_t)std::min<long long>(c, MAX_COUNT);
-				words[(size_t)fm[p]++] = (uint32_t)dl | (cc << IDX_BITS);
-				c -= cc;
-			}
+		const std::unique_ptr<uint32_t[]> words(new uint32_t[(size_t)std::max<long long>(off[P], 1)]);
+		parallel_ranges(ch.nc, nth, [&](int th, long long b, long long e) {
+			long long *f1 = c1.data() + (size_t)th * P, *fm = cm.data() + (size_t)th * P;
+			each(b, e, [&](int p, int dl, long long c) {
+				if (c == 1) {
+					words[(size_t)f1[p]++] = (uint32_t)dl;
+					return;
+				}
+				while (c > 0) {
+					const uint32_t cc = (uint32_t)std::min<long long>(c, MAX_COUNT);
+					words[(size_t)fm[p]++] = (uint32_t)dl | (cc << IDX_BITS);
+					c -= cc;
+				}
+			});
 		});
+		for (int p = 0; p < P; ++p) {
+			std::fill(words.get() + end1[p], words.get() + midv[p], pad);
+			std::fill(words.get() + endm[p], words.get() + off[p + 1], pad);
+		}
 		std::vector<int> pix;
 		for (int p = 0; p < P; ++p)
 			if (off[p + 1] > off[p])
@@ -785,7 +823,7 @@ static int build_chunks(dfg_ctx *ctx) {
 		                 [&](int a, int b) { return off[a + 1] - off[a] > off[b + 1] - off[b]; });
 		ch.npix = (int)pix.size();
 		ch.entries = real;
-		CK(upload(ch.cs, words.data(), words.size(), ctx->stream));
+		CK(upload(ch.cs, words.get(), (size_t)off[P], ctx->stream));
 		CK(upload(ch.cs_off, off.data(), off.size(), ctx->stream));
 		CK(upload(ch.cs_mid, midv.data(), midv.size(), ctx->stream));
 		CK(upload(ch.pix, pix.data(), pix.size(), ctx->stream));
@@ -2285,6 +2323,11 @@ static bool blocked_wanted(dfg_ctx *ctx) {
 	if (ctx->block_budget_mb > 0.)
 		return true;
 	const size_t RT = ((size_t)ctx->M * ctx->num_rot + TILE - 1) / TILE;
+	// resident already, with the chunks laid out beside them: no query of the
+	// free memory, which takes 0.08 ms
+	if (!ctx->blocked && ctx->chunks_R == ctx->M * ctx->num_rot && ctx->logW_P == ctx->P &&
+	    ctx->logW.n >= RT * (size_t)(ctx->P + 1) * TILE && ctx->T.n >= RT * (size_t)ctx->P * TILE)
+		return false;
 	const size_t need = RT * ((size_t)2 * ctx->P + 1) * TILE * sizeof(float);
 	size_t fr = 0, tot = 0;
 	if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
@@ -2757,7 +2800,8 @@ static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par) {
 			ctx->tune_estep_minb = cand[i];
 			rc = timed([&] { return launch_estep(ctx, c0, use_scale, bg, rm, false); }, rep[10 + i]);
 		}
-		for (int i = 0; i < 3; ++i)
+		e_minb = cand[0];   // the fewest of equally fast ones
+		for (int i = 1; i < 3; ++i)
 			if (rep[10 + i] >= 0. && rep[10 + i] < rep[10 + (e_minb - 2)])
 				e_minb = cand[i];
 		ctx->tune_estep_minb = ESTEP_MINB;
@@ -2769,7 +2813,8 @@ static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par) {
 			ctx->tune_mstep_minb = cand[i];
 			rc = timed([&] { return launch_mstep(ctx, c0, false); }, rep[13 + i]);
 		}
-		for (int i = 0; i < 3; ++i)
+		m_minb = cand[0];
+		for (int i = 1; i < 3; ++i)
 			if (rep[13 + i] >= 0. && rep[13 + i] < rep[13 + (m_minb - 3)])
 				m_minb = cand[i];
 		ctx->tune_mstep_minb = MSTEP_MINB;
@@ -3716,21 +3761,53 @@ static cudaError_t fetch(T *h, const DevBuf<T> &b, size_t n, cudaStream_t s) {
 	return cudaMemcpyAsync(h, b.p, n * sizeof(T), cudaMemcpyDeviceToHost, s);
 }
 
+// Several results at once. Small ones go through page-locked staging: one
+// wait for all of them, where a copy into pageable memory waits by itself (six
+// arrays of 450 frames 0.09 ms).
+struct FetchItem {
+	void *host;
+	const void *dev;
+	size_t bytes;
+};
+constexpr size_t kStageBytes = (size_t)1 << 20;
+
+static int fetch_all(dfg_ctx *ctx, std::initializer_list<FetchItem> items) {
+	size_t total = 0;
+	for (const FetchItem &f : items)
+		total += f.host ? (f.bytes + 15) / 16 * 16 : 0;
+	const bool staged = total <= kStageBytes && ctx->stage_out.ensure(kStageBytes) == cudaSuccess;
+	if (!staged)
+		cudaGetLastError();
+	size_t at = 0;
+	for (const FetchItem &f : items)
+		if (f.host) {
+			CK(cudaMemcpyAsync(staged ? ctx->stage_out.p + at : f.host, f.dev, f.bytes, cudaMemcpyDeviceToHost,
+			                   ctx->stream));
+			at += (f.bytes + 15) / 16 * 16;
+		}
+	CK(cudaStreamSynchronize(ctx->stream));
+	at = 0;
+	for (const FetchItem &f : items)
+		if (staged && f.host) {
+			std::memcpy(f.host, ctx->stage_out.p + at, f.bytes);
+			at += (f.bytes + 15) / 16 * 16;
+		}
+	return DFG_OK;
+}
+
 extern "C" int dfg_get_frame_results(dfg_ctx *ctx, int *rmax, double *info, double *likelihood,
                                      double *max_exp, double *p_norm, double *psum_d) {
 	if (!ctx)
 		return DFG_ERR_ARG;
 	NEED(ctx->have_results, DFG_ERR_STATE, "no results yet");
 	CK(cudaSetDevice(ctx->device));
-	const size_t N = (size_t)ctx->N;
-	CK(fetch(rmax, ctx->rmax, N, ctx->stream));
-	CK(fetch(info, ctx->info, N, ctx->stream));
-	CK(fetch(likelihood, ctx->likelihood, N, ctx->stream));
-	CK(fetch(max_exp, ctx->max_exp, N, ctx->stream));
-	CK(fetch(p_norm, ctx->p_norm, N, ctx->stream));
-	CK(fetch(psum_d, ctx->psum_d, N, ctx->stream));
-	CK(cudaStreamSynchronize(ctx->stream));
-	return DFG_OK;
+	const size_t N = (size_t)ctx->N, D = N * sizeof(double);
+	return fetch_all(ctx, {{rmax, ctx->rmax.p, N * sizeof(int)},
+	                       {info, ctx->info.p, D},
+	                       {likelihood, ctx->likelihood.p, D},
+	                       {max_exp, ctx->max_exp.p, D},
+	                       {p_norm, ctx->p_norm.p, D},
+	                       {psum_d, ctx->psum_d.p, D}});
 }
 
 extern "C" int dfg_get_num_prob(dfg_ctx *ctx, int *num_prob) {
@@ -3827,17 +3904,13 @@ extern "C" int dfg_get_frame_params(dfg_ctx *ctx, double *scale, double *beta, d
 	if (int rc = need_frames(ctx))
 		return rc;
 	CK(cudaSetDevice(ctx->device));
-	const size_t N = (size_t)ctx->N;
-	CK(fetch(scale, ctx->scale, N, ctx->stream));
-	if (ctx->beta_set) {
-		CK(fetch(beta, ctx->beta, N, ctx->stream));
-		CK(fetch(beta_start, ctx->beta_start, N, ctx->stream));
-	}
-	CK(fetch(fcounts, ctx->fcounts, N, ctx->stream));
-	CK(fetch(sum_fact, ctx->sum_fact, N, ctx->stream));
-	CK(fetch(blacklist, ctx->blacklist, N, ctx->stream));
-	CK(cudaStreamSynchronize(ctx->stream));
-	return DFG_OK;
+	const size_t N = (size_t)ctx->N, D = N * sizeof(double);
+	return fetch_all(ctx, {{scale, ctx->scale.p, D},
+	                       {ctx->beta_set ? beta : nullptr, ctx->beta.p, D},
+	                       {ctx->beta_set ? beta_start : nullptr, ctx->beta_start.p, D},
+	                       {fcounts, ctx->fcounts.p, N * sizeof(int)},
+	                       {sum_fact, ctx->sum_fact.p, D},
+	                       {blacklist, ctx->blacklist.p, N}});
 }
 
 extern "C" int dfg_get_scalars(dfg_ctx *ctx, double *out) {
@@ -3884,25 +3957,22 @@ extern "C" int dfg_slice_gen(dfg_ctx *ctx, const double *quat, int mode, double 
 	NEED(mode >= 0 && mode < ctx->M, DFG_ERR_ARG, "slice_gen: mode %d out of range", mode);
 	CK(cudaSetDevice(ctx->device));
 	CK(ctx->scalars.ensure(8));
-	DevBuf<double> q, o;
-	double g[8];
-	const int ng = orientation_params(ctx, quat, g);
-	CK(upload(q, g, (size_t)ng, ctx->stream));
-	CK(o.ensure((size_t)ctx->P));
+	OneOrientation g{};
+	orientation_params(ctx, quat, g.v);
+	CK(ctx->one_out.ensure((size_t)ctx->P));
 	const unsigned nb = blocks_for(ctx->P, 256);
+#define DFG_SLICE_ONE(G)                                                                                       \
+	slice_one_kernel<G><<<nb, 256, 0, ctx->stream>>>(g, mode, ctx->qvals.p, ctx->corr.p, ctx->P, ctx->model1.p,  \
+	                                                 ctx->S, ctx->V, ctx->one_out.p)
 	if (ctx->model_type == MT_2D)
-		slice_one_kernel<MT_2D><<<nb, 256, 0, ctx->stream>>>(q.p, mode, ctx->qvals.p, ctx->corr.p, ctx->P,
-		                                                     ctx->model1.p, ctx->S, ctx->V, o.p);
+		DFG_SLICE_ONE(MT_2D);
 	else if (ctx->model_type == MT_RZ)
-		slice_one_kernel<MT_RZ><<<nb, 256, 0, ctx->stream>>>(q.p, mode, ctx->qvals.p, ctx->corr.p, ctx->P,
-		                                                     ctx->model1.p, ctx->S, ctx->V, o.p);
+		DFG_SLICE_ONE(MT_RZ);
 	else
-		slice_one_kernel<MT_3D><<<nb, 256, 0, ctx->stream>>>(q.p, mode, ctx->qvals.p, ctx->corr.p, ctx->P,
-		                                                     ctx->model1.p, ctx->S, ctx->V, o.p);
+		DFG_SLICE_ONE(MT_3D);
+#undef DFG_SLICE_ONE
 	CKL("slice_one_kernel");
-	CK(cudaMemcpyAsync(out, o.p, (size_t)ctx->P * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-	CK(cudaStreamSynchronize(ctx->stream));
-	return DFG_OK;
+	return fetch_all(ctx, {{out, ctx->one_out.p, (size_t)ctx->P * sizeof(double)}});
 }
 
 extern "C" int dfg_slice_merge(dfg_ctx *ctx, const double *quat, int mode, const double *view, double *model2,

@@ -205,6 +205,8 @@ struct dfg_ctx {
 	DevBuf<int> prob_count, d_place;
 	DevBuf<long long> d_prob_off;
 	DevBuf<double> d_prob, tomo_out;
+	DevBuf<double> one_out;    // the slice of dfg_slice_gen
+	HostBuf<uint8_t> stage_out;  // page-locked staging of small results (kStageBytes)
 	// dense (tensor-core) form of the E-step photon term. estep_form 0 =
 	// sparse gathers, 1 = dense, 2 = chosen by the autotuner; dense_active is
 	// this iteration's choice. K mask-0 pixels (kpix [K] their indices, pcol

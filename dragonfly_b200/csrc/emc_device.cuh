@@ -1974,8 +1974,13 @@ __global__ void __launch_bounds__(256) voronoi_kernel(const double *__restrict__
 // One slice, un-logged (Model.slice_gen, model.c:11-59)
 // (slice_gen2d / slice_genrz, model.c:65-150, for 2-D and RZ models: g holds
 // the quaternion, or (cos, sin) of the angle, or the five RZ parameters)
+// (by value: no upload before the launch)
+struct OneOrientation {
+	double v[8];
+};
+
 template <int GEO>
-__global__ void slice_one_kernel(const double *__restrict__ g, int mode, const double *__restrict__ qvals,
+__global__ void slice_one_kernel(const OneOrientation g, int mode, const double *__restrict__ qvals,
                                  const double *__restrict__ corr, int P, const double *__restrict__ model,
                                  long long S, long long V, double *__restrict__ out) {
 	int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1983,10 +1988,10 @@ __global__ void slice_one_kernel(const double *__restrict__ g, int mode, const d
 		return;
 	double rot[9];
 	if constexpr (GEO == MT_3D)
-		rot_from_quat(g, rot);
+		rot_from_quat(g.v, rot);
 	else
 		for (int k = 0; k < 5; ++k)
-			rot[k] = g[k];
+			rot[k] = g.v[k];
 	out[p] = geo_sample<GEO>(rot, qvals[3 * (size_t)p], qvals[3 * (size_t)p + 1], qvals[3 * (size_t)p + 2],
 	                         (double)(S / 2), S, model + (size_t)mode * V, corr[p]);
 }
