@@ -250,6 +250,29 @@ __global__ void __launch_bounds__(256) sum_splits_kernel(const float *__restrict
 	}
 }
 
+// The same for at most 8 splits: sum_splits_kernel's order is then the splits'
+// own, which one thread per four elements adds without shared memory (1048576
+// elements of 4 splits 30 -> 5 us). n and the pointers are multiples of 4 floats.
+__global__ void __launch_bounds__(256) sum_few_splits_kernel(const float4 *__restrict__ part, int S, long long n4,
+                                                             float4 *__restrict__ out) {
+	const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+	if (i >= n4)
+		return;
+	float4 v[8];
+#pragma unroll
+	for (int z = 0; z < 8; ++z)
+		v[z] = z < S ? __ldg(part + z * n4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+	float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+	for (int z = 0; z < 8; ++z) {
+		t.x += 0.f + v[z].x;
+		t.y += 0.f + v[z].y;
+		t.z += 0.f + v[z].z;
+		t.w += 0.f + v[z].w;
+	}
+	out[i] = t;
+}
+
 // *acc += sum of loss[0, n) (one block, fixed-order tree).
 __global__ void __launch_bounds__(256) loss_sum_kernel(const float *__restrict__ loss, int n, double *__restrict__ acc) {
 	__shared__ double s[256];
@@ -302,8 +325,11 @@ __global__ void __launch_bounds__(256) colsum_part_kernel(const float *__restric
 			out[threadIdx.x] = t;
 		}
 	} else {
-		for (int c = threadIdx.x; c < cols; c += 256) {
+		// blockIdx.y: 256 columns each
+		const int c = blockIdx.y * 256 + threadIdx.x;
+		if (c < cols) {
 			float acc = 0.f;
+#pragma unroll 8
 			for (long long r = r0; r < r1; ++r)
 				acc += dY[r * cols + c];
 			out[c] = acc;
@@ -312,14 +338,27 @@ __global__ void __launch_bounds__(256) colsum_part_kernel(const float *__restric
 }
 
 // out[c] = sum over b < nb of part[b][c], b in order.
-__global__ void colsum_final_kernel(const float *__restrict__ part, int nb, int cols, float *__restrict__ out) {
-	const int c = blockIdx.x * blockDim.x + threadIdx.x;
-	if (c >= cols)
-		return;
+// (32 columns per block of 32 x 8 threads, 64 partials at a time through shared
+// memory: added by one thread per column straight from memory, 296 partials took 18 us)
+__global__ void __launch_bounds__(256) colsum_final_kernel(const float *__restrict__ part, int nb, int cols,
+                                                           float *__restrict__ out) {
+	__shared__ float s[64][33];
+	const int c = blockIdx.x * 32 + threadIdx.x;
 	float t = 0.f;
-	for (int b = 0; b < nb; ++b)
-		t += part[(size_t)b * cols + c];
-	out[c] = t;
+	for (int b0 = 0; b0 < nb; b0 += 64) {
+		const int n = min(64, nb - b0);
+#pragma unroll
+		for (int k = threadIdx.y; k < 64; k += 8)
+			if (k < n && c < cols)
+				s[k][threadIdx.x] = part[(size_t)(b0 + k) * cols + c];
+		__syncthreads();
+		if (threadIdx.y == 0)
+			for (int k = 0; k < n; ++k)
+				t += s[k][threadIdx.x];
+		__syncthreads();
+	}
+	if (threadIdx.y == 0 && c < cols)
+		out[c] = t;
 }
 
 // Layer 0's weight and bias gradients (cout 32, K = 9 taps of one channel),
@@ -810,19 +849,37 @@ __global__ void __launch_bounds__(192, 1) pnet_gemm_tc_kernel(const __grid_const
 		}
 		tc_fence_after();
 		if (ok && !*abort_flag) {
+			// a lane holds a row: four columns per store where C's rows are 16-byte
+			// aligned (single columns cost a sector each: 65536 x 288 outputs of
+			// 64-deep products 155 -> 51 us)
+			const bool vec = (ldc & 3) == 0 && ((uintptr_t)C & 15) == 0;
 			for (int c = 0; c < BN / 16; ++c) {
 				float v[16];
+				const int col0 = nt * BN + c * 16;
+				if (col0 >= N)
+					break;
 				tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 16), v);
 				if (row < M) {
 #pragma unroll
-					for (int j = 0; j < 16; ++j) {
-						const int col = nt * BN + c * 16 + j;
-						if (col < N) {
-							const float x = bias != nullptr ? v[j] + bias[col] : v[j];
-							C[(size_t)row * ldc + col] = relu ? fmaxf(x, 0.f) : x;
+					for (int j = 0; j < 16; ++j)
+						if (col0 + j < N) {
+							const float x = bias != nullptr ? v[j] + bias[col0 + j] : v[j];
+							v[j] = relu ? fmaxf(x, 0.f) : x;
+						}
+					float *out = C + (size_t)row * ldc + col0;
+#pragma unroll
+					for (int j = 0; j < 16; j += 4) {
+						if (vec && col0 + j + 3 < N) {
+							*reinterpret_cast<float4 *>(out + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+						} else {
+#pragma unroll
+							for (int e = 0; e < 4; ++e)
+								if (col0 + j + e < N)
+									out[j + e] = v[j + e];
 						}
 					}
 				}
+				__syncwarp();
 			}
 		}
 	}
@@ -946,30 +1003,49 @@ __global__ void gather_rows_kernel(const float *__restrict__ src, const int *__r
 		lab_out[e] = lab[idx[e]];
 }
 
-// Y[c][r] = bf16(X[r][c]) for r < rows, 0 for rows <= r < rows_p: a 32 x 32
+// Y[c][r] = bf16(X[r][c]) for r < rows, 0 for rows <= r < rows_p: a 64 x 64
 // tile through shared memory per block (coalesced reads of X's rows and
-// writes of Y's rows). Grid: ceil(cols / 32) x ceil(rows_p / 32), 32 x 8
+// writes of Y's rows). Grid: ceil(cols / 64) x ceil(rows_p / 64), 32 x 8
 // threads.
 template <typename T>
 __global__ void transpose_bf16_kernel(const T *__restrict__ X, long long rows, int cols, long long rows_p,
                                       __nv_bfloat16 *__restrict__ Y) {
-	__shared__ float tile[32][33];
-	const int c0 = blockIdx.x * 32;
-	const long long r0 = (long long)blockIdx.y * 32;
-	for (int k = threadIdx.y; k < 32; k += 8) {
+	// 64 x 64 tiles, two elements per thread both ways (32 x 32 with one: 65536 x
+	// 320 BF16 52 -> 32 us); rows_p is even, an odd cols is read by singles
+	__shared__ __nv_bfloat16 tile[64][66];
+	const bool pairs = (cols & 1) == 0;
+	const int c0 = blockIdx.x * 64;
+	const long long r0 = (long long)blockIdx.y * 64;
+	for (int k = threadIdx.y; k < 64; k += 8) {
 		const long long r = r0 + k;
-		const int c = c0 + threadIdx.x;
-		float v = 0.f;
-		if (r < rows && c < cols)
-			v = (float)X[r * cols + c];
-		tile[k][threadIdx.x] = v;
+		const int c = c0 + 2 * threadIdx.x;
+		float a = 0.f, b = 0.f;
+		if (r < rows && c < cols && !pairs) {
+			a = (float)X[r * cols + c];
+			b = c + 1 < cols ? (float)X[r * cols + c + 1] : 0.f;
+		} else if (r < rows && c < cols) {
+			if constexpr (sizeof(T) == 2) {
+				const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162 *>(X + r * cols + c);
+				a = __low2float(x);
+				b = __high2float(x);
+			} else {
+				const float2 x = *reinterpret_cast<const float2 *>(X + r * cols + c);
+				a = x.x;
+				b = x.y;
+			}
+		}
+		*reinterpret_cast<__nv_bfloat162 *>(&tile[k][2 * threadIdx.x]) = __floats2bfloat162_rn(a, b);
 	}
 	__syncthreads();
-	for (int k = threadIdx.y; k < 32; k += 8) {
+	for (int k = threadIdx.y; k < 64; k += 8) {
 		const int c = c0 + k;
-		const long long r = r0 + threadIdx.x;
-		if (c < cols && r < rows_p)
-			Y[(size_t)c * rows_p + r] = __float2bfloat16(tile[threadIdx.x][k]);
+		const long long r = r0 + 2 * threadIdx.x;
+		if (c < cols && r < rows_p) {
+			__nv_bfloat162 y;
+			y.x = tile[2 * threadIdx.x][k];
+			y.y = tile[2 * threadIdx.x + 1][k];
+			*reinterpret_cast<__nv_bfloat162 *>(Y + (size_t)c * rows_p + r) = y;
+		}
 	}
 }
 
@@ -1053,6 +1129,17 @@ struct dfg_pnet {
 
 static unsigned grid_for(long long n) { return (unsigned)std::min<long long>((n + 255) / 256, 1 << 20); }
 
+// C [n] = the sum of S partial products in split order.
+static int sum_splits(dfg_pnet *net, const float *part, int S, long long n, float *C) {
+	if (S <= 8 && n % 4 == 0 && (((uintptr_t)part | (uintptr_t)C) & 15) == 0)
+		sum_few_splits_kernel<<<(unsigned)((n / 4 + 255) / 256), 256, 0, net->stream>>>(
+		    reinterpret_cast<const float4 *>(part), S, n / 4, reinterpret_cast<float4 *>(C));
+	else
+		sum_splits_kernel<<<(unsigned)((n + 31) / 32), dim3(32, 8), 0, net->stream>>>(part, S, n, C);
+	PKL("sum_splits_kernel");
+	return DFG_OK;
+}
+
 // Split of the k range of an M x N product so that the grid fills about two
 // blocks per SM (chunks of at least 512, multiples of 16): (splits, chunk).
 static void k_split(int M, int N, long long K, int *S, int *chunk) {
@@ -1086,10 +1173,7 @@ static int gemm_wgrad(dfg_pnet *net, int M, int N, int K, const float *A, const 
 	                                                                      net->wsplit.p, N, chunk,
 	                                                                      (long long)M * N);
 	PKL("gemm_kernel");
-	sum_splits_kernel<<<(unsigned)(((long long)M * N + 31) / 32), dim3(32, 8), 0, net->stream>>>(net->wsplit.p, S,
-	                                                                                          (long long)M * N, C);
-	PKL("sum_splits_kernel");
-	return DFG_OK;
+	return sum_splits(net, net->wsplit.p, S, (long long)M * N, C);
 }
 
 // dX [B][H][H][C] from the column gradients of a 3 x 3 convolution.
@@ -1115,9 +1199,10 @@ static int bias_grad(dfg_pnet *net, const float *dY, long long rows, int cols, f
 	const int nb = (int)((rows + chunk - 1) / chunk);
 	if ((size_t)nb * cols > net->gpart.n)
 		PK(net->gpart.ensure((size_t)nb * cols));
-	colsum_part_kernel<<<nb, 256, 0, net->stream>>>(dY, rows, cols, chunk, net->gpart.p);
+	const unsigned cb = 256 % cols == 0 ? 1u : (unsigned)((cols + 255) / 256);
+	colsum_part_kernel<<<dim3(nb, cb), 256, 0, net->stream>>>(dY, rows, cols, chunk, net->gpart.p);
 	PKL("colsum_part_kernel");
-	colsum_final_kernel<<<(cols + 255) / 256, 256, 0, net->stream>>>(net->gpart.p, nb, cols, db);
+	colsum_final_kernel<<<(cols + 31) / 32, dim3(32, 8), 0, net->stream>>>(net->gpart.p, nb, cols, db);
 	PKL("colsum_final_kernel");
 	return DFG_OK;
 }
@@ -1367,8 +1452,8 @@ static int tc_product(dfg_pnet *net, const __nv_bfloat16 *A, long long M, int Kp
 #undef DFG_TC
 	PKL("pnet_gemm_tc_kernel");
 	if (S > 1) {
-		sum_splits_kernel<<<(unsigned)((M * N + 31) / 32), dim3(32, 8), 0, net->stream>>>(net->tsplit.p, S, M * N, C);
-		PKL("sum_splits_kernel");
+		if (int rc = sum_splits(net, net->tsplit.p, S, M * N, C))
+			return rc;
 		if (bias != nullptr) {
 			bias_act_kernel<<<grid_for(M * N), 256, 0, net->stream>>>(C, M, N, bias, relu);
 			PKL("bias_act_kernel");
@@ -1464,10 +1549,10 @@ static int backward_tc(dfg_pnet *net, const float *X, const int *lab, int n, con
 		const long long rows_p = (rows + 63) / 64 * 64;
 		// dW [cout][K] = dY^T X: both operands with the batch rows as the reduction
 		dim3 tb(32, 8);
-		transpose_bf16_kernel<float><<<dim3((s.cout + 31) / 32, (unsigned)(rows_p / 32)), tb, 0, st>>>(
+		transpose_bf16_kernel<float><<<dim3((s.cout + 63) / 64, (unsigned)((rows_p + 63) / 64)), tb, 0, st>>>(
 		    dY, rows, s.cout, rows_p, net->dyt.p);
 		PKL("transpose_bf16_kernel");
-		transpose_bf16_kernel<__nv_bfloat16><<<dim3((Kp + 31) / 32, (unsigned)(rows_p / 32)), tb, 0, st>>>(
+		transpose_bf16_kernel<__nv_bfloat16><<<dim3((Kp + 63) / 64, (unsigned)((rows_p + 63) / 64)), tb, 0, st>>>(
 		    net->colsbl[l].p, rows, Kp, rows_p, net->colst.p);
 		PKL("transpose_bf16_kernel");
 		if (int rc = tc_product(net, net->dyt.p, s.cout, (int)rows_p, net->colst.p, K, net->gw[l].p, nullptr, 0))
