@@ -1279,6 +1279,23 @@ static int encode_byte_map(dfg_ctx *ctx, CUtensorMap *map, const void *base, lon
 // 8.5 / 8.5 / 8.6 / 9.5 against 39.6.
 constexpr double kHotOccupancy = 0.012;
 
+// Tensor map of a chunk's log-likelihoods [tiles][nc][128] in FP64, written in
+// boxes of 16 orientations x 32 frames of one tile with the 128-byte swizzle (frames
+// past the chunk's are clipped).
+static int encode_pval_map(dfg_ctx *ctx, CUtensorMap *map, const void *base, int nc, int tiles) {
+	auto fn = tensor_map_encoder();
+	NEED(fn != nullptr, DFG_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+	cuuint64_t dims[3] = {(cuuint64_t)TILE, (cuuint64_t)nc, (cuuint64_t)tiles};
+	cuuint64_t strides[2] = {TILE * sizeof(double), (cuuint64_t)nc * TILE * sizeof(double)};
+	cuuint32_t box[3] = {16, 32, 1};
+	cuuint32_t estr[3] = {1, 1, 1};
+	const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<void *>(base), dims, strides, box, estr,
+	                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+	                      CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+	NEED(r == CUDA_SUCCESS, DFG_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+	return DFG_OK;
+}
+
 // Chooses the hot pixels of the current chunk layout and lays out what depends
 // on the frames alone: the count matrices of every chunk and the photon lists
 // without them. hot_n = 0 leaves everything to the gathers.
@@ -1486,9 +1503,12 @@ static int hot_prepare(dfg_ctx *ctx) {
 	CK(ctx->rowmax_part.ensure((size_t)psum_splits(ctx) * ctx->R_pad));
 	CK(ctx->derr.ensure(1));
 	CK(cudaMemsetAsync(ctx->derr.p, 0, sizeof(int), ctx->stream));
-	for (Chunk &ch : ctx->chunks)
+	for (Chunk &ch : ctx->chunks) {
 		if (int rc = encode_byte_map(ctx, &ch.map_pdig, ctx->pval.p, rows, ch.k_pitch))
 			return rc;
+		if (int rc = encode_pval_map(ctx, &ch.map_pval, ctx->pval.p, ch.nc, ctx->RT))
+			return rc;
+	}
 	CK(cudaFuncSetAttribute(hot_product_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, HSMEM_BYTES));
 	CK(cudaFuncSetAttribute(hot_product_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HSMEM_BYTES));
 	ctx->hot_active = true;
@@ -1513,8 +1533,7 @@ static int launch_hot_digits(dfg_ctx *ctx) {
 static int launch_hot_estep(dfg_ctx *ctx, const Chunk &ch) {
 	const int OT = ctx->RT * 2, FT = (ch.nc + HM - 1) / HM;
 	hot_product_kernel<false><<<hot_grid(ctx, (long long)OT * FT), HTHREADS, HSMEM_BYTES, ctx->stream>>>(
-	    ch.map_frame, ctx->map_wdig, ctx->hot_pitch / HK, OT, FT, ch.nc, HotOut{ctx->pval.p, nullptr, nullptr, nullptr, 0, 0},
-	    ctx->derr.p, ctx->dense_wait_cycles, ctx->dense_withhold);
+	    ch.map_frame, ctx->map_wdig, ch.map_pval, ctx->hot_pitch / HK, OT, FT, ch.nc, HotOut{}, ctx->derr.p, ctx->dense_wait_cycles, ctx->dense_withhold);
 	CKL("hot_product_kernel");
 	return DFG_OK;
 }
@@ -1528,8 +1547,8 @@ static int launch_hot_mstep(dfg_ctx *ctx, const Chunk &ch) {
 	CKL("hot_digits_kernel");
 	const int OT = ctx->RT * 2, FT = (ctx->hot_n + HM - 1) / HM;
 	hot_product_kernel<true><<<hot_grid(ctx, (long long)OT * FT), HTHREADS, HSMEM_BYTES, st>>>(
-	    ch.map_pixel, ch.map_pdig, ch.k_pitch / HK, OT, FT, ctx->hot_n,
-	    HotOut{nullptr, ctx->T.p, ctx->hot_pix.p, ctx->rowmax.p, ctx->P, ch.d0 == 0 ? 1 : 0}, ctx->derr.p,
+	    ch.map_pixel, ch.map_pdig, ch.map_pval, ch.k_pitch / HK, OT, FT, ctx->hot_n,
+	    HotOut{ctx->T.p, ctx->hot_pix.p, ctx->rowmax.p, ctx->P, ch.d0 == 0 ? 1 : 0}, ctx->derr.p,
 	    ctx->dense_wait_cycles, ctx->dense_withhold);
 	CKL("hot_product_kernel");
 	return DFG_OK;

@@ -98,13 +98,13 @@ struct Chunk {
 	long long entries = 0;
 	// hot pixels (emc_hot.cuh): counts as bytes [nc][hot_pitch] and
 	// [hot_n][k_pitch] (k_pitch = nc rounded up to 128), their tensor maps and
-	// that of the chunk's probability digits, and the pixels left to the gathers
+	// those of the chunk's probability digits and log-likelihoods, and the pixels left to the gathers
 	DevBuf<uint8_t> by_frame, by_pixel;
 	DevBuf<int> pix_cold;
 	DevBuf<uint32_t> csc;      // their frame lists
 	DevBuf<long long> csc_off, csc_mid;
 	int npix_cold = 0, k_pitch = 0;
-	CUtensorMap map_frame, map_pixel, map_pdig;
+	CUtensorMap map_frame, map_pixel, map_pdig, map_pval;
 };
 
 }  // namespace dfg

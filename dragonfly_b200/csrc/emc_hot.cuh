@@ -53,7 +53,8 @@ constexpr int HSTAGES = 3;
 constexpr int HA_BYTES = HM * HK;
 constexpr int HB_BYTES = 4 * HO * HK;
 constexpr int HSTAGE_BYTES = HA_BYTES + HB_BYTES;  // 64 KB
-constexpr int HSMEM_BYTES = 1024 + HSTAGES * HSTAGE_BYTES + 128;
+constexpr int HOUT_BYTES = 32 * 128;                // one warp's 32 rows x 16 doubles on their way out
+constexpr int HSMEM_BYTES = 1024 + HSTAGES * HSTAGE_BYTES + 8 * HOUT_BYTES + 128;
 constexpr int HTHREADS = 320;
 constexpr int HGROUP = 12;   // orientation tiles per rasterisation group: 12 x 12 resident tiles share operands in L2
 constexpr float HE_SCALE = 67108864.f;  // log-slices in steps of 2^-26
@@ -106,12 +107,26 @@ __device__ __forceinline__ double join_digits(uint32_t d0, uint32_t d1, uint32_t
 	return fma(v, 256., i32_to_f64(d0));
 }
 
+// 3-D tiled TMA store from this CTA's shared memory, and the waits for the
+// stores of this thread: until they have read it, until they are done.
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, const void *src, int x, int y, int z) {
+	asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+	                 (uint64_t)map),
+	             "r"(smem_addr(src)), "r"(x), "r"(y), "r"(z)
+	             : "memory");
+	asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void tma_store_wait_read() {
+	asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+__device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // Where a tile's sums go. MSTEP false: pval[tile][frame][128] (FP64 photon sums
-// of the hot pixels; rows = frames); true: T[tile][pix[row]][128] += sum x
+// of the hot pixels; rows = frames), by TMA through map_out, whose rows past the
+// chunk's frames are clipped; true: T[tile][pix[row]][128] += sum x
 // rmax[r] / HP_STEPS (rows = hot pixels; overwritten for the first chunk,
 // whose tomograms are zero).
 struct HotOut {
-	double *pval;
 	float *T;
 	const int *pix;     // hot pixel of each row
 	const float *rmax;  // [R_pad] largest probability of each orientation in the chunk
@@ -120,11 +135,12 @@ struct HotOut {
 
 template <bool MSTEP>
 __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
-    const __grid_constant__ CUtensorMap map_cnt, const __grid_constant__ CUtensorMap map_dig, int num_kb, int OT,
-    int FT, int nrows, HotOut out, int *__restrict__ err, long long wait_cycles, int withhold_kb) {
+    const __grid_constant__ CUtensorMap map_cnt, const __grid_constant__ CUtensorMap map_dig,
+    const __grid_constant__ CUtensorMap map_out, int num_kb, int OT, int FT, int nrows, HotOut out, int *__restrict__ err, long long wait_cycles, int withhold_kb) {
 	extern __shared__ uint8_t hsm_raw[];
 	uint8_t *sm = (uint8_t *)(((uintptr_t)hsm_raw + 1023) & ~(uintptr_t)1023);
-	uint64_t *bars = (uint64_t *)(sm + HSTAGES * HSTAGE_BYTES);
+	uint8_t *outs = sm + HSTAGES * HSTAGE_BYTES;
+	uint64_t *bars = (uint64_t *)(outs + 8 * HOUT_BYTES);
 	uint64_t *full = bars, *empty = bars + HSTAGES, *tfull = bars + 2 * HSTAGES, *tempty = tfull + 1;
 	uint32_t *tmem_slot = (uint32_t *)(tempty + 1);
 	volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
@@ -255,12 +271,8 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 			tc_fence_after();
 			const int rt = ot >> 1, j0 = (ot & 1) * HO, row = ft * HM + i;
 			const bool valid = row < nrows;
-			double *pv = nullptr;
-			float *tp = nullptr;
-			if constexpr (MSTEP)
-				tp = out.T + ((size_t)rt * out.P + (valid ? out.pix[row] : 0)) * TILE + j0;
-			else
-				pv = out.pval + ((size_t)rt * nrows + (valid ? row : 0)) * TILE + j0;
+			float *const tp =
+			    MSTEP ? out.T + ((size_t)rt * out.P + (valid ? out.pix[row] : 0)) * TILE + j0 : nullptr;
 			// all sums into registers first, so that the next tile's products
 			// run while this one's results are stored (the stores alone take about
 			// 10000 cycles a tile, as long as the products over 1250 pixels)
@@ -281,8 +293,8 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 			__syncwarp();
 			if (lane == 0)
 				mbar_arrive(tempty);
-			if (valid) {
-				if constexpr (MSTEP) {
+			if constexpr (MSTEP) {
+				if (valid) {
 					const float *rm = out.rmax + (size_t)rt * TILE + j0;
 #pragma unroll
 					for (int k = 0; k < HO; k += 4) {
@@ -298,17 +310,35 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 							o[e] = (float)((double)o[e] + v[k + e] * ((double)rr[e] * (1. / HP_STEPS)));
 						*dst = make_float4(o[0], o[1], o[2], o[3]);
 					}
-				} else {
+				}
+			} else {
+				// rows are a KB apart: stored from the lanes, each instruction touched
+				// 32 lines. 16 doubles of every row go to shared memory (128-byte
+				// swizzle, as the tensor map has it) and leave as one TMA store.
+				uint8_t *const mine = outs + (warp - 2) * HOUT_BYTES;
+				const int row0 = ft * HM + m * 128 + q * 32;
+				if (row0 < nrows) {
 #pragma unroll
-					for (int k = 0; k < HO; k += 4)  // 32 bytes per lane: a whole sector in one store
-						asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(pv + k),
-						             "d"(v[k] * (1. / HE_SCALE)), "d"(v[k + 1] * (1. / HE_SCALE)),
-						             "d"(v[k + 2] * (1. / HE_SCALE)), "d"(v[k + 3] * (1. / HE_SCALE))
-						             : "memory");
+					for (int c = 0; c < HO / 16; ++c) {
+						if (lane == 0)
+							tma_store_wait_read();
+						__syncwarp();
+#pragma unroll
+						for (int k = 0; k < 8; ++k)
+							*reinterpret_cast<double2 *>(mine + lane * 128 + ((k ^ (lane & 7)) << 4)) =
+							    make_double2(v[c * 16 + 2 * k] * (1. / HE_SCALE), v[c * 16 + 2 * k + 1] * (1. / HE_SCALE));
+						asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+						__syncwarp();
+						if (lane == 0)
+							tma_store_3d(&map_out, mine, j0 + c * 16, row0, rt);
+					}
 				}
 			}
 			__syncwarp();
 		}
+		if (!MSTEP && lane == 0)
+			tma_store_wait();
+		__syncwarp();
 	}
 	tc_fence_before();
 	__syncthreads();
