@@ -2627,7 +2627,8 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 				return rc;
 		if (int rc = launch_estep(ctx, ch, use_scale, bg, rm, ctx->dense_active))
 			return rc;
-		phase_end(ctx, PH_ESTEP, (ctx->dense_active || ctx->m_dense_active ? 1 : 0) + 1);
+		phase_end(ctx, PH_ESTEP,
+		          (ctx->dense_active || ctx->m_dense_active ? 1 : 0) + (ctx->hot_estep && !ctx->dense_active ? 1 : 0) + 1);
 		// normalisation and per-frame sums (normalize_prob + calc_psum_r)
 		phase_begin(ctx, PH_NORM);
 		if (int rc = launch_norm(ctx, ch, psum_d_on, bg))
@@ -2672,7 +2673,7 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 				CKL("mstep_bg_kernel");
 			}
 		}
-		phase_end(ctx, PH_MSTEP, ctx->m_dense_active ? 2 : (ch.npix > 0 ? 1 : 0));
+		phase_end(ctx, PH_MSTEP, ctx->m_dense_active ? 2 : (ch.npix > 0 ? 1 : 0) + (ctx->hot_active ? 2 : 0));
 	}
 
 	// merge (merge_tomogram -> slice_merge3d); the weight grid is rebuilt only
