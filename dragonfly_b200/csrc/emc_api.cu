@@ -751,22 +751,26 @@ static int build_chunks(dfg_ctx *ctx) {
 				}
 			}
 		};
-		// per range and pixel: count-1 words, counted words, photons, counts past
-		// a byte; then the cursors of the two segments
+		// per range and pixel: count-1 words, counted words, photons, the last frame
+		// that lists it, and whether the byte products cannot hold it (a count past
+		// a byte, or two entries of one frame); then the cursors of the two segments
 		std::vector<long long> c1((size_t)nth * P, 0), cm((size_t)nth * P, 0), photons((size_t)nth * P, 0);
 		std::vector<uint8_t> big((size_t)nth * P, 0);
+		std::vector<int> last((size_t)nth * P, -1);
 		parallel_ranges(ch.nc, nth, [&](int th, long long b, long long e) {
 			long long *t1 = c1.data() + (size_t)th * P, *tm = cm.data() + (size_t)th * P;
 			long long *tp = photons.data() + (size_t)th * P;
 			uint8_t *tb = big.data() + (size_t)th * P;
-			each(b, e, [&](int p, int, long long c) {
+			int *tl = last.data() + (size_t)th * P;
+			each(b, e, [&](int p, int dl, long long c) {
 				if (c == 1)
 					t1[p]++;
 				else
 					tm[p] += (c + MAX_COUNT - 1) / MAX_COUNT;
 				tp[p] += c;
-				if (c > 255)
+				if (c > 255 || tl[p] == dl)
 					tb[p] = 1;
+				tl[p] = dl;
 			});
 		});
 		std::vector<long long> off(P + 1, 0), midv(P, 0), end1(P), endm(P);
@@ -2600,7 +2604,7 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 		    (__nv_bfloat16 *)ctx->Alo.p);
 		CKL("split_logw_kernel");
 	}
-	const bool hot_e = ctx->hot_active && ctx->hot_estep;
+	const bool hot_e = ctx->hot_estep && !ctx->dense_active;
 	if (hot_e)
 		if (int rc = launch_hot_digits(ctx))
 			return rc;

@@ -245,7 +245,7 @@ struct dfg_ctx {
 	bool hot_estep = false;    // and the E-step's
 	double refine_live = -1.;  // share of (tile, frame) pairs a refinement evaluates; -1 = not counted
 	std::vector<long long> h_pix_entries;  // [P] photon words over all chunks
-	std::vector<uint8_t> h_pix_big;        // [P] counts that the byte products cannot hold
+	std::vector<uint8_t> h_pix_big;        // [P] not for the byte products (build_chunks)
 	DevBuf<int> hot_pix, hot_special;
 	DevBuf<uint8_t> is_hot;
 	DevBuf<uint32_t> phc;

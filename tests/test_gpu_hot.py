@@ -16,7 +16,7 @@ from dragonfly_b200 import synth
 pytestmark = pytest.mark.gpu
 
 
-def _problem(frames, div, side, photons, zeros=False, big=False):
+def _problem(frames, div, side, photons, zeros=False, big=False, twice=False):
     d = synth.small_problem(seed=frames + div, det_side=side, size=side + 3, qmax=side / 2., n_atoms=60,
                             atom_radius=4., num_div=div, n_frames=frames, mean_count=photons, hole_radius=2.)
     model = d["model_start"] * photons / (d["mask"] == 0).sum() * 2.
@@ -27,7 +27,11 @@ def _problem(frames, div, side, photons, zeros=False, big=False):
     if big:     # counts past a byte keep their pixels out of the products
         count[::97] = 300
         count[5] = 1200
-    return EMCProblem(d["qvals"], d["corr"], d["mask"], d["ones"], d["multi"], d["place_ones"], d["place_multi"],
+    place = d["place_ones"].copy()
+    if twice:   # a pixel listed twice in one frame: both photons count
+        mid = (np.cumsum(d["ones"]) - d["ones"] + d["ones"] // 2)[::3]
+        place[mid + 1] = place[mid]
+    return EMCProblem(d["qvals"], d["corr"], d["mask"], d["ones"], d["multi"], place, d["place_multi"],
                       count, d["quats"], model, need_scaling=1, update_scale=1, beta=0.1)
 
 
@@ -37,16 +41,17 @@ def _photons(prob):
     return n
 
 
-@pytest.mark.parametrize("frames,div,side,photons,zeros,big,budget", [
-    (256, 1, 24, 150., False, False, 0.),    # one row tile exactly, under half an orientation tile
-    (257, 2, 24, 200., False, False, 0.),    # one frame past it
-    (300, 2, 40, 100., False, False, 0.),    # some pixels left to the gathers
-    (800, 2, 24, 120., False, False, 2.0),   # chunks of 267 frames: tomograms added over three
-    (511, 1, 24, 200., True, False, 0.),     # tiles with log 0
-    (400, 2, 24, 250., False, True, 0.),     # counts past a byte
+@pytest.mark.parametrize("frames,div,side,photons,zeros,big,twice,budget", [
+    (256, 1, 24, 150., False, False, False, 0.),    # one row tile exactly, under half an orientation tile
+    (257, 2, 24, 200., False, False, False, 0.),    # one frame past it
+    (300, 2, 40, 100., False, False, False, 0.),    # some pixels left to the gathers
+    (800, 2, 24, 120., False, False, False, 2.0),   # chunks of 267 frames: tomograms added over three
+    (511, 1, 24, 200., True, False, False, 0.),     # tiles with log 0
+    (400, 2, 24, 250., False, True, False, 0.),     # counts past a byte
+    (300, 2, 40, 100., False, False, True, 0.),     # a pixel twice in a frame
 ])
-def test_products_match_oracle_and_gathers(oracle_built, frames, div, side, photons, zeros, big, budget):
-    prob = _problem(frames, div, side, photons, zeros, big)
+def test_products_match_oracle_and_gathers(oracle_built, frames, div, side, photons, zeros, big, twice, budget):
+    prob = _problem(frames, div, side, photons, zeros, big, twice)
     hot = GPUEngine(prob, pair_budget_mb=budget)
     plain = GPUEngine(prob, pair_budget_mb=budget, tile_skip=1)
     orc = OracleEngine(prob)
