@@ -1313,8 +1313,7 @@ static int hot_choose(dfg_ctx *ctx) {
 	ctx->hot_layout = ctx->layout;
 	ctx->phc.release();
 	for (Chunk &ch : ctx->chunks) {
-		ch.by_frame.release();
-		ch.by_pixel.release();
+		ch.counts.release();
 		ch.pix_cold.release();
 		ch.csc.release();
 	}
@@ -1351,23 +1350,22 @@ static int hot_choose(dfg_ctx *ctx) {
 	bool room = true;
 	for (Chunk &ch : ctx->chunks) {
 		ch.k_pitch = (ch.nc + HK - 1) / HK * HK;
-		cudaError_t e = fits(ch.by_frame.ensure((size_t)ch.nc * pitch));
-		if (e == cudaSuccess)
-			e = fits(ch.by_pixel.ensure((size_t)n * ch.k_pitch));
+		const size_t by_frame_n = (size_t)ch.nc * pitch, counts_n = by_frame_n + (size_t)n * ch.k_pitch;
+		const cudaError_t e = fits(ch.counts.ensure(counts_n));
 		if (e == cudaErrorMemoryAllocation) {
 			room = false;
 			break;
 		}
 		CK(e);
-		CK(cudaMemsetAsync(ch.by_frame.p, 0, (size_t)ch.nc * pitch, st));
-		CK(cudaMemsetAsync(ch.by_pixel.p, 0, (size_t)n * ch.k_pitch, st));
+		CK(cudaMemsetAsync(ch.counts.p, 0, counts_n, st));
+		uint8_t *by_frame = ch.counts.p, *by_pixel = ch.counts.p + by_frame_n;
 		hot_counts_kernel<<<blocks_for((long long)n * 32, 256), 256, 0, st>>>(
-		    ch.cs.p, ch.cs_off.p, ch.cs_mid.p, ctx->hot_pix.p, n, pitch, ch.nc, ch.k_pitch, ch.by_frame.p,
-		    ch.by_pixel.p);
+		    ch.cs.p, ch.cs_off.p, ch.cs_mid.p, ctx->hot_pix.p, n, pitch, ch.nc, ch.k_pitch, by_frame,
+		    by_pixel);
 		CKL("hot_counts_kernel");
-		if (int rc = encode_byte_map(ctx, &ch.map_frame, ch.by_frame.p, ch.nc, pitch))
+		if (int rc = encode_byte_map(ctx, &ch.map_frame, by_frame, ch.nc, pitch))
 			return rc;
-		if (int rc = encode_byte_map(ctx, &ch.map_pixel, ch.by_pixel.p, n, ch.k_pitch))
+		if (int rc = encode_byte_map(ctx, &ch.map_pixel, by_pixel, n, ch.k_pitch))
 			return rc;
 		std::vector<int> pix((size_t)ch.npix), rest;
 		if (ch.npix > 0)
@@ -1440,8 +1438,7 @@ static int hot_choose(dfg_ctx *ctx) {
 	if (!room) {
 		ctx->phc.release();
 		for (Chunk &ch : ctx->chunks) {
-			ch.by_frame.release();
-			ch.by_pixel.release();
+			ch.counts.release();
 			ch.pix_cold.release();
 			ch.csc.release();
 		}
@@ -3794,12 +3791,14 @@ struct FetchItem {
 	size_t bytes;
 };
 constexpr size_t kStageBytes = (size_t)1 << 20;
+constexpr size_t kStageStep = (size_t)1 << 16;  // locking pages takes time: no more than a call needs
 
 static int fetch_all(dfg_ctx *ctx, std::initializer_list<FetchItem> items) {
 	size_t total = 0;
 	for (const FetchItem &f : items)
 		total += f.host ? (f.bytes + 15) / 16 * 16 : 0;
-	const bool staged = total <= kStageBytes && ctx->stage_out.ensure(kStageBytes) == cudaSuccess;
+	const bool staged = total <= kStageBytes &&
+	                    ctx->stage_out.ensure((total + kStageStep - 1) / kStageStep * kStageStep) == cudaSuccess;
 	if (!staged)
 		cudaGetLastError();
 	size_t at = 0;

@@ -96,10 +96,10 @@ struct Chunk {
 	DevBuf<int> pix;           // pixels with non-empty lists, longest first
 	int npix = 0;
 	long long entries = 0;
-	// hot pixels (emc_hot.cuh): counts as bytes [nc][hot_pitch] and
+	// hot pixels (emc_hot.cuh): counts as bytes [nc][hot_pitch] and behind them
 	// [hot_n][k_pitch] (k_pitch = nc rounded up to 128), their tensor maps and
 	// those of the chunk's probability digits and log-likelihoods, and the pixels left to the gathers
-	DevBuf<uint8_t> by_frame, by_pixel;
+	DevBuf<uint8_t> counts;
 	DevBuf<int> pix_cold;
 	DevBuf<uint32_t> csc;      // their frame lists
 	DevBuf<long long> csc_off, csc_mid;
@@ -206,7 +206,7 @@ struct dfg_ctx {
 	DevBuf<long long> d_prob_off;
 	DevBuf<double> d_prob, tomo_out;
 	DevBuf<double> one_out;    // the slice of dfg_slice_gen
-	HostBuf<uint8_t> stage_out;  // page-locked staging of small results (kStageBytes)
+	HostBuf<uint8_t> stage_out;  // page-locked staging of small results (up to kStageBytes)
 	// dense (tensor-core) form of the E-step photon term. estep_form 0 =
 	// sparse gathers, 1 = dense, 2 = chosen by the autotuner; dense_active is
 	// this iteration's choice. K mask-0 pixels (kpix [K] their indices, pcol
