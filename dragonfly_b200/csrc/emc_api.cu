@@ -1862,6 +1862,11 @@ static int launch_estep(dfg_ctx *ctx, const Chunk &ch, int use_scale, bool bg, c
 			DFG_ECOLD(false, 4);
 #undef DFG_ECOLD
 		CKL("estep_cold_kernel");
+		estep_ties_kernel<<<blocks_for(Nc, 32), 256, 0, st>>>(
+		    ctx->logW.p, ctx->u.p, ctx->logw.p, R, ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p, ctx->scale.p,
+		    ctx->blacklist.p, ctx->fcounts.p, ch.d0, Nc, RT, use_scale, ctx->scalars.p, P, ctx->pval.p, ctx->tmax.p,
+		    ctx->targ.p);
+		CKL("estep_ties_kernel");
 		return DFG_OK;
 	}
 #define DFG_ESTEP(REF, MB)                                                                                    \
@@ -2629,7 +2634,7 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 		if (int rc = launch_estep(ctx, ch, use_scale, bg, rm, ctx->dense_active))
 			return rc;
 		phase_end(ctx, PH_ESTEP,
-		          (ctx->dense_active || ctx->m_dense_active ? 1 : 0) + (ctx->hot_estep && !ctx->dense_active ? 1 : 0) + 1);
+		          (ctx->dense_active || ctx->m_dense_active ? 1 : 0) + (ctx->hot_estep && !ctx->dense_active ? 2 : 0) + 1);
 		// normalisation and per-frame sums (normalize_prob + calc_psum_r)
 		phase_begin(ctx, PH_NORM);
 		if (int rc = launch_norm(ctx, ch, psum_d_on, bg))

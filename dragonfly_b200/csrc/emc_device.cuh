@@ -486,6 +486,162 @@ __global__ void __launch_bounds__(256, MINB) estep_cold_kernel(
 	}
 }
 
+// Near ties of the most likely orientation. The products add the log-slices
+// exactly, the gathers round once per photon word, so two orientations that agree
+// to a few parts in 1e9 could change places with the form of the E-step (one frame
+// of 40000 at 17220 orientations). Every orientation within the forms' rounding of
+// its frame's maximum is therefore summed again as estep_kernel does (the frame's
+// full lists, same order, same operations): where there are several, the
+// maximum and its orientation are those of the gathers, bit for bit.
+// Width: a compensated FP32 addition of x is off by at most 2u|x| (u = 2^-24, the
+// roundings of x - comp and, where |s| < |x|, of t - s), a digit by 2^-27. For both
+// forms and two orientations that is 8u sum|x| + n 2^-26 over n photons, and sum|x|
+// <= |sum x| + 2 n 31 while no log-slice is above 31; near_tie_width is twice that.
+// Block = 32 frames: the tile maxima are read with one frame per lane, then each warp
+// looks at four frames, listing the orientations of a frame and summing up to 32
+// of them at once, one per lane.
+__device__ __forceinline__ double near_tie_width(double sum, int photons) {
+	return 0x1p-20 * (fabs(sum) + 32. * photons);
+}
+
+__global__ void __launch_bounds__(256) estep_ties_kernel(
+    const float *__restrict__ logW, const double *__restrict__ u, const double *__restrict__ logw, int R,
+    const uint32_t *__restrict__ ph, const long long *__restrict__ ph_off, const long long *__restrict__ ph_mid,
+    const double *__restrict__ scale, const uint8_t *__restrict__ blacklist, const int *__restrict__ fcounts, int d0,
+    int Nc, int RT, int use_scale, const double *__restrict__ scalars, int P, double *pval, double *tmax, int *targ) {
+	__shared__ double s_m[8][32];
+	__shared__ int s_a[8][32];
+	__shared__ int s_list[8][64];
+	const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	{
+		const int dl = blockIdx.x * 32 + lane;
+		double m = MAX_EXP_START;
+		int am = -1;
+		if (dl < Nc && !blacklist[d0 + dl]) {
+#pragma unroll 8
+			for (int rt = w; rt < RT; rt += 8) {
+				const double v = tmax[(size_t)rt * Nc + dl];
+				if (v > m) {
+					m = v;
+					am = rt;
+				}
+			}
+			if (am >= 0)
+				am = targ[(size_t)am * Nc + dl];
+		}
+		s_m[w][lane] = m;
+		s_a[w][lane] = am;
+	}
+	__syncthreads();
+	int *const list = s_list[w];
+	for (int f = w; f < 32; f += 8) {
+		double m = MAX_EXP_START;
+		int am = -1;
+#pragma unroll
+		for (int k = 0; k < 8; ++k)
+			if (s_m[k][f] > m) {
+				m = s_m[k][f];
+				am = s_a[k][f];
+			}
+		if (am < 0)
+			continue;
+		const int dl = blockIdx.x * 32 + f, d = d0 + dl;
+		const double sd = use_scale ? scale[d] : scalars[0];
+		const double low = m - near_tie_width(m - (logw[am] - u[am] * sd), fcounts[d]);
+		const long long beg = ph_off[d], mid = ph_mid[d], end = ph_off[d + 1];
+		// the first n listed orientations, one per lane, as estep_kernel
+		auto again = [&](int n) {
+			__syncwarp();
+			if (lane < n) {
+				const int r = list[lane], rt = r / TILE, j = r % TILE;
+				const float *L = logW + (size_t)rt * (P + 1) * TILE + j;
+				const uint4 *w4 = reinterpret_cast<const uint4 *>(ph);
+				float s = 0.f, c = 0.f;
+				for (long long q = beg; q < end; q += 8) {
+					const uint4 a = __ldg(w4 + (q >> 2)), b = __ldg(w4 + (q >> 2) + 1);
+					const uint32_t e[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+					const bool ones = q < mid;
+					float v[8];
+#pragma unroll
+					for (int k = 0; k < 8; ++k)
+						v[k] = __ldg(L + (size_t)(ones ? e[k] : e[k] & IDX_MASK) * TILE);
+#pragma unroll
+					for (int k = 0; k < 8; ++k)
+						if (ones)
+							kahan_add(s, c, v[k]);
+						else
+							kahan_add_count(s, c, e[k] >> IDX_BITS, v[k]);
+				}
+				pval[((size_t)rt * Nc + dl) * TILE + j] = dadd(dsub(logw[r], dmul(u[r], sd)), kahan_value(s, c));
+			}
+			__syncwarp();
+		};
+		// calls f(rt, v) for every tile whose maximum is near, v its row's values of this lane
+		auto near_tiles = [&](auto &&f) {
+			for (int rt0 = 0; rt0 < RT; rt0 += 32) {
+				const bool near = rt0 + lane < RT && tmax[(size_t)(rt0 + lane) * Nc + dl] >= low;
+				for (unsigned tiles = __ballot_sync(FULL, near); tiles; tiles &= tiles - 1) {
+					const int rt = rt0 + __ffs(tiles) - 1;
+					const double *row = pval + ((size_t)rt * Nc + dl) * TILE + lane * LW;
+					double v[LW];
+#pragma unroll
+					for (int k = 0; k < LW; ++k)
+						v[k] = row[k];
+					f(rt, v);
+				}
+			}
+		};
+		int n = 0;
+		bool any = false;   // several: summed again (one alone stays as it is)
+		near_tiles([&](int rt, const double (&v)[LW]) {
+#pragma unroll
+			for (int k = 0; k < LW; ++k) {
+				const int r = rt * TILE + lane * LW + k;
+				const unsigned got = __ballot_sync(FULL, r < R && v[k] >= low);
+				if (got >> lane & 1u)
+					list[n + __popc(got & ((1u << lane) - 1u))] = r;
+				n += __popc(got);
+				if (n >= 32) {
+					again(32);
+					any = true;
+					n -= 32;
+					if (lane < n)
+						list[lane] = list[32 + lane];
+					__syncwarp();
+				}
+			}
+		});
+		if (!any && n <= 1)
+			continue;
+		again(n);
+		near_tiles([&](int rt, const double (&v)[LW]) {
+			double tm = MAX_EXP_START;
+			int ta = -1;
+#pragma unroll
+			for (int k = 0; k < LW; ++k) {
+				const int r = rt * TILE + lane * LW + k;
+				if (r < R && v[k] > tm) {
+					tm = v[k];
+					ta = r;
+				}
+			}
+#pragma unroll
+			for (int o = 16; o > 0; o >>= 1) {
+				const double om = __shfl_xor_sync(FULL, tm, o);
+				const int oa = __shfl_xor_sync(FULL, ta, o);
+				if (om > tm || (om == tm && oa >= 0 && (ta < 0 || oa < ta))) {
+					tm = om;
+					ta = oa;
+				}
+			}
+			if (lane == 0) {
+				tmax[(size_t)rt * Nc + dl] = tm;
+				targ[(size_t)rt * Nc + dl] = ta;
+			}
+		});
+	}
+}
+
 // ---------------------------------------------------------------------------
 // (c) per-frame maximum, pruning, normalisation and frame reductions
 // ---------------------------------------------------------------------------

@@ -69,6 +69,35 @@ def test_products_match_oracle_and_gathers(oracle_built, frames, div, side, phot
     plain.close()
 
 
+@pytest.mark.parametrize("copies,turn,scaling", [
+    (2, 1e-9, 1),     # pairs of orientations that only rounding tells apart
+    (3, 3e-8, 0),     # the same past it, without scale factors
+    (40, 1e-9, 1),    # more near ones than a warp sums at once
+    (40, 0., 1),      # exact ties: the lowest index
+])
+def test_near_ties_fall_as_with_the_gathers(copies, turn, scaling):
+    """Every orientation repeated a tiny turn further on: the most likely one of a
+    frame and its log-likelihood are the gathers', bit for bit."""
+    prob = _problem(300, 1, 24, 200.)
+    n = prob.quats.shape[0]
+    q = np.repeat(prob.quats, copies, 0)
+    q[:, 1:4] += turn * (np.arange(n * copies) % copies)[:, None]
+    q[:, :4] /= np.linalg.norm(q[:, :4], axis=1)[:, None]
+    q[:, 4] /= copies
+    prob = EMCProblem(prob.qvals, prob.corr, prob.mask, prob.ones, prob.multi, prob.place_ones, prob.place_multi,
+                      prob.count_multi, q, prob.model1, need_scaling=scaling, update_scale=scaling, beta=0.1)
+    got = []
+    for skip in (0, 1):
+        gpu = GPUEngine(prob, tile_skip=skip)
+        got.append(gpu.run_iteration(1))
+        got[-1]["launches"] = gpu.ctx.workload()["launches"]
+        gpu.close()
+    a, b = got
+    assert a["launches"] > b["launches"]   # the products ran
+    np.testing.assert_array_equal(a["rmax"], b["rmax"])
+    np.testing.assert_array_equal(a["max_exp"], b["max_exp"])
+
+
 def test_products_lose_no_precision_at_small_logarithms(oracle_built):
     """A start model of about one photon per pixel, where log W is small and FP32
     holds it finely: the digits must too. The gathers' compensated sums round once
