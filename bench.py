@@ -139,24 +139,6 @@ def measured_tensor_peak():
         return 1400., "of fallback (sustained)"
 
 
-# The library's rule for the pixels that go through integer tensor-core products
-# instead of row gathers (kHotOccupancy in csrc/emc_api.cu): mask-0 pixels with
-# photons on at least this share of the frames, in multiples of 128.
-HOT_OCCUPANCY = 0.012
-
-
-def hot_split(ctx, mask):
-    """(hot pixels, their photon words, all mask-0 photon words) of the
-    context's frames by that rule."""
-    _, _, po, pm, cm = ctx.get_frames()
-    words = np.bincount(po, minlength=mask.size) + np.bincount(pm, minlength=mask.size)
-    big = np.zeros(mask.size, bool)
-    big[pm[cm > 255]] = True
-    n = np.sort(words[(mask == 0) & ~big & (words > 0)])[::-1]
-    hot = min((int((n >= HOT_OCCUPANCY * ctx.num_data).sum()) + 64) // 128 * 128, n.size)
-    return hot, int(n[:hot].sum()), int(words[mask == 0].sum())
-
-
 def measured_int8_peak():
     """Dense INT8 rate in TOP/s: twice the measured BF16 burst rate (the
     tensor pipe's ratio), else of the fallback figure."""
@@ -497,11 +479,12 @@ def run_ours(args, rank, world, local_rank):
         roof = {"kernel": dom + " (dense, tensor cores)", "bound": "tensor", "achieved": achieved, "peak": tpeak,
                 "unit": "TFLOP/s", "frac": achieved / tpeak, "peak_source": tsrc, "traffic": None,
                 "phase_ms_per_step": {k: v[0] / args.steps for k, v in phases.items()}}
-    elif dom in gather_peak and hot_split(ctx, inp["mask"])[0] >= 128 and wl["chunk_frames"] >= 256:
+    elif dom in gather_peak and ctx.products()[dom]:
         # the hot pixels' integer products (2 operations x 4 digit bytes per
         # orientation, frame and pixel) and the other photons' row gathers, one
         # after the other: the floor is the sum of both at their peaks
-        hot, hot_words, words = hot_split(ctx, inp["mask"])
+        prod = ctx.products()
+        hot, hot_words, words = prod["pixels"], prod["words"], E
         ipeak, isrc = measured_int8_peak()
         R_pad = -(-R // 128) * 128
         t_prod = 8. * R_pad * N * (-(-hot // 128) * 128) / (ipeak * 1e12)

@@ -121,6 +121,7 @@ _SIGS = {
     "dfg_phase_name": (C.c_char_p, [C.c_int]),
     "dfg_reset_phase_times": (C.c_int, [_V]),
     "dfg_get_workload": (C.c_int, [_V, C.POINTER(C.c_longlong)]),
+    "dfg_get_products": (C.c_int, [_V, C.POINTER(C.c_longlong)]),
     "dfg_simulate_frames": (C.c_int, [_V, C.c_long, _D, C.c_int, _D, _D, C.c_ulonglong,
                                       C.POINTER(C.c_longlong)]),
     "dfg_get_frames": (C.c_int, [_V, _I, _I, _I, _I, _I]),
@@ -610,6 +611,13 @@ class Context:
         keys = ("num_orient", "num_data", "estep_entries", "mstep_entries", "chunks", "chunk_frames",
                 "launches", "k_pad", "dense_estep", "live_pairs", "block_tiles")
         return dict(zip(keys, list(out)))
+
+    def products(self):
+        """The integer products of the last iteration: their pixels, the photon words on them, and whether the
+        E-step and the M-step took them."""
+        out = (C.c_longlong * 4)()
+        self.call("dfg_get_products", out)
+        return dict(zip(("pixels", "words", "estep", "mstep"), list(out)))
 
 
 class Batch:

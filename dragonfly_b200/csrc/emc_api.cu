@@ -1332,9 +1332,9 @@ static int hot_choose(dfg_ctx *ctx) {
 	if (n < HK)
 		return DFG_OK;
 	cand.resize(n);
-	ctx->hot_words = 0.;
+	ctx->hot_words = 0;
 	for (int p : cand)
-		ctx->hot_words += (double)ctx->h_pix_entries[p] / N;
+		ctx->hot_words += ctx->h_pix_entries[p];
 	const int pitch = (n + HK - 1) / HK * HK;
 	std::vector<uint8_t> is_hot((size_t)P, 0);
 	for (int p : cand)
@@ -1487,7 +1487,7 @@ static int hot_prepare(dfg_ctx *ctx) {
 	if (ctx->hot_n == 0)
 		return DFG_OK;
 	const long long rows = (long long)ctx->RT * 2 * 4 * HO;
-	ctx->hot_estep = !ctx->refine || refine_share(ctx) * ctx->hot_words >= kHotColumnWords * ctx->hot_n;
+	ctx->hot_estep = !ctx->refine || refine_share(ctx) * (double)ctx->hot_words >= kHotColumnWords * ctx->hot_n * (double)ctx->N;
 	if (ctx->hot_estep) {
 		const cudaError_t e = ctx->wdig.ensure((size_t)rows * ctx->hot_pitch);
 		if (e == cudaErrorMemoryAllocation) {
@@ -4171,6 +4171,17 @@ extern "C" int dfg_event_elapsed(dfg_ctx *ctx, int a, int b, double *ms) {
 	float f = 0.f;
 	CK(cudaEventElapsedTime(&f, ctx->user_ev[a], ctx->user_ev[b]));
 	*ms = f;
+	return DFG_OK;
+}
+
+extern "C" int dfg_get_products(dfg_ctx *ctx, long long *out) {
+	if (!ctx || !out)
+		return DFG_ERR_ARG;
+	const bool on = ctx->hot_active;
+	out[0] = on ? ctx->hot_n : 0;
+	out[1] = on ? ctx->hot_words : 0;
+	out[2] = on && ctx->hot_estep && !ctx->dense_active;
+	out[3] = on && !ctx->m_dense_active;
 	return DFG_OK;
 }
 

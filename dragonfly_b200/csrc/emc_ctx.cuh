@@ -240,7 +240,7 @@ struct dfg_ctx {
 	// each orientation's largest probability in the chunk. layout counts the
 	// chunk layouts built, hot_layout is the one the hot set was made for
 	int hot_n = 0, hot_pitch = 0, layout = 0, hot_layout = -1;
-	double hot_words = 0.;     // photon words per frame on hot pixels
+	long long hot_words = 0;   // photon words on hot pixels
 	bool hot_active = false;   // this iteration takes the products (M-step)
 	bool hot_estep = false;    // and the E-step's
 	double refine_live = -1.;  // share of (tile, frame) pairs a refinement evaluates; -1 = not counted

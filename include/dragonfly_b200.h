@@ -485,6 +485,12 @@ DFG_API int dfg_reset_phase_times(dfg_ctx *ctx);
  * orientation tiles per block of the pair lists. out must hold 11 values. */
 DFG_API int dfg_get_workload(dfg_ctx *ctx, long long *out);
 
+/* The integer products of the last iteration: out[0] = pixels they took (0:
+ * every photon was gathered), out[1] = photon words of the E-step lists on
+ * these pixels, out[2] = 1 when the E-step took them, out[3] = 1 when the
+ * M-step did. out must hold 4 values. No counterpart in the reference. */
+DFG_API int dfg_get_products(dfg_ctx *ctx, long long *out);
+
 /* Ceiling of the gather kernels' access pattern on the context's device. No
  * counterpart in the reference (a measurement helper): reads uniformly random
  * 512-byte rows (one 16-byte load per lane, eight rows in flight per lane, all

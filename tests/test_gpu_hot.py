@@ -90,10 +90,9 @@ def test_near_ties_fall_as_with_the_gathers(copies, turn, scaling):
     for skip in (0, 1):
         gpu = GPUEngine(prob, tile_skip=skip)
         got.append(gpu.run_iteration(1))
-        got[-1]["launches"] = gpu.ctx.workload()["launches"]
+        assert gpu.ctx.products()["estep"] == 1 - skip
         gpu.close()
     a, b = got
-    assert a["launches"] > b["launches"]   # the products ran
     np.testing.assert_array_equal(a["rmax"], b["rmax"])
     np.testing.assert_array_equal(a["max_exp"], b["max_exp"])
 
@@ -112,6 +111,8 @@ def test_products_lose_no_precision_at_small_logarithms(oracle_built):
     for skip in (0, 1):
         gpu = GPUEngine(prob, tile_skip=skip)
         off.append(np.linalg.norm(gpu.run_iteration(1)["model1"] - want))
+        took = gpu.ctx.products()
+        assert took["estep"] == took["mstep"] == 1 - skip and (took["pixels"] >= 128) == (skip == 0)
         gpu.close()
     assert off[0] <= 1.5 * off[1]
 
@@ -135,6 +136,7 @@ def test_tomograms_are_the_sums_over_the_kept_pairs(cells_per_frame):
             g.ctx.set_refinement(7, cells, lists)
     lister.ctx.maximize(par)
     gpu.ctx.maximize(par)
+    assert gpu.ctx.products()["estep"] and gpu.ctx.products()["mstep"]
     off, place, p = lister.ctx.sparse_prob()
     if cells_per_frame:
         own = np.zeros((n, 7), bool)
@@ -152,6 +154,29 @@ def test_tomograms_are_the_sums_over_the_kept_pairs(cells_per_frame):
     np.testing.assert_allclose(gpu.ctx.tomograms(0, R), want, rtol=4 * 2. ** -24, atol=1e-8 * want.max())
     lister.close()
     gpu.close()
+
+
+@pytest.mark.parametrize("cells_per_frame,products", [(30, 1), (1, 0)])
+def test_refined_estep_on_both_sides_of_its_rule(cells_per_frame, products):
+    """A refined search whose frames evaluate many cells takes the E-step's products, one
+    with few gathers; both find what the pair lists find, which always gather."""
+    prob = _problem(300, 4, 24, 12.)
+    R, n = prob.quats.shape[0], prob.num_data
+    cells = (np.arange(R) * 108 // R).astype(np.int32)
+    rng = np.random.default_rng(4)
+    lists = np.array([rng.permutation(108)[:cells_per_frame] for _ in range(n)], np.int32)
+    got = []
+    for pairs in (0, 1):
+        gpu = GPUEngine(prob, pair_lists=pairs)
+        gpu.ctx.set_refinement(108, cells, lists)
+        gpu.ctx.maximize(gpu.ctx.params(1, 1, 0, 0, 1., 100, 1.))
+        took = gpu.ctx.products()
+        assert (took["estep"], took["mstep"]) == ((0, 0) if pairs else (products, 1))
+        got.append(gpu.ctx.frame_results())
+        gpu.close()
+    a, b = got
+    np.testing.assert_array_equal(a["rmax"], b["rmax"])
+    assert np.all(np.abs(a["likelihood"] - b["likelihood"]) <= 2. ** -24 * 40. * _photons(prob))
 
 
 def test_product_wait_gives_up_and_the_context_recovers(oracle_built):
