@@ -1306,6 +1306,23 @@ static int encode_pval_map(dfg_ctx *ctx, CUtensorMap *map, const void *base, int
 static bool tile_skipping(const dfg_ctx *ctx);
 static int prepare_qmap(dfg_ctx *ctx);
 
+// Memory that an iteration can do without: whether the buffer holds n elements. A
+// refusal for want of memory leaves no error behind (*e: any other error).
+// refuse_memory (test hook) refuses the bits' buffers.
+constexpr int kSpareDigits = 1, kSpareCounts = 2;
+
+template <typename T>
+static bool spare_memory(dfg_ctx *ctx, int what, DevBuf<T> &b, size_t n, cudaError_t *e) {
+	if (ctx->refuse_memory & what)
+		b.release();
+	*e = ctx->refuse_memory & what ? cudaErrorMemoryAllocation : b.ensure(n);
+	if (*e != cudaErrorMemoryAllocation)
+		return *e == cudaSuccess;
+	cudaGetLastError();
+	*e = cudaSuccess;
+	return false;
+}
+
 static int hot_choose(dfg_ctx *ctx) {
 	const int N = ctx->N, P = ctx->P;
 	cudaStream_t st = ctx->stream;
@@ -1342,21 +1359,15 @@ static int hot_choose(dfg_ctx *ctx) {
 	CK(upload(ctx->hot_pix, cand.data(), cand.size(), st));
 	CK(upload(ctx->is_hot, is_hot.data(), is_hot.size(), st));
 	// a failure to allocate leaves the gathers in charge
-	auto fits = [](cudaError_t e) {
-		if (e == cudaErrorMemoryAllocation)
-			cudaGetLastError();
-		return e;
-	};
+	cudaError_t e = cudaSuccess;
 	bool room = true;
 	for (Chunk &ch : ctx->chunks) {
 		ch.k_pitch = (ch.nc + HK - 1) / HK * HK;
 		const size_t by_frame_n = (size_t)ch.nc * pitch, counts_n = by_frame_n + (size_t)n * ch.k_pitch;
-		const cudaError_t e = fits(ch.counts.ensure(counts_n));
-		if (e == cudaErrorMemoryAllocation) {
-			room = false;
-			break;
-		}
+		room = spare_memory(ctx, kSpareCounts, ch.counts, counts_n, &e);
 		CK(e);
+		if (!room)
+			break;
 		CK(cudaMemsetAsync(ch.counts.p, 0, counts_n, st));
 		uint8_t *by_frame = ch.counts.p, *by_pixel = ch.counts.p + by_frame_n;
 		hot_counts_kernel<<<blocks_for((long long)n * 32, 256), 256, 0, st>>>(
@@ -1399,10 +1410,9 @@ static int hot_choose(dfg_ctx *ctx) {
 		CK(cudaMemcpyAsync(h.data(), cnt.p, (size_t)N * sizeof(int2), cudaMemcpyDeviceToHost, st));
 		CK(cudaStreamSynchronize(st));
 		lay_out(N);
-		const cudaError_t e = fits(ctx->phc.ensure((size_t)off[N]));
-		room = e != cudaErrorMemoryAllocation;
+		room = spare_memory(ctx, kSpareCounts, ctx->phc, (size_t)off[N], &e);
+		CK(e);
 		if (room) {
-			CK(e);
 			CK(upload(ctx->phc_off, off.data(), off.size(), st));
 			CK(upload(ctx->phc_mid, mid.data(), mid.size(), st));
 			cold_write_kernel<false><<<blocks_for((long long)N * 32, 256), 256, 0, st>>>(
@@ -1422,10 +1432,9 @@ static int hot_choose(dfg_ctx *ctx) {
 		CK(cudaMemcpyAsync(h.data(), cnt.p, (size_t)P * sizeof(int2), cudaMemcpyDeviceToHost, st));
 		CK(cudaStreamSynchronize(st));
 		lay_out(P);
-		const cudaError_t e = fits(ch.csc.ensure((size_t)off[P]));
-		room = e != cudaErrorMemoryAllocation;
+		room = spare_memory(ctx, kSpareCounts, ch.csc, (size_t)off[P], &e);
+		CK(e);
 		if (room) {
-			CK(e);
 			CK(upload(ch.csc_off, off.data(), off.size(), st));
 			CK(upload(ch.csc_mid, mid.data(), mid.size(), st));
 			cold_write_kernel<true><<<blocks_for((long long)P * 32, 256), 256, 0, st>>>(
@@ -1464,8 +1473,10 @@ static double refine_share(dfg_ctx *ctx) {
 		DevBuf<unsigned long long> n;
 		unsigned long long h = 0;
 		if (prepare_qmap(ctx) != DFG_OK || n.ensure(1) != cudaSuccess ||
-		    cudaMemsetAsync(n.p, 0, sizeof(h), ctx->stream) != cudaSuccess)
+		    cudaMemsetAsync(n.p, 0, sizeof(h), ctx->stream) != cudaSuccess) {
+			cudaGetLastError();
 			return 0.;
+		}
 		refine_count_kernel<<<dim3((unsigned)std::min<long long>(blocks_for(ctx->N, 8), 64), ctx->RT), 256, 0, ctx->stream>>>(
 		    RefineMask{ctx->qmap.p, ctx->rel_bits.p, ctx->rwords}, ctx->N, ctx->RT, n.p);
 		ctx->launches++;
@@ -1487,18 +1498,16 @@ static int hot_prepare(dfg_ctx *ctx) {
 	if (ctx->hot_n == 0)
 		return DFG_OK;
 	const long long rows = (long long)ctx->RT * 2 * 4 * HO;
+	cudaError_t e = cudaSuccess;
 	ctx->hot_estep = !ctx->refine || refine_share(ctx) * (double)ctx->hot_words >= kHotColumnWords * ctx->hot_n * (double)ctx->N;
 	if (ctx->hot_estep) {
-		const cudaError_t e = ctx->wdig.ensure((size_t)rows * ctx->hot_pitch);
-		if (e == cudaErrorMemoryAllocation) {
-			cudaGetLastError();
-			ctx->hot_n = 0;
-			return DFG_OK;
-		}
+		// no memory for them: the E-step gathers, the M-step's products need none
+		ctx->hot_estep = spare_memory(ctx, kSpareDigits, ctx->wdig, (size_t)rows * ctx->hot_pitch, &e);
 		CK(e);
+	}
+	if (ctx->hot_estep)
 		if (int rc = encode_byte_map(ctx, &ctx->map_wdig, ctx->wdig.p, rows, ctx->hot_pitch))
 			return rc;
-	}
 	CK(ctx->hot_special.ensure((size_t)ctx->RT));
 	CK(ctx->rowmax.ensure((size_t)ctx->R_pad));
 	CK(ctx->rowmax_part.ensure((size_t)psum_splits(ctx) * ctx->R_pad));
@@ -4099,6 +4108,12 @@ extern "C" int dfg_set_option(dfg_ctx *ctx, const char *key, double value) {
 	if (!strcmp(key, "dense_wait_cycles")) {
 		NEED(value >= 1e4 && value <= 1e11, DFG_ERR_ARG, "dense_wait_cycles must be in [1e4, 1e11]");
 		ctx->dense_wait_cycles = (long long)value;
+		return DFG_OK;
+	}
+	if (!strcmp(key, "refuse_memory")) {
+		NEED(value >= 0 && value <= 3, DFG_ERR_ARG, "refuse_memory must be 0 to 3");
+		ctx->refuse_memory = (int)value;
+		ctx->hot_layout = -1;
 		return DFG_OK;
 	}
 	if (!strcmp(key, "dense_withhold_stage")) {

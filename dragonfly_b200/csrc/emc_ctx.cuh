@@ -254,6 +254,7 @@ struct dfg_ctx {
 	DevBuf<float> rowmax, rowmax_part;
 	CUtensorMap map_wdig;
 	int max_fcount = 0;        // most photons of a frame
+	int refuse_memory = 0;     // test hook: the products' buffers that get no memory (spare_memory)
 	// failure-detection test hooks of the dense kernels: the clock cycles
 	// after which a pipeline wait gives up, and a stage whose copies are never
 	// issued (-1: none)

@@ -462,7 +462,10 @@ DFG_API int dfg_save_emc(dfg_ctx *ctx, const char *path);
  * "dense_wait_cycles" (clock cycles after which a pipeline wait gives up,
  * default 2e9, about a second) and "dense_withhold_stage" (a stage index
  * whose copies are never issued, so the waits on it run out and the call
- * returns DFG_ERR_CUDA; -1, the default, issues every stage). */
+ * returns DFG_ERR_CUDA; -1, the default, issues every stage). Test hook
+ * "refuse_memory" (bits): the integer products' buffers that get no memory, 1
+ * the log-slices' digits (the E-step gathers), 2 the count matrices and lists
+ * (both steps gather); 0, the default, none. */
 DFG_API int dfg_set_option(dfg_ctx *ctx, const char *key, double value);
 /* Phase times in ms summed since the last reset, and launch counts:
  * names[i] = "slice", "estep", "norm", "psum", "mstep", "merge", "update".

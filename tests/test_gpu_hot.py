@@ -179,6 +179,34 @@ def test_refined_estep_on_both_sides_of_its_rule(cells_per_frame, products):
     assert np.all(np.abs(a["likelihood"] - b["likelihood"]) <= 2. ** -24 * 40. * _photons(prob))
 
 
+@pytest.mark.parametrize("refused", [1, 2, 3])
+def test_without_memory_for_the_products(refused):
+    """No memory for the log-slices' digits: the E-step gathers and the M-step keeps its
+    products; none for the counts: both gather. The same later, when more orientations
+    need larger buffers than the first call's."""
+    small, large = _problem(300, 1, 24, 200.), _problem(300, 2, 24, 200.)
+    plain, gpu = GPUEngine(small, tile_skip=1), GPUEngine(small)
+    par = plain.ctx.params(1, 1, 0, 0, 1., 100, 1.)
+    c = gpu.ctx
+    for first in (True, False):
+        if not first:
+            for g in (plain, gpu):
+                g.ctx.set_quaternions(large.quats)
+        for mem in (0, refused) if first else (refused, 0):
+            c.set_option("refuse_memory", mem)
+            for g in (plain, gpu):
+                g.ctx.maximize(par)
+            took = c.products()
+            assert (took["estep"], took["mstep"]) == (int(mem == 0), int(mem < 2))
+            a, b = c.frame_results(), plain.ctx.frame_results()
+            np.testing.assert_array_equal(a["rmax"], b["rmax"])
+            assert np.all(np.abs(a["likelihood"] - b["likelihood"]) <= 2. ** -24 * 40. * _photons(small))
+            want = plain.ctx.tomograms(0, 60)
+            np.testing.assert_allclose(c.tomograms(0, 60), want, rtol=8 * 2. ** -24, atol=1e-8 * want.max())
+    plain.close()
+    gpu.close()
+
+
 def test_product_wait_gives_up_and_the_context_recovers(oracle_built):
     """A stage whose copies are withheld (test hook): its waits run out, the
     kernels return, the call reports the error, and the next call succeeds."""
