@@ -1525,6 +1525,10 @@ static int hot_prepare(dfg_ctx *ctx) {
 	return DFG_OK;
 }
 
+// Blocks of hot_digits_kernel. (128 x 512 bytes of log-slices or probabilities each:
+// 2^31 of them exceed any memory.)
+static unsigned digit_blocks(int tiles, int k_pitch) { return (unsigned)tiles * 2u * (unsigned)(k_pitch / HK); }
+
 static unsigned hot_grid(const dfg_ctx *ctx, long long tiles) {
 	return (unsigned)std::min<long long>(tiles, ctx->num_sms);
 }
@@ -1533,7 +1537,7 @@ static unsigned hot_grid(const dfg_ctx *ctx, long long tiles) {
 static int launch_hot_digits(dfg_ctx *ctx) {
 	cudaStream_t st = ctx->stream;
 	CK(cudaMemsetAsync(ctx->hot_special.p, 0, (size_t)ctx->RT * sizeof(int), st));
-	hot_digits_kernel<false><<<dim3(ctx->hot_pitch / HK, ctx->RT * 2), 256, 0, st>>>(
+	hot_digits_kernel<false><<<digit_blocks(ctx->RT, ctx->hot_pitch), 256, 0, st>>>(
 	    ctx->logW.p, (size_t)(ctx->P + 1) * TILE, ctx->hot_pix.p, ctx->hot_n, ctx->hot_pitch, nullptr, ctx->wdig.p,
 	    ctx->hot_special.p, nullptr);
 	CKL("hot_digits_kernel");
@@ -1551,7 +1555,7 @@ static int launch_hot_estep(dfg_ctx *ctx, const Chunk &ch) {
 static int launch_hot_mstep(dfg_ctx *ctx, const Chunk &ch) {
 	cudaStream_t st = ctx->stream;
 	int8_t *dig = reinterpret_cast<int8_t *>(ctx->pval.p);
-	hot_digits_kernel<true><<<dim3(ch.k_pitch / HK, ctx->RT * 2), 256, 0, st>>>(
+	hot_digits_kernel<true><<<digit_blocks(ctx->RT, ch.k_pitch), 256, 0, st>>>(
 	    ctx->Pst.p, (size_t)(ch.nc + 1) * TILE, nullptr, ch.nc, ch.k_pitch, ctx->rowmax.p, dig, nullptr,
 	    tile_skipping(ctx) ? ctx->tlive.p : nullptr);
 	CKL("hot_digits_kernel");

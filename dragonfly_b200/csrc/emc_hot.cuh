@@ -359,7 +359,9 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 // the rows that hold probabilities (tile skipping), the others count as zero.
 // Block = 128 reduction rows x 64 orientations,
 // transposed through shared memory; the rotation by 4 (k / 16) keeps the
-// column reads free of bank conflicts. Memory-bound: 4 bytes read, 4 written.
+// column reads free of bank conflicts. Memory-bound: 4 bytes read, 4 written. The
+// grid is flat, blocks of one 64-orientation half in turn (digit_blocks): from
+// 32768 tiles on there are more halves than a grid's second extent takes.
 template <bool MSTEP>
 __global__ void __launch_bounds__(256) hot_digits_kernel(const float *__restrict__ src, size_t tile_stride,
                                                          const int *__restrict__ pix, int nk, int k_pitch,
@@ -368,7 +370,7 @@ __global__ void __launch_bounds__(256) hot_digits_kernel(const float *__restrict
                                                          const uint8_t *__restrict__ live) {
 	__shared__ int s[HK][HO + 1];
 	__shared__ double s_scale[HO];
-	const int kb = blockIdx.x, ot = blockIdx.y, t = threadIdx.x;
+	const int kblocks = k_pitch / HK, ot = blockIdx.x / kblocks, kb = blockIdx.x - ot * kblocks, t = threadIdx.x;
 	const int rt = ot >> 1, j0 = (ot & 1) * HO;
 	if (MSTEP && t < HO) {
 		const float m = rmax[(size_t)rt * TILE + j0 + t];

@@ -9,7 +9,7 @@ value to 2^-24 of it, the products add exactly.
 import numpy as np
 import pytest
 
-from common import GPUEngine, compare_iteration
+from common import MODEL_REL_L2, GPUEngine, compare_iteration
 from oracle.oracle import EMCProblem, OracleEngine
 from dragonfly_b200 import synth
 
@@ -177,6 +177,29 @@ def test_refined_estep_on_both_sides_of_its_rule(cells_per_frame, products):
     a, b = got
     np.testing.assert_array_equal(a["rmax"], b["rmax"])
     assert np.all(np.abs(a["likelihood"] - b["likelihood"]) <= 2. ** -24 * 40. * _photons(prob))
+
+
+def test_more_tiles_than_a_grid_extent_of_their_halves():
+    """32768 orientation tiles (4.2 million orientations): twice as many 64-orientation
+    halves as a grid's second extent takes. The products find what the gathers find."""
+    prob = _problem(256, 1, 24, 200.)
+    rng = np.random.default_rng(9)
+    q = rng.normal(size=(32768 * 128, 5))
+    q[:, :4] /= np.linalg.norm(q[:, :4], axis=1)[:, None]
+    q[:, 4] = 1. / q.shape[0]
+    got = []
+    for skip in (0, 1):
+        gpu = GPUEngine(prob, tile_skip=skip, pair_budget_mb=30000)
+        gpu.ctx.set_quaternions(q)
+        gpu.ctx.maximize(gpu.ctx.params(1, 1, 0, 0, 1., 100, 1.))
+        assert gpu.ctx.products()["estep"] == gpu.ctx.products()["mstep"] == 1 - skip
+        gpu.ctx.update_model(0.)
+        got.append((gpu.ctx.frame_results(), gpu.ctx.model()[0]))
+        gpu.close()
+    (a, ma), (b, mb) = got
+    np.testing.assert_array_equal(a["rmax"], b["rmax"])
+    assert np.all(np.abs(a["likelihood"] - b["likelihood"]) <= 2. ** -24 * 40. * _photons(prob))
+    assert np.linalg.norm(ma - mb) <= MODEL_REL_L2 * np.linalg.norm(mb)
 
 
 @pytest.mark.parametrize("refused", [1, 2, 3])
