@@ -1547,7 +1547,8 @@ static int launch_hot_digits(dfg_ctx *ctx) {
 static int launch_hot_estep(dfg_ctx *ctx, const Chunk &ch) {
 	const int OT = ctx->RT * 2, FT = (ch.nc + HM - 1) / HM;
 	hot_product_kernel<false><<<hot_grid(ctx, (long long)OT * FT), HTHREADS, HSMEM_BYTES, ctx->stream>>>(
-	    ch.map_frame, ctx->map_wdig, ch.map_pval, ctx->hot_pitch / HK, OT, FT, ch.nc, HotOut{}, ctx->derr.p, ctx->dense_wait_cycles, ctx->dense_withhold);
+	    ch.map_frame, ctx->map_wdig, ch.map_pval, ctx->hot_pitch / HK, OT, FT, ch.nc, HotOut{}, ctx->hot_special.p,
+	    ctx->derr.p, ctx->dense_wait_cycles, ctx->dense_withhold);
 	CKL("hot_product_kernel");
 	return DFG_OK;
 }
@@ -1562,7 +1563,7 @@ static int launch_hot_mstep(dfg_ctx *ctx, const Chunk &ch) {
 	const int OT = ctx->RT * 2, FT = (ctx->hot_n + HM - 1) / HM;
 	hot_product_kernel<true><<<hot_grid(ctx, (long long)OT * FT), HTHREADS, HSMEM_BYTES, st>>>(
 	    ch.map_pixel, ch.map_pdig, ch.map_pval, ch.k_pitch / HK, OT, FT, ctx->hot_n,
-	    HotOut{ctx->T.p, ctx->hot_pix.p, ctx->rowmax.p, ctx->P, ch.d0 == 0 ? 1 : 0}, ctx->derr.p,
+	    HotOut{ctx->T.p, ctx->hot_pix.p, ctx->rowmax.p, ctx->P, ch.d0 == 0 ? 1 : 0}, nullptr, ctx->derr.p,
 	    ctx->dense_wait_cycles, ctx->dense_withhold);
 	CKL("hot_product_kernel");
 	return DFG_OK;

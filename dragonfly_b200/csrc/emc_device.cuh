@@ -437,10 +437,11 @@ __global__ void __launch_bounds__(256, MINB) estep_cold_kernel(
 			for (int h = 0; h < NPAIR; ++h)
 				kahan_add_count2(s[h], c[h], e[q] >> IDX_BITS, v[q][h]);
 	}
-	double hot[LW], ur[LW], lw[LW], acc[LW];
-	asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
-	             : "=d"(hot[0]), "=d"(hot[1]), "=d"(hot[2]), "=d"(hot[3])
-	             : "l"(row));
+	double hot[LW] = {0., 0., 0., 0.}, ur[LW], lw[LW], acc[LW];
+	if (!special)
+		asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+		             : "=d"(hot[0]), "=d"(hot[1]), "=d"(hot[2]), "=d"(hot[3])
+		             : "l"(row));
 	const int r0 = rt * TILE + lane * LW;
 	ld_row32(u + r0, ur);
 	ld_row32(logw + r0, lw);

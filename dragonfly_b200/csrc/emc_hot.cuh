@@ -136,7 +136,8 @@ struct HotOut {
 template <bool MSTEP>
 __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
     const __grid_constant__ CUtensorMap map_cnt, const __grid_constant__ CUtensorMap map_dig,
-    const __grid_constant__ CUtensorMap map_out, int num_kb, int OT, int FT, int nrows, HotOut out, int *__restrict__ err, long long wait_cycles, int withhold_kb) {
+    const __grid_constant__ CUtensorMap map_out, int num_kb, int OT, int FT, int nrows, HotOut out,
+    const int *__restrict__ special, int *__restrict__ err, long long wait_cycles, int withhold_kb) {
 	extern __shared__ uint8_t hsm_raw[];
 	uint8_t *sm = (uint8_t *)(((uintptr_t)hsm_raw + 1023) & ~(uintptr_t)1023);
 	uint8_t *outs = sm + HSTAGES * HSTAGE_BYTES;
@@ -179,6 +180,9 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 		ft = rem / rows;
 	};
 
+	// E-step tiles that gather all of their photons (hot_digits_kernel)
+	auto skipped = [&](int ot) { return !MSTEP && __ldg(special + (ot >> 1)) != 0; };
+
 	if (warp == 0) {
 		if (lane == 0) {
 			long long it = 0, issued = 0;  // stage counter over all tiles; stages whose copies were issued
@@ -186,6 +190,8 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 			for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
 				int ot, ft;
 				locate_tile(t, ot, ft);
+				if (skipped(ot))
+					continue;
 				for (int kb = 0; kb < num_kb; ++kb, ++it) {
 					const int s = (int)(it % HSTAGES);
 					const uint32_t ph = (uint32_t)(it / HSTAGES) & 1u;
@@ -217,7 +223,11 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 			long long it = 0;
 			uint32_t n = 0;  // tiles done by this CTA
 			bool ok = true;
-			for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++n) {
+			for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+				int ot, ft;
+				locate_tile(t, ot, ft);
+				if (skipped(ot))
+					continue;
 				// the epilogue has read the previous tile's sums
 				if (*abort_flag || !mbar_wait(tempty, (n & 1u) ^ 1u, wait_cycles)) {
 					*abort_flag = 1;
@@ -247,6 +257,7 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 				}
 				if (ok)
 					umma_commit(tfull);
+				++n;
 			}
 		}
 		__syncwarp();
@@ -255,11 +266,14 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 		const int m = (warp - 2) >> 2, q = warp & 3, i = m * 128 + q * 32 + lane;
 		const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(m * 4 * HO);
 		uint32_t n = 0;
-		for (long long t = blockIdx.x; t < tiles; t += gridDim.x, ++n) {
+		for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
 			int ot, ft;
 			locate_tile(t, ot, ft);
+			if (skipped(ot))
+				continue;
 			// the flag may change between the lanes' reads: decide for the warp
 			bool ok = mbar_wait(tfull, n & 1u, wait_cycles) && !*abort_flag;
+			++n;
 			ok = __all_sync(FULL, ok);
 			if (!ok) {
 				if (lane == 0) {
@@ -355,7 +369,8 @@ __global__ void __launch_bounds__(HTHREADS, 1) hot_product_kernel(
 // Balanced digits: x = sum_g d_g 256^g with -128 <= d_g <= 127. K past the last
 // pixel or frame is zero. A log-slice that the digits cannot hold (log 0, the
 // value outside the model, NaN) sets special[tile]: the E-step then gathers
-// that tile's photons all. live (true; may be null): [tile][Nc + 1] flags of
+// that tile's photons all, and its products are left out (an empty one of several
+// modes does that to every tile). live (true; may be null): [tile][Nc + 1] flags of
 // the rows that hold probabilities (tile skipping), the others count as zero.
 // Block = 128 reduction rows x 64 orientations,
 // transposed through shared memory; the rotation by 4 (k / 16) keeps the

@@ -179,6 +179,28 @@ def test_refined_estep_on_both_sides_of_its_rule(cells_per_frame, products):
     assert np.all(np.abs(a["likelihood"] - b["likelihood"]) <= 2. ** -24 * 40. * _photons(prob))
 
 
+def test_tiles_that_gather_all_take_no_products():
+    """One of two modes is empty: each tile has log 0, gathers all of its photons and its
+    products are left out. A withheld stage that only E-step products would reach (their
+    depth is the pixels, the M-step's the 256 frames) shows that none ran."""
+    prob = _problem(256, 2, 40, 600.)
+    model = np.concatenate([prob.model1, 0. * prob.model1])
+    prob = EMCProblem(prob.qvals, prob.corr, prob.mask, prob.ones, prob.multi, prob.place_ones, prob.place_multi,
+                      prob.count_multi, prob.quats, model, need_scaling=1, update_scale=1, beta=0.1)
+    assert prob.num_modes == 2
+    got = []
+    for skip in (0, 1):
+        gpu = GPUEngine(prob, tile_skip=skip, dense_wait_cycles=2e7, dense_withhold_stage=3)
+        got.append(gpu.run_iteration(1))
+        took = gpu.ctx.products()
+        assert took["estep"] == 1 - skip and (took["pixels"] > 3 * 128) == (skip == 0)
+        gpu.close()
+    a, b = got
+    np.testing.assert_array_equal(a["rmax"], b["rmax"])
+    np.testing.assert_array_equal(a["max_exp"], b["max_exp"])
+    assert np.all(a["rmax"] % 2 == 0)
+
+
 def test_more_tiles_than_a_grid_extent_of_their_halves():
     """32768 orientation tiles (4.2 million orientations): twice as many 64-orientation
     halves as a grid's second extent takes. The products find what the gathers find."""
