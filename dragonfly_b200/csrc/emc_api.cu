@@ -728,14 +728,14 @@ static int build_chunks(dfg_ctx *ctx) {
 		ch.d0 = (int)(k * nc);
 		ch.nc = (int)std::min<long long>(nc, N - ch.d0);
 		const uint32_t pad = (uint32_t)ch.nc;
-		// contiguous frame ranges, one per host thread (at least a million words
-		// each): every range counts its words per pixel and fills them in from its
+		// contiguous frame ranges, one per host thread (at least a million words each,
+		// and more words than counters): every range counts its words per pixel and fills them in from its
 		// own cursors, so the lists keep the frames' order
 		const int d1 = ch.d0 + ch.nc;
 		const long long given = ctx->h_ones_off[d1] - ctx->h_ones_off[ch.d0] + ctx->h_multi_off[d1] -
 		                        ctx->h_multi_off[ch.d0];
 		const int nth = (int)std::max<long long>(
-		    1, std::min<long long>({16, (long long)std::thread::hardware_concurrency(), given >> 20, ch.nc}));
+		    1, std::min<long long>({16, (long long)std::thread::hardware_concurrency(), given >> 20, given / P, ch.nc}));
 		auto each = [&](long long b, long long e, auto fn) {
 			for (int dl = (int)b; dl < (int)e; ++dl) {
 				const int d = ch.d0 + dl;
@@ -751,26 +751,33 @@ static int build_chunks(dfg_ctx *ctx) {
 				}
 			}
 		};
-		// per range and pixel: count-1 words, counted words, photons, the last frame
-		// that lists it, and whether the byte products cannot hold it (a count past
-		// a byte, or two entries of one frame); then the cursors of the two segments
-		std::vector<long long> c1((size_t)nth * P, 0), cm((size_t)nth * P, 0), photons((size_t)nth * P, 0);
-		std::vector<uint8_t> big((size_t)nth * P, 0);
-		std::vector<int> last((size_t)nth * P, -1);
+		// per range and pixel: count-1 words, the last frame that lists it and whether
+		// the byte products cannot hold it (a count past a byte, or two entries of one
+		// frame); counted words and their photons apart (most words are single
+		// photons). Then the words are the cursors of the two segments.
+		struct Ones {
+			long long words = 0;
+			int last = -1, big = 0;
+		};
+		struct Multi {
+			long long words = 0, photons = 0;
+		};
+		std::vector<Ones> ones((size_t)nth * P);
+		std::vector<Multi> multi((size_t)nth * P);
 		parallel_ranges(ch.nc, nth, [&](int th, long long b, long long e) {
-			long long *t1 = c1.data() + (size_t)th * P, *tm = cm.data() + (size_t)th * P;
-			long long *tp = photons.data() + (size_t)th * P;
-			uint8_t *tb = big.data() + (size_t)th * P;
-			int *tl = last.data() + (size_t)th * P;
+			Ones *o = ones.data() + (size_t)th * P;
+			Multi *m = multi.data() + (size_t)th * P;
 			each(b, e, [&](int p, int dl, long long c) {
-				if (c == 1)
-					t1[p]++;
-				else
-					tm[p] += (c + MAX_COUNT - 1) / MAX_COUNT;
-				tp[p] += c;
-				if (c > 255 || tl[p] == dl)
-					tb[p] = 1;
-				tl[p] = dl;
+				Ones &x = o[p];
+				if (c == 1) {
+					x.words++;
+				} else {
+					m[p].words += (c + MAX_COUNT - 1) / MAX_COUNT;
+					m[p].photons += c;
+					x.big |= c > 255;
+				}
+				x.big |= x.last == dl;
+				x.last = dl;
 			});
 		});
 		std::vector<long long> off(P + 1, 0), midv(P, 0), end1(P), endm(P);
@@ -778,10 +785,12 @@ static int build_chunks(dfg_ctx *ctx) {
 		for (int p = 0; p < P; ++p) {
 			long long n1 = 0, nm = 0, ph = 0;
 			for (int th = 0; th < nth; ++th) {
-				n1 += c1[(size_t)th * P + p];
-				nm += cm[(size_t)th * P + p];
-				ph += photons[(size_t)th * P + p];
-				ctx->h_pix_big[p] |= big[(size_t)th * P + p];
+				const Ones &o = ones[(size_t)th * P + p];
+				const Multi &m = multi[(size_t)th * P + p];
+				n1 += o.words;
+				nm += m.words;
+				ph += o.words + m.photons;
+				ctx->h_pix_big[p] |= o.big != 0;
 			}
 			midv[p] = off[p] + (n1 + 7) / 8 * 8;
 			off[p + 1] = midv[p] + (nm + 7) / 8 * 8;
@@ -789,11 +798,11 @@ static int build_chunks(dfg_ctx *ctx) {
 			endm[p] = midv[p] + nm;
 			long long f1 = off[p], fm = midv[p];
 			for (int th = 0; th < nth; ++th) {
-				const long long a = c1[(size_t)th * P + p], b = cm[(size_t)th * P + p];
-				c1[(size_t)th * P + p] = f1;
-				cm[(size_t)th * P + p] = fm;
-				f1 += a;
-				fm += b;
+				long long &o = ones[(size_t)th * P + p].words, &m = multi[(size_t)th * P + p].words;
+				f1 += o;
+				fm += m;
+				o = f1 - o;
+				m = fm - m;
 			}
 			real += n1 + nm;
 			ctx->h_pix_entries[p] += n1 + nm;
@@ -802,15 +811,16 @@ static int build_chunks(dfg_ctx *ctx) {
 		}
 		const std::unique_ptr<uint32_t[]> words(new uint32_t[(size_t)std::max<long long>(off[P], 1)]);
 		parallel_ranges(ch.nc, nth, [&](int th, long long b, long long e) {
-			long long *f1 = c1.data() + (size_t)th * P, *fm = cm.data() + (size_t)th * P;
+			Ones *o = ones.data() + (size_t)th * P;
+			Multi *m = multi.data() + (size_t)th * P;
 			each(b, e, [&](int p, int dl, long long c) {
 				if (c == 1) {
-					words[(size_t)f1[p]++] = (uint32_t)dl;
+					words[(size_t)o[p].words++] = (uint32_t)dl;
 					return;
 				}
 				while (c > 0) {
 					const uint32_t cc = (uint32_t)std::min<long long>(c, MAX_COUNT);
-					words[(size_t)fm[p]++] = (uint32_t)dl | (cc << IDX_BITS);
+					words[(size_t)m[p].words++] = (uint32_t)dl | (cc << IDX_BITS);
 					c -= cc;
 				}
 			});
@@ -819,7 +829,7 @@ static int build_chunks(dfg_ctx *ctx) {
 			std::fill(words.get() + end1[p], words.get() + midv[p], pad);
 			std::fill(words.get() + endm[p], words.get() + off[p + 1], pad);
 		}
-		std::vector<int> pix;
+		std::vector<int> &pix = ch.h_pix;
 		for (int p = 0; p < P; ++p)
 			if (off[p + 1] > off[p])
 				pix.push_back(p);
@@ -839,29 +849,44 @@ static int build_chunks(dfg_ctx *ctx) {
 	return DFG_OK;
 }
 
-// The corner quads take four times the model; past kQuadMaxBytes (or without
-// the memory) the slices gather voxels instead.
+// The corner quads take four times the model. Where the tomograms of all
+// orientations are resident the quads lie in them: they are read by the slices alone,
+// which come before the tomograms are cleared. Otherwise they have a buffer; past
+// kQuadMaxBytes (or without the memory) the slices gather voxels instead.
 constexpr size_t kQuadMaxBytes = (size_t)8 << 30;
 
-static int ensure_quads(dfg_ctx *ctx) {
+static int ensure_quads(dfg_ctx *ctx, bool resident) {
 	const size_t n = (size_t)ctx->M * ctx->V;
-	ctx->use_quads = n * sizeof(double4) <= kQuadMaxBytes;
-	if (!ctx->use_quads) {
+	const bool in_T = resident && ctx->T.n * sizeof(float) >= n * sizeof(double4);
+	if (in_T || n * sizeof(double4) > kQuadMaxBytes) {
 		ctx->quads.release();
+		ctx->quad_p = in_T ? reinterpret_cast<double4 *>(ctx->T.p) : nullptr;
 		return DFG_OK;
 	}
+	ctx->quad_p = nullptr;
 	const cudaError_t e = ctx->quads.ensure(n);
 	if (e == cudaErrorMemoryAllocation) {
 		cudaGetLastError();
-		ctx->use_quads = false;
 		return DFG_OK;
 	}
 	CK(e);
+	ctx->quad_p = ctx->quads.p;
 	return DFG_OK;
 }
 
-static SliceModel slice_model(const dfg_ctx *ctx) {
-	return SliceModel{ctx->use_quads ? ctx->quads.p : nullptr, ctx->model1.p};
+static SliceModel slice_model(const dfg_ctx *ctx) { return SliceModel{ctx->quad_p, ctx->model1.p}; }
+
+// The arrays over a chunk's (orientation, frame) and (tile, frame) pairs.
+static int ensure_pairs(dfg_ctx *ctx) {
+	const size_t R = (size_t)ctx->R_pad, RT = (size_t)ctx->RT, nc = (size_t)ctx->chunk_frames;
+	CK(ctx->pair_slab.ensure(SlabPart<double>{ctx->pval, R * nc}, SlabPart<float>{ctx->Pst, R * (nc + 1)},
+	                         SlabPart<double>{ctx->tmax, RT * nc}, SlabPart<int>{ctx->targ, RT * nc},
+	                         SlabPart<uint8_t>{ctx->tlive, RT * (nc + 1)}));
+	return DFG_OK;
+}
+
+static void release_pairs(dfg_ctx *ctx) {
+	ctx->pair_slab.release(ctx->pval, ctx->Pst, ctx->tmax, ctx->targ, ctx->tlive);
 }
 
 static int ensure_buffers(dfg_ctx *ctx) {
@@ -873,21 +898,21 @@ static int ensure_buffers(dfg_ctx *ctx) {
 	ctx->R = ctx->M * ctx->num_rot;
 	ctx->RT = (ctx->R + TILE - 1) / TILE;
 	ctx->R_pad = ctx->RT * TILE;
-	const size_t tiles_px = (size_t)ctx->RT * ctx->P * TILE;
+	// (tomograms: room for the log-slices' digits of 128-pixel blocks, see hot_prepare)
+	const size_t tiles_px = (size_t)ctx->RT * ((ctx->P + HK - 1) / HK * HK) * TILE;
 	const size_t logw_n = (size_t)ctx->RT * (ctx->P + 1) * TILE;
-	if (ctx->logW.n < logw_n || ctx->logW_P != ctx->P) {
-		CK(ctx->logW.ensure(logw_n));
+	if (ctx->logW.n < logw_n || ctx->T.n < tiles_px || ctx->logW_P != ctx->P) {
+		CK(ctx->tile_slab.ensure(SlabPart<float>{ctx->logW, logw_n}, SlabPart<float>{ctx->T, tiles_px}));
 		// the zero rows (pixel P of every tile) stay zero: the slice kernel
 		// writes rows 0..P-1 only
 		CK(cudaMemsetAsync(ctx->logW.p, 0, logw_n * sizeof(float), ctx->stream));
 		ctx->logW_P = ctx->P;
 	}
-	CK(ctx->T.ensure(tiles_px));
 	CK(ctx->u.ensure((size_t)ctx->R_pad));
 	CK(ctx->logw.ensure((size_t)ctx->R_pad));
 	CK(ctx->psum_r.ensure((size_t)ctx->R_pad));
 	CK(ctx->scalars.ensure(8));
-	if (int rc = ensure_quads(ctx))
+	if (int rc = ensure_quads(ctx, true))
 		return rc;
 	CK(ctx->red_part.ensure(std::max<size_t>(blocks_for((long long)ctx->M * ctx->V, 256), 1024)));
 	const size_t N = (size_t)ctx->N;
@@ -901,19 +926,12 @@ static int ensure_buffers(dfg_ctx *ctx) {
 	CK(ctx->quat_norm.ensure(N * ctx->M));
 	if (ctx->chunks_R != ctx->R ||
 	    ctx->chunks_dense != ((ctx->dense_active ? 1 : 0) | (ctx->m_dense_active ? 2 : 0))) {
-		ctx->pval.release();
-		ctx->Pst.release();
-		ctx->tmax.release();
-		ctx->targ.release();
+		release_pairs(ctx);
 		if (int rc = build_chunks(ctx))
 			return rc;
 	}
-	const size_t pairs = (size_t)ctx->R_pad * ctx->chunk_frames;
-	CK(ctx->pval.ensure(pairs));
-	CK(ctx->Pst.ensure((size_t)ctx->R_pad * (ctx->chunk_frames + 1)));
-	CK(ctx->tmax.ensure((size_t)ctx->RT * ctx->chunk_frames));
-	CK(ctx->targ.ensure((size_t)ctx->RT * ctx->chunk_frames));
-	CK(ctx->tlive.ensure((size_t)ctx->RT * (ctx->chunk_frames + 1)));
+	if (int rc = ensure_pairs(ctx))
+		return rc;
 	CK(ctx->psum_part.ensure((size_t)psum_splits(ctx) * ctx->R_pad));
 	return DFG_OK;
 }
@@ -1378,11 +1396,8 @@ static int hot_choose(dfg_ctx *ctx) {
 			return rc;
 		if (int rc = encode_byte_map(ctx, &ch.map_pixel, by_pixel, n, ch.k_pitch))
 			return rc;
-		std::vector<int> pix((size_t)ch.npix), rest;
-		if (ch.npix > 0)
-			CK(cudaMemcpyAsync(pix.data(), ch.pix.p, pix.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
-		CK(cudaStreamSynchronize(st));
-		for (int p : pix)
+		std::vector<int> rest;
+		for (int p : ch.h_pix)
 			if (!is_hot[p])
 				rest.push_back(p);
 		ch.npix_cold = (int)rest.size();
@@ -1500,13 +1515,21 @@ static int hot_prepare(dfg_ctx *ctx) {
 	const long long rows = (long long)ctx->RT * 2 * 4 * HO;
 	cudaError_t e = cudaSuccess;
 	ctx->hot_estep = !ctx->refine || refine_share(ctx) * (double)ctx->hot_words >= kHotColumnWords * ctx->hot_n * (double)ctx->N;
-	if (ctx->hot_estep) {
+	// the log-slices' digits: with one chunk the E-step is done with them before the
+	// tomograms are cleared, whose memory holds them; else in a buffer
+	ctx->dig_p = nullptr;
+	if (ctx->chunks.size() == 1 && ctx->T.n * sizeof(float) >= (size_t)rows * ctx->hot_pitch && !ctx->dense_active &&
+	    !(ctx->refuse_memory & kSpareDigits)) {
+		ctx->wdig.release();
+		ctx->dig_p = reinterpret_cast<int8_t *>(ctx->T.p);
+	} else if (ctx->hot_estep) {
 		// no memory for them: the E-step gathers, the M-step's products need none
 		ctx->hot_estep = spare_memory(ctx, kSpareDigits, ctx->wdig, (size_t)rows * ctx->hot_pitch, &e);
 		CK(e);
+		ctx->dig_p = ctx->wdig.p;
 	}
 	if (ctx->hot_estep)
-		if (int rc = encode_byte_map(ctx, &ctx->map_wdig, ctx->wdig.p, rows, ctx->hot_pitch))
+		if (int rc = encode_byte_map(ctx, &ctx->map_wdig, ctx->dig_p, rows, ctx->hot_pitch))
 			return rc;
 	CK(ctx->hot_special.ensure((size_t)ctx->RT));
 	CK(ctx->rowmax.ensure((size_t)ctx->R_pad));
@@ -1538,7 +1561,7 @@ static int launch_hot_digits(dfg_ctx *ctx) {
 	cudaStream_t st = ctx->stream;
 	CK(cudaMemsetAsync(ctx->hot_special.p, 0, (size_t)ctx->RT * sizeof(int), st));
 	hot_digits_kernel<false><<<digit_blocks(ctx->RT, ctx->hot_pitch), 256, 0, st>>>(
-	    ctx->logW.p, (size_t)(ctx->P + 1) * TILE, ctx->hot_pix.p, ctx->hot_n, ctx->hot_pitch, nullptr, ctx->wdig.p,
+	    ctx->logW.p, (size_t)(ctx->P + 1) * TILE, ctx->hot_pix.p, ctx->hot_n, ctx->hot_pitch, nullptr, ctx->dig_p,
 	    ctx->hot_special.p, nullptr);
 	CKL("hot_digits_kernel");
 	return DFG_OK;
@@ -1721,9 +1744,9 @@ static int slice_block_for(const dfg_ctx *ctx) {
 // The model's corner quads, read by every slice kernel of this iteration.
 static int launch_quads(dfg_ctx *ctx) {
 	const long long n = (long long)ctx->M * ctx->V;
-	if (!ctx->use_quads)
+	if (ctx->quad_p == nullptr)
 		return DFG_OK;
-	quad_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(ctx->model1.p, n, ctx->S, ctx->quads.p);
+	quad_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(ctx->model1.p, n, ctx->S, ctx->quad_p);
 	CKL("quad_kernel");
 	return DFG_OK;
 }
@@ -2159,13 +2182,8 @@ static int ensure_pair_buffers(dfg_ctx *ctx, const dfg_iter_params *par) {
 	if (!ctx->mw_valid)
 		if (int rc = build_mstep_words(ctx))
 			return rc;
-	ctx->logW.release();
-	ctx->T.release();
-	ctx->pval.release();
-	ctx->Pst.release();
-	ctx->tmax.release();
-	ctx->targ.release();
-	ctx->tlive.release();
+	ctx->tile_slab.release(ctx->logW, ctx->T);
+	release_pairs(ctx);
 	ctx->chunks_R = -1;
 	dense_release(ctx);
 	const size_t N = (size_t)ctx->N, P = (size_t)ctx->P;
@@ -2174,7 +2192,7 @@ static int ensure_pair_buffers(dfg_ctx *ctx, const dfg_iter_params *par) {
 	CK(ctx->psum_r.ensure((size_t)ctx->R_pad));
 	CK(ctx->wsign.ensure((size_t)ctx->R_pad));
 	CK(ctx->scalars.ensure(8));
-	if (int rc = ensure_quads(ctx))
+	if (int rc = ensure_quads(ctx, false))
 		return rc;
 	CK(ctx->red_part.ensure(std::max<size_t>(blocks_for((long long)ctx->M * ctx->V, 256), 1024)));
 	CK(ctx->rmax.ensure(N));
@@ -2373,7 +2391,7 @@ static bool blocked_wanted(dfg_ctx *ctx) {
 		cudaGetLastError();
 		return false;
 	}
-	const size_t held = (ctx->logW.n + ctx->T.n + ctx->blk.n + ctx->blkT.n) * sizeof(float);
+	const size_t held = ctx->tile_slab.mem.n + (ctx->blk.n + ctx->blkT.n) * sizeof(float);
 	return need > (fr + held) / 2;
 }
 
@@ -2392,8 +2410,7 @@ static int blocked_prepare(dfg_ctx *ctx, const dfg_iter_params *par) {
 	ctx->R = ctx->num_rot;
 	ctx->RT = (ctx->R + TILE - 1) / TILE;
 	ctx->R_pad = ctx->RT * TILE;
-	ctx->logW.release();
-	ctx->T.release();
+	ctx->tile_slab.release(ctx->logW, ctx->T);
 	ctx->raw.release();  // per-pair buffer of the pair lists
 	dense_release(ctx);
 	const size_t N = (size_t)ctx->N, P = (size_t)ctx->P;
@@ -2401,7 +2418,7 @@ static int blocked_prepare(dfg_ctx *ctx, const dfg_iter_params *par) {
 	CK(ctx->logw.ensure((size_t)ctx->R_pad));
 	CK(ctx->psum_r.ensure((size_t)ctx->R_pad));
 	CK(ctx->scalars.ensure(8));
-	if (int rc = ensure_quads(ctx))
+	if (int rc = ensure_quads(ctx, false))
 		return rc;
 	CK(ctx->red_part.ensure(std::max<size_t>(blocks_for((long long)ctx->M * ctx->V, 256), 1024)));
 	CK(ctx->rmax.ensure(N));
@@ -2430,19 +2447,12 @@ static int blocked_prepare(dfg_ctx *ctx, const dfg_iter_params *par) {
 		CK(ctx->blkT.ensure((size_t)ctx->blk_tiles * P * TILE));
 	}
 	if (ctx->chunks_R != ctx->R || ctx->chunks_dense != 0) {
-		ctx->pval.release();
-		ctx->Pst.release();
-		ctx->tmax.release();
-		ctx->targ.release();
+		release_pairs(ctx);
 		if (int rc = build_chunks(ctx))
 			return rc;
 	}
-	const size_t pairs = (size_t)ctx->R_pad * ctx->chunk_frames;
-	CK(ctx->pval.ensure(pairs));
-	CK(ctx->Pst.ensure((size_t)ctx->R_pad * (ctx->chunk_frames + 1)));
-	CK(ctx->tmax.ensure((size_t)ctx->RT * ctx->chunk_frames));
-	CK(ctx->targ.ensure((size_t)ctx->RT * ctx->chunk_frames));
-	CK(ctx->tlive.ensure((size_t)ctx->RT * (ctx->chunk_frames + 1)));
+	if (int rc = ensure_pairs(ctx))
+		return rc;
 	CK(ctx->psum_part.ensure((size_t)psum_splits(ctx) * ctx->R_pad));
 	return prepare_weight_cache(ctx);
 }
@@ -2626,7 +2636,11 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 			return rc;
 	phase_end(ctx, PH_SLICE, 4 + (ctx->dense_active ? 1 : 0) + (hot_e ? 1 : 0));
 
-	CK(cudaMemsetAsync(ctx->T.p, 0, (size_t)RT * P * TILE * sizeof(float), st));
+	// the tomograms' memory may hold the digits until the (one) chunk's E-step is done
+	const bool clear_late = hot_e && ctx->dig_p == reinterpret_cast<int8_t *>(ctx->T.p);
+	const size_t tomo_bytes = (size_t)RT * P * TILE * sizeof(float);
+	if (!clear_late)
+		CK(cudaMemsetAsync(ctx->T.p, 0, tomo_bytes, st));
 	CK(cudaMemsetAsync(ctx->psum_r.p, 0, (size_t)R_pad * sizeof(double), st));
 	CK(cudaMemsetAsync(ctx->accum.p, 0, (size_t)M * V * sizeof(double2), st));
 	const int use_scale = par->need_scaling && (par->iteration > 1 || par->known_scale);
@@ -2649,6 +2663,8 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 			return rc;
 		phase_end(ctx, PH_ESTEP,
 		          (ctx->dense_active || ctx->m_dense_active ? 1 : 0) + (ctx->hot_estep && !ctx->dense_active ? 2 : 0) + 1);
+		if (clear_late)
+			CK(cudaMemsetAsync(ctx->T.p, 0, tomo_bytes, st));
 		// normalisation and per-frame sums (normalize_prob + calc_psum_r)
 		phase_begin(ctx, PH_NORM);
 		if (int rc = launch_norm(ctx, ch, psum_d_on, bg))
@@ -2836,6 +2852,8 @@ static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par) {
 	int e_minb = ESTEP_MINB, m_minb = MSTEP_MINB;
 	if (rc == DFG_OK && plain && e_sparse) {
 		const int cand[3] = {2, 3, 4};
+		if (ctx->hot_estep && rc == DFG_OK)   // (the M-step may have written over them)
+			rc = launch_hot_digits(ctx);
 		for (int i = 0; i < 3 && rc == DFG_OK; ++i) {
 			ctx->tune_estep_minb = cand[i];
 			rc = timed([&] { return launch_estep(ctx, c0, use_scale, bg, rm, false); }, rep[10 + i]);

@@ -22,29 +22,40 @@ enum Phase { PH_SLICE, PH_ESTEP, PH_NORM, PH_PSUM, PH_MSTEP, PH_MERGE, PH_UPDATE
 constexpr int kTimingEvents = 2048;  // phase-timing events per context
 static const char *kPhaseNames[PH_COUNT] = {"slice", "estep", "norm", "psum", "mstep", "merge", "update"};
 
-// Owning device buffer; move-only.
+// Owning device buffer, or one lent from a Slab; move-only.
 template <typename T>
 struct DevBuf {
 	T *p = nullptr;
 	size_t n = 0;
+	bool lent = false;
 	DevBuf() = default;
 	DevBuf(const DevBuf &) = delete;
 	DevBuf &operator=(const DevBuf &) = delete;
-	DevBuf(DevBuf &&o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
+	DevBuf(DevBuf &&o) noexcept : p(o.p), n(o.n), lent(o.lent) { o.forget(); }
 	DevBuf &operator=(DevBuf &&o) noexcept {
 		if (this != &o) {
 			release();
-			p = o.p; n = o.n;
-			o.p = nullptr; o.n = 0;
+			p = o.p; n = o.n; lent = o.lent;
+			o.forget();
 		}
 		return *this;
 	}
 	~DevBuf() { release(); }
 	void release() {
-		if (p)
+		if (p && !lent)
 			cudaFree(p);
+		forget();
+	}
+	void borrow(void *from, size_t count) {
+		release();
+		p = static_cast<T *>(from);
+		n = count;
+		lent = true;
+	}
+	void forget() {
 		p = nullptr;
 		n = 0;
+		lent = false;
 	}
 	cudaError_t ensure(size_t count) {
 		if (count <= n && p)
@@ -56,6 +67,37 @@ struct DevBuf {
 		else
 			p = nullptr;
 		return e;
+	}
+};
+
+// Buffers of one lifetime in one allocation: a cudaMalloc of more than a few MB takes
+// 0.4 ms whatever its size, and the first iteration of a small search waits for
+// each.
+template <typename T>
+struct SlabPart {
+	DevBuf<T> &b;
+	size_t n;
+	static size_t bytes(size_t n) { return (n * sizeof(T) + 255) / 256 * 256; }
+};
+struct Slab {
+	DevBuf<uint8_t> mem;
+	// Every part holds its n elements afterwards; parts that already do keep their place.
+	template <typename... T>
+	cudaError_t ensure(SlabPart<T>... part) {
+		if (((part.b.p != nullptr && part.b.n >= part.n) && ...))
+			return cudaSuccess;
+		(part.b.release(), ...);
+		const cudaError_t e = mem.ensure((SlabPart<T>::bytes(part.n) + ...));
+		if (e != cudaSuccess)
+			return e;
+		uint8_t *at = mem.p;
+		((part.b.borrow(at, part.n), at += SlabPart<T>::bytes(part.n)), ...);
+		return cudaSuccess;
+	}
+	template <typename... T>
+	void release(DevBuf<T> &...b) {
+		(b.release(), ...);
+		mem.release();
 	}
 };
 
@@ -94,6 +136,7 @@ struct Chunk {
 	DevBuf<long long> cs_off;  // [P + 1]
 	DevBuf<long long> cs_mid;  // [P] start of the multi-photon segment
 	DevBuf<int> pix;           // pixels with non-empty lists, longest first
+	std::vector<int> h_pix;    // the same on the host
 	int npix = 0;
 	long long entries = 0;
 	// hot pixels (emc_hot.cuh): counts as bytes [nc][hot_pitch] and behind them
@@ -151,7 +194,7 @@ struct dfg_ctx {
 	DevBuf<double> model1, model2, weight;
 	DevBuf<double2> accum;
 	DevBuf<double4> quads;  // the model's corner quads (quad_kernel), remade every iteration
-	bool use_quads = false;
+	double4 *quad_p = nullptr;  // where this iteration has them (ensure_quads); null: none
 	// inter_weight of the last merge and the psum_r > 0 pattern it was built
 	// for (the weights depend on nothing else once geometry is fixed); the
 	// pattern and the flags (accumulate weights, grid cached) live on the
@@ -168,6 +211,7 @@ struct dfg_ctx {
 
 	// work buffers
 	DevBuf<float> logW, Pst, T;
+	Slab tile_slab, pair_slab;  // logW and T; pval, Pst, tmax, targ and tlive
 	DevBuf<double> u, pval, psum_r, psum_part, scalars, red_part;
 	DevBuf<double> logw;  // log w_r per orientation
 	DevBuf<int> rmax, num_prob, targ;
@@ -251,6 +295,7 @@ struct dfg_ctx {
 	DevBuf<uint32_t> phc;
 	DevBuf<long long> phc_off, phc_mid;
 	DevBuf<int8_t> wdig;
+	int8_t *dig_p = nullptr;   // where this iteration has them (hot_prepare)
 	DevBuf<float> rowmax, rowmax_part;
 	CUtensorMap map_wdig;
 	int max_fcount = 0;        // most photons of a frame
