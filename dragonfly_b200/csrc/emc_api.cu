@@ -686,9 +686,10 @@ extern "C" int dfg_calc_beta(dfg_ctx *ctx, double start, int need_scaling) {
 // ---------------------------------------------------------------------------
 // work buffers and the frame chunks
 // ---------------------------------------------------------------------------
-// Largest photon sum that the byte products' INT32 accumulators hold: 2^24
-// counts times a digit of at most 128 in magnitude.
-constexpr long long kHotMaxSum = 1LL << 24;
+// Photon sums that the byte products' INT32 accumulators hold: of a frame, below 2^24
+// counts times a signed digit of at most 128 in magnitude; of a pixel over a
+// chunk, below 2^23 times an unsigned one of at most 255.
+constexpr long long kHotMaxFrame = 1LL << 24, kHotMaxPixel = 1LL << 23;
 
 static int build_chunks(dfg_ctx *ctx) {
 	const int N = ctx->N, P = ctx->P;
@@ -806,7 +807,7 @@ static int build_chunks(dfg_ctx *ctx) {
 			}
 			real += n1 + nm;
 			ctx->h_pix_entries[p] += n1 + nm;
-			if (ph >= kHotMaxSum)
+			if (ph >= kHotMaxPixel)
 				ctx->h_pix_big[p] = 1;
 		}
 		const std::unique_ptr<uint32_t[]> words(new uint32_t[(size_t)std::max<long long>(off[P], 1)]);
@@ -1352,7 +1353,7 @@ static int hot_choose(dfg_ctx *ctx) {
 		ch.pix_cold.release();
 		ch.csc.release();
 	}
-	if (TILE != 128 || ctx->RT > 65535 || ctx->chunk_frames < HM || ctx->max_fcount >= kHotMaxSum)
+	if (TILE != 128 || ctx->RT > 65535 || ctx->chunk_frames < HM || ctx->max_fcount >= kHotMaxFrame)
 		return DFG_OK;
 	std::vector<int> cand;
 	for (int p = 0; p < P; ++p)

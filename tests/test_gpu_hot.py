@@ -100,21 +100,51 @@ def test_near_ties_fall_as_with_the_gathers(copies, turn, scaling):
 def test_products_lose_no_precision_at_small_logarithms(oracle_built):
     """A start model of about one photon per pixel, where log W is small and FP32
     holds it finely: the digits must too. The gathers' compensated sums round once
-    more per photon, so the products' model is as close to the oracle's (its error
-    is a sum over few orientations here, hence the half)."""
-    d, shared = synth.two_detector_problem(seed=8, n_frames=(300, 200))
-    d = d[0]
-    prob = EMCProblem(d["qvals"], d["corr"], d["mask"], d["ones"], d["multi"], d["place_ones"], d["place_multi"],
-                      d["count_multi"], shared["quats"], shared["model_start"], need_scaling=1, update_scale=1, beta=0.5)
-    want = OracleEngine(prob).run_iteration(1)["model1"]
-    off = []
-    for skip in (0, 1):
-        gpu = GPUEngine(prob, tile_skip=skip)
-        off.append(np.linalg.norm(gpu.run_iteration(1)["model1"] - want))
-        took = gpu.ctx.products()
-        assert took["estep"] == took["mstep"] == 1 - skip and (took["pixels"] >= 128) == (skip == 0)
-        gpu.close()
-    assert off[0] <= 1.5 * off[1]
+    more per photon, so the products' log-likelihoods are as close to the oracle's;
+    the model's error is a sum over few orientations here (hence the half)."""
+    model, like = [], []
+    for seed in (8, 9, 10, 11):
+        d, shared = synth.two_detector_problem(seed=seed, n_frames=(300, 200))
+        d = d[0]
+        prob = EMCProblem(d["qvals"], d["corr"], d["mask"], d["ones"], d["multi"], d["place_ones"], d["place_multi"],
+                          d["count_multi"], shared["quats"], shared["model_start"], need_scaling=1, update_scale=1,
+                          beta=0.5)
+        want = OracleEngine(prob).run_iteration(1)
+        off = []
+        for skip in (0, 1):
+            gpu = GPUEngine(prob, tile_skip=skip)
+            got = gpu.run_iteration(1)
+            off.append([np.linalg.norm(got[k] - want[k]) for k in ("model1", "likelihood")])
+            took = gpu.ctx.products()
+            assert took["estep"] == took["mstep"] == 1 - skip and (took["pixels"] >= 128) == (skip == 0)
+            gpu.close()
+        model.append(off[0][0] / off[1][0])
+        like.append(off[0][1] / off[1][1])
+    assert model[0] <= 1.5
+    assert np.exp(np.mean(np.log(like))) <= 1.
+
+
+@pytest.mark.parametrize("frames,fits", [(32800, True), (33000, False)])
+def test_a_pixel_at_the_range_of_the_accumulators(frames, fits):
+    """Every frame has 255 photons on one pixel and is sure of the only orientation: the
+    top digits' sum is 250 x 255 x frames, 0.974 of 2^31 at 32800. With 33000 the pixel
+    has more than 2^23 photons and stays with the gathers."""
+    prob = _problem(300, 1, 24, 200.)
+    good = np.nonzero(prob.mask == 0)[0]
+    rng = np.random.default_rng(12)
+    place = np.concatenate([rng.choice(good[1:], 12, replace=False) for _ in range(frames)]).astype(np.int32)
+    ones, multi = np.full(frames, 12, np.int32), np.ones(frames, np.int32)
+    prob = EMCProblem(prob.qvals, prob.corr, prob.mask, ones, multi, place, np.full(frames, good[0], np.int32),
+                      np.full(frames, 255, np.int32), prob.quats[:1], prob.model1, need_scaling=0, beta=0.1)
+    gpu = GPUEngine(prob)
+    gpu.ctx.maximize(gpu.ctx.params(1, 0, 0, 0, 1., 100, 1.))
+    took = gpu.ctx.products()
+    # 512 of the 540 pixels: the bright one and 511 others, or 512 others
+    assert took["mstep"] and (took["words"] > 11.9 * frames) == fits
+    want = np.bincount(place, minlength=prob.num_pix) / frames
+    want[good[0]] = 255.
+    np.testing.assert_allclose(gpu.ctx.tomograms(0, 1)[0], want, rtol=4 * 2. ** -24)
+    gpu.close()
 
 
 @pytest.mark.parametrize("cells_per_frame", [0, 1, 6])
