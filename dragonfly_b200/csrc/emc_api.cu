@@ -691,8 +691,30 @@ extern "C" int dfg_calc_beta(dfg_ctx *ctx, double start, int need_scaling) {
 // chunk, below 2^23 times an unsigned one of at most 255.
 constexpr long long kHotMaxFrame = 1LL << 24, kHotMaxPixel = 1LL << 23;
 
+// Gives the products' buffers back (the next iteration that takes products lays
+// them out again).
+static void hot_release(dfg_ctx *ctx) {
+	for (Chunk &ch : ctx->chunks) {
+		ch.counts.release();
+		ch.pix_cold.release();
+		ch.csc.release();
+		ch.csc_off.release();
+		ch.csc_mid.release();
+	}
+	ctx->phc.release();
+	ctx->phc_off.release();
+	ctx->phc_mid.release();
+	ctx->wdig.release();
+	ctx->hot_n = 0;
+	ctx->hot_layout = -1;
+}
+
 static int build_chunks(dfg_ctx *ctx) {
 	const int N = ctx->N, P = ctx->P;
+	// the last layout's lists and count matrices are no part of the memory in use
+	hot_release(ctx);
+	ctx->chunks.clear();
+	ctx->chunks_R = -1;
 	// per frame: pval and Pst of every orientation, plus its BF16 count row
 	// in the dense form
 	const bool any_dense = ctx->dense_active || ctx->m_dense_active;
@@ -713,7 +735,6 @@ static int build_chunks(dfg_ctx *ctx) {
 	const int n_chunks = (int)((N + nc - 1) / nc);
 	nc = (N + n_chunks - 1) / n_chunks;  // even chunks
 	ctx->chunk_frames = (int)nc;
-	ctx->chunks.clear();
 	ctx->chunks.resize(n_chunks);
 
 	// M-step index per chunk: photons on mask < 2 pixels grouped by pixel
@@ -913,8 +934,6 @@ static int ensure_buffers(dfg_ctx *ctx) {
 	CK(ctx->logw.ensure((size_t)ctx->R_pad));
 	CK(ctx->psum_r.ensure((size_t)ctx->R_pad));
 	CK(ctx->scalars.ensure(8));
-	if (int rc = ensure_quads(ctx, true))
-		return rc;
 	CK(ctx->red_part.ensure(std::max<size_t>(blocks_for((long long)ctx->M * ctx->V, 256), 1024)));
 	const size_t N = (size_t)ctx->N;
 	CK(ctx->rmax.ensure(N));
@@ -1345,14 +1364,8 @@ static bool spare_memory(dfg_ctx *ctx, int what, DevBuf<T> &b, size_t n, cudaErr
 static int hot_choose(dfg_ctx *ctx) {
 	const int N = ctx->N, P = ctx->P;
 	cudaStream_t st = ctx->stream;
-	ctx->hot_n = 0;
+	hot_release(ctx);
 	ctx->hot_layout = ctx->layout;
-	ctx->phc.release();
-	for (Chunk &ch : ctx->chunks) {
-		ch.counts.release();
-		ch.pix_cold.release();
-		ch.csc.release();
-	}
 	if (TILE != 128 || ctx->RT > 65535 || ctx->chunk_frames < HM || ctx->max_fcount >= kHotMaxFrame)
 		return DFG_OK;
 	std::vector<int> cand;
@@ -1461,12 +1474,8 @@ static int hot_choose(dfg_ctx *ctx) {
 		}
 	}
 	if (!room) {
-		ctx->phc.release();
-		for (Chunk &ch : ctx->chunks) {
-			ch.counts.release();
-			ch.pix_cold.release();
-			ch.csc.release();
-		}
+		hot_release(ctx);
+		ctx->hot_layout = ctx->layout;
 		return DFG_OK;
 	}
 	ctx->hot_n = n;
@@ -1685,13 +1694,6 @@ static int max_prepare(dfg_ctx *ctx, const dfg_iter_params *par) {
 	if (ctx->dense_active || ctx->m_dense_active)
 		if (int rc = dense_prepare_counts(ctx))
 			return rc;
-	// the sparse forms leave the hot pixels to the products: both steps of the
-	// full search, the M-step of a refined one (10860 orientations x 12000 frames
-	// near 12 of 420 cells: M-step 3.95 -> 1.04 ms)
-	if ((ctx->refine || !ctx->mstep_skip) && !(ctx->with_bg && par->need_scaling) &&
-	    (ctx->tuning || !(ctx->dense_active && ctx->m_dense_active)))
-		if (int rc = hot_prepare(ctx))
-			return rc;
 	cudaStream_t st = ctx->stream;
 	if (ctx->refine && !ctx->h_watch.empty()) {  // chunk-local indices of the watched frames
 		std::vector<int> local(ctx->h_watch.size());
@@ -1717,7 +1719,19 @@ static int max_prepare(dfg_ctx *ctx, const dfg_iter_params *par) {
 	if (ctx->refine)
 		if (int rc = prepare_qmap(ctx))
 			return rc;
-	return prepare_weight_cache(ctx);
+	if (int rc = prepare_weight_cache(ctx))
+		return rc;
+	// what an iteration can do without comes last: the corner quads' buffer and the
+	// products'. The sparse forms leave the hot pixels to the products: both steps of
+	// the full search, the M-step of a refined one (10860 orientations x 12000 frames
+	// near 12 of 420 cells: M-step 3.95 -> 1.04 ms)
+	if (int rc = ensure_quads(ctx, true))
+		return rc;
+	if ((ctx->refine || !ctx->mstep_skip) && !(ctx->with_bg && par->need_scaling) &&
+	    (ctx->tuning || !(ctx->dense_active && ctx->m_dense_active)))
+		return hot_prepare(ctx);
+	hot_release(ctx);
+	return DFG_OK;
 }
 
 // Whether one iteration queues its kernels without waiting on the host: the
@@ -2185,6 +2199,7 @@ static int ensure_pair_buffers(dfg_ctx *ctx, const dfg_iter_params *par) {
 			return rc;
 	ctx->tile_slab.release(ctx->logW, ctx->T);
 	release_pairs(ctx);
+	hot_release(ctx);
 	ctx->chunks_R = -1;
 	dense_release(ctx);
 	const size_t N = (size_t)ctx->N, P = (size_t)ctx->P;
@@ -2193,8 +2208,6 @@ static int ensure_pair_buffers(dfg_ctx *ctx, const dfg_iter_params *par) {
 	CK(ctx->psum_r.ensure((size_t)ctx->R_pad));
 	CK(ctx->wsign.ensure((size_t)ctx->R_pad));
 	CK(ctx->scalars.ensure(8));
-	if (int rc = ensure_quads(ctx, false))
-		return rc;
 	CK(ctx->red_part.ensure(std::max<size_t>(blocks_for((long long)ctx->M * ctx->V, 256), 1024)));
 	CK(ctx->rmax.ensure(N));
 	CK(ctx->num_prob.ensure(N));
@@ -2212,8 +2225,11 @@ static int ensure_pair_buffers(dfg_ctx *ctx, const dfg_iter_params *par) {
 		ctx->blk.release();
 		ctx->blk_tiles = 0;
 		ctx->raw.release();
+		ctx->quads.release();
 		CK(ctx->raw.ensure(need + need / 10));
 	}
+	if (int rc = ensure_quads(ctx, false))
+		return rc;
 	// one orientation block: (P + 1) x 128 floats per tile (log-slices with
 	// their zero row; the tomograms use P rows of the same space)
 	const size_t tile_bytes = (P + 1) * TILE * sizeof(float);
@@ -2412,6 +2428,7 @@ static int blocked_prepare(dfg_ctx *ctx, const dfg_iter_params *par) {
 	ctx->RT = (ctx->R + TILE - 1) / TILE;
 	ctx->R_pad = ctx->RT * TILE;
 	ctx->tile_slab.release(ctx->logW, ctx->T);
+	hot_release(ctx);
 	ctx->raw.release();  // per-pair buffer of the pair lists
 	dense_release(ctx);
 	const size_t N = (size_t)ctx->N, P = (size_t)ctx->P;

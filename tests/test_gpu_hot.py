@@ -282,6 +282,36 @@ def test_without_memory_for_the_products(refused):
     gpu.close()
 
 
+def test_products_give_their_memory_back():
+    """A context that goes from a full search to pair lists holds no more than one that
+    began with them (the count matrices alone are 20 MB here)."""
+    import torch
+    prob = _problem(300, 2, 24, 200.)
+    n, R = 20100, prob.quats.shape[0]
+    rep = lambda a: np.tile(a, n // 300)
+    prob = EMCProblem(prob.qvals, prob.corr, prob.mask, rep(prob.ones), rep(prob.multi), rep(prob.place_ones),
+                      rep(prob.place_multi), rep(prob.count_multi), prob.quats, prob.model1, need_scaling=1,
+                      update_scale=1, beta=0.1)
+    cells = (np.arange(R) * 7 // R).astype(np.int32)
+    lists = np.tile(np.array([[0, 3]], np.int32), (n, 1))
+    held = []
+    for full_first in (False, True):
+        before = torch.cuda.mem_get_info()[0]
+        gpu = GPUEngine(prob)
+        par = gpu.ctx.params(1, 1, 0, 0, 1., 100, 1.)
+        if full_first:
+            gpu.ctx.maximize(par)
+            assert gpu.ctx.products()["pixels"] >= 256
+        gpu.ctx.set_refinement(7, cells, lists)
+        gpu.ctx.set_option("pair_lists", 1)
+        gpu.ctx.set_option("block_budget_mb", 16)
+        gpu.ctx.maximize(par)
+        assert gpu.ctx.products()["pixels"] == 0
+        held.append(before - torch.cuda.mem_get_info()[0])
+        gpu.close()
+    assert held[1] - held[0] <= 8 << 20
+
+
 def test_product_wait_gives_up_and_the_context_recovers(oracle_built):
     """A stage whose copies are withheld (test hook): its waits run out, the
     kernels return, the call reports the error, and the next call succeeds."""
