@@ -2764,7 +2764,7 @@ static int max_enqueue(dfg_ctx *ctx, const dfg_iter_params *par) {
 }
 
 // Project autotuner. On the context's own inputs it times (CUDA events, best
-// of two after a warm-up launch) the slice kernel with 128, 64, 32 and 16 orientations per block and
+// of two after a warm-up launch) the slice kernel with 128, 64, 32, 16 and 8 orientations per block and
 // both forms of the E-step photon term and of the M-step (sparse gathers,
 // dense tensor-core products where the inputs allow them) on the first frame
 // chunk, and keeps the fastest of each; then, where the sparse gathers won,
@@ -2823,6 +2823,11 @@ static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par) {
 			bi = i;
 	}
 	const int best_ob = bi >= 0 ? obs[bi] : 0;
+	// (the report has no place for it: slice_block_for's choice for small sets)
+	double ms8 = -1.;
+	if (rc == DFG_OK)
+		rc = timed([&] { return launch_slices(ctx, 8, Wd); }, ms8);
+	const bool narrow = bi >= 0 && ms8 >= 0. && ms8 < rep[bi];
 	const int use_scale = par->need_scaling && (par->iteration > 1 || par->known_scale);
 	if (rc == DFG_OK) {
 		// the E-step's other inputs
@@ -2830,21 +2835,26 @@ static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par) {
 		CKL("rescale_kernel");
 		logw_kernel<<<blocks_for(ctx->R, 256), 256, 0, st>>>(ctx->quats.p, ctx->M, ctx->R, ctx->logw.p);
 		CKL("logw_kernel");
-		if (ctx->hot_estep)
-			rc = launch_hot_digits(ctx);
+		// each form with its conversion of the log-slices
+		rc = timed(
+		    [&] {
+			    if (ctx->hot_estep)
+				    if (int r = launch_hot_digits(ctx))
+					    return r;
+			    return launch_estep(ctx, ctx->chunks[0], use_scale, bg, rm, false);
+		    },
+		    rep[4]);
 	}
-	if (rc == DFG_OK)
-		rc = timed([&] { return launch_estep(ctx, ctx->chunks[0], use_scale, bg, rm, false); }, rep[4]);
 	const Chunk &c0 = ctx->chunks[0];
 	if (rc == DFG_OK && dense_ok) {
-		split_logw_kernel<<<dim3(ctx->K_pad / DK, ctx->RT), 256, 0, st>>>(
-		    ctx->logW.p, ctx->P, ctx->kpix.p, ctx->mask.p, ctx->K, ctx->K_pad, (__nv_bfloat16 *)ctx->Ahi.p,
-		    (__nv_bfloat16 *)ctx->Alo.p);
-		CKL("split_logw_kernel");
 		// the densification counts to the dense E-step (when the M-step stays
 		// sparse it is needed for the E-step alone)
 		rc = timed(
-		    [&] {
+		    [&]() -> int {
+			    split_logw_kernel<<<dim3(ctx->K_pad / DK, ctx->RT), 256, 0, st>>>(
+			        ctx->logW.p, ctx->P, ctx->kpix.p, ctx->mask.p, ctx->K, ctx->K_pad, (__nv_bfloat16 *)ctx->Ahi.p,
+			        (__nv_bfloat16 *)ctx->Alo.p);
+			    CKL("split_logw_kernel");
 			    if (int r = launch_densify(ctx, c0))
 				    return r;
 			    return launch_estep(ctx, c0, use_scale, bg, rm, true);
@@ -2909,7 +2919,7 @@ static int run_autotune(dfg_ctx *ctx, const dfg_iter_params *par) {
 	ctx->timing = save_timing;
 	if (rc != DFG_OK)
 		return rc;
-	ctx->tuned_ob = best_ob;
+	ctx->tuned_ob = narrow ? 8 : best_ob;
 	ctx->tuned_form = (dense_ok && rep[5] >= 0. && rep[5] < rep[4]) ? 1 : 0;
 	ctx->tuned_mform = (dense_ok && rep[9] >= 0. && (rep[8] < 0. || rep[9] < rep[8])) ? 1 : 0;
 	ctx->tuned_estep_minb = e_minb;

@@ -271,7 +271,7 @@ DFG_API int dfg_slice_gen_noalloc(dfg_ctx *ctx, const double *quat, int mode, do
 DFG_API int dfg_run_iteration(dfg_ctx *ctx, const dfg_iter_params *par, double alpha, double *out);
 
 /* Autotuner: on the context's current inputs, times the slice kernel with
- * 128, 64, 32 and 16 orientations per block, and the E-step photon term and
+ * 128, 64, 32, 16 and 8 orientations per block, and the E-step photon term and
  * the M-step each in their sparse (gathers) and dense (tensor-core) forms on
  * the first frame chunk, and keeps the fastest of each for later iterations
  * when option autotune is 1 (with option autotune, dfg_maximize /
@@ -279,9 +279,10 @@ DFG_API int dfg_run_iteration(dfg_ctx *ctx, const dfg_iter_params *par, double a
  * When the sparse forms win it also times the sparse E-step at 2, 3 and 4
  * resident blocks per SM and the sparse M-step at 3, 4 and 5 (launch bounds:
  * registers per thread traded against warps in flight) and keeps the fastest.
- * report[DFG_TUNE_REPORT] (may be NULL): [0-3] slice ms per block size (-1:
- * not tried), [4-5] sparse and dense E-step ms (-1: form refused), [6] the
- * chosen block, [7] the chosen forms (E-step + 2 x M-step, 1 = dense), [8-9]
+ * report[DFG_TUNE_REPORT] (may be NULL): [0-3] slice ms at 128, 64, 32 and 16
+ * (-1: not tried), [4-5] sparse and dense E-step ms with their conversions of
+ * the log-slices (-1: form refused), [6] the fastest of these blocks (8, whose
+ * time has no slot, is taken where it is faster still), [7] the chosen forms (E-step + 2 x M-step, 1 = dense), [8-9]
  * sparse and dense M-step ms, [10-12] sparse E-step ms at 2, 3, 4 blocks per
  * SM, [13-15] sparse M-step ms at 3, 4, 5 blocks per SM (-1: not timed),
  * [16] and [17] the chosen E-step and M-step blocks per SM. */

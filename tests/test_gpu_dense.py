@@ -97,6 +97,30 @@ def test_autotuner_times_both_forms_and_keeps_the_fastest(oracle_built, case):
     plain.close()
 
 
+def test_autotuned_slices_are_no_slower_than_the_automatic_block():
+    """3240 orientations x 64 x 64 pixels, where 8 orientations per block (the automatic
+    choice) take 0.24 ms and 16 take 0.31."""
+    from dragonfly_b200 import synth
+    d = synth.small_problem(seed=5, det_side=64, size=61, qmax=29., n_atoms=60, atom_radius=4., num_div=4, n_frames=300,
+                            mean_count=100., hole_radius=2.)
+    prob = EMCProblem(d["qvals"], d["corr"], d["mask"], d["ones"], d["multi"], d["place_ones"], d["place_multi"],
+                      d["count_multi"], d["quats"], d["model_start"], need_scaling=0, beta=0.1)
+    ms = []
+    for tune in (0, 1):
+        gpu = GPUEngine(prob, autotune=tune)
+        par = gpu.ctx.params(1, 0, 0, 0, 1., 100, 1.)
+        gpu.ctx.maximize(par)
+        gpu.ctx.set_option("timing", 1)
+        best = 1e30
+        for _ in range(10):
+            gpu.ctx.reset_phase_times()
+            gpu.ctx.maximize(par)
+            best = min(best, gpu.ctx.phase_times()["slice"][0])
+        ms.append(best)
+        gpu.close()
+    assert ms[1] <= 1.15 * ms[0], ms
+
+
 @pytest.mark.parametrize("forms", [(1, 0), (0, 1)], ids=["estep", "mstep"])
 def test_dense_pipeline_wait_gives_up_and_the_context_recovers(oracle_built, forms):
     """Failure detection of the tensor-core kernels without a GPU fault: with
