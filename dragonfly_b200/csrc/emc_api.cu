@@ -1898,6 +1898,7 @@ static int launch_estep(dfg_ctx *ctx, const Chunk &ch, int use_scale, bool bg, c
 	if (ctx->hot_estep) {
 		if (int rc = launch_hot_estep(ctx, ch))
 			return rc;
+#if DFG_LANE_W == 4
 		const HotLists full{ctx->hot_special.p, ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p};
 #define DFG_ECOLD(REF, MB)                                                                                    \
 	estep_cold_kernel<REF, MB><<<dim3(blocks_for(Nc, 8), RT), 256, 0, st>>>(                                       \
@@ -1919,6 +1920,7 @@ static int launch_estep(dfg_ctx *ctx, const Chunk &ch, int use_scale, bool bg, c
 		    ctx->blacklist.p, ctx->fcounts.p, ch.d0, Nc, RT, use_scale, ctx->scalars.p, P, ctx->pval.p, ctx->tmax.p,
 		    ctx->targ.p);
 		CKL("estep_ties_kernel");
+#endif
 		return DFG_OK;
 	}
 #define DFG_ESTEP(REF, MB)                                                                                    \

@@ -42,7 +42,7 @@
 namespace dfg {
 
 constexpr int LW = DFG_LANE_W;
-static_assert(LW == 1 || LW == 2 || LW == 4, "lane width must be 1, 2 or 4");
+static_assert(LW == 2 || LW == 4, "lane width must be 2 or 4");
 constexpr int TILE = 32 * LW;
 constexpr int IDX_BITS = 22;
 constexpr uint32_t IDX_MASK = (1u << IDX_BITS) - 1u;
@@ -50,7 +50,7 @@ constexpr uint32_t MAX_COUNT = (1u << (32 - IDX_BITS)) - 1u;
 constexpr double PROB_MIN = 1.e-6;          // dragonfly/src/max_internal.h:6
 constexpr double PDIFF_THRESH = 14.;        // dragonfly/src/max_internal.h:7
 constexpr double MAX_EXP_START = -1.e100;   // dragonfly/src/max_internal.h:8
-constexpr int PB = 64;                      // pixels per block in slice / merge kernels
+constexpr int PB = 64;                      // pixels per block of merge_change_kernel
 constexpr int MAX_MODES = 16;
 constexpr unsigned FULL = 0xffffffffu;
 
@@ -339,7 +339,7 @@ __device__ __forceinline__ double kahan_value(float s, float comp) {
 // component): a compensated addition of two orientations costs four
 // instructions instead of eight, with results identical to the scalar form.
 typedef unsigned long long f32x2;
-constexpr int NPAIR = LW / 2 > 0 ? LW / 2 : 1;  // pairs per lane
+constexpr int NPAIR = LW / 2;  // pairs per lane
 
 __device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
 	f32x2 d;
@@ -404,11 +404,9 @@ __device__ __forceinline__ void ld_row(const float *__restrict__ p, float (&v)[L
 	if constexpr (LW == 4) {
 		const float4 x = __ldg(reinterpret_cast<const float4 *>(p));
 		v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-	} else if constexpr (LW == 2) {
+	} else {
 		const float2 x = __ldg(reinterpret_cast<const float2 *>(p));
 		v[0] = x.x; v[1] = x.y;
-	} else {
-		v[0] = __ldg(p);
 	}
 }
 
@@ -429,33 +427,25 @@ __device__ __forceinline__ void ld_row_rw(const float *p, float (&v)[LW]) {
 	if constexpr (LW == 4) {
 		const float4 x = *reinterpret_cast<const float4 *>(p);
 		v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-	} else if constexpr (LW == 2) {
+	} else {
 		const float2 x = *reinterpret_cast<const float2 *>(p);
 		v[0] = x.x; v[1] = x.y;
-	} else {
-		v[0] = *p;
 	}
 }
 
 __device__ __forceinline__ void st_row(float *p, const float (&v)[LW]) {
 	if constexpr (LW == 4)
 		*reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-	else if constexpr (LW == 2)
-		*reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
 	else
-		*p = v[0];
+		*reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
 }
 
 __device__ __forceinline__ void ld_row(const double *__restrict__ p, double (&v)[LW]) {
-	if constexpr (LW == 1) {
-		v[0] = __ldg(p);
-	} else {
 #pragma unroll
-		for (int k = 0; k < LW; k += 2) {
-			const double2 x = __ldg(reinterpret_cast<const double2 *>(p + k));
-			v[k] = x.x;
-			v[k + 1] = x.y;
-		}
+	for (int k = 0; k < LW; k += 2) {
+		const double2 x = __ldg(reinterpret_cast<const double2 *>(p + k));
+		v[k] = x.x;
+		v[k + 1] = x.y;
 	}
 }
 
@@ -469,13 +459,9 @@ __device__ __forceinline__ void ld_row32(const double *__restrict__ p, double (&
 }
 
 __device__ __forceinline__ void st_row(double *p, const double (&v)[LW]) {
-	if constexpr (LW == 1) {
-		*p = v[0];
-	} else {
 #pragma unroll
-		for (int k = 0; k < LW; k += 2)
-			*reinterpret_cast<double2 *>(p + k) = make_double2(v[k], v[k + 1]);
-	}
+	for (int k = 0; k < LW; k += 2)
+		*reinterpret_cast<double2 *>(p + k) = make_double2(v[k], v[k + 1]);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {

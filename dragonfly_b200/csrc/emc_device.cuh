@@ -175,13 +175,11 @@ __global__ void __launch_bounds__(256) rescale_kernel(const double *__restrict__
 // One warp per (orientation tile, frame), tiles outermost so that resident
 // warps share one tile's log-slices in L2. Each photon costs one coalesced
 // row read (one LW-wide vector load per lane) and a compensated FP32
-// addition per orientation (no conversion instructions in the loop; with one
-// orientation per lane two interleaved accumulators halve the dependency
-// chain); padded segments need no per-photon bounds test. The photon sum is
-// formed in FP64 once per pair. s_d = phi_d when need_scaling &&
+// addition per orientation (no conversion instructions in the loop); padded
+// segments need no per-photon bounds test. The photon sum is formed in FP64
+// once per pair. s_d = phi_d when need_scaling &&
 // (iteration > 1 || known_scale), else the rescale factor (max_prob.c:122-128).
-constexpr int ECH = LW == 1 ? 2 : 1;  // accumulator chains per orientation
-constexpr int ESTEP_MINB = LW == 1 ? 6 : (LW == 2 ? 4 : 3);
+constexpr int ESTEP_MINB = LW == 2 ? 4 : 3;
 
 // Coarse-to-fine refinement (param->refine, max_prob.c:110-120): frame d
 // evaluates orientation r only when r's coarse cell qmap[r] is one of the
@@ -251,12 +249,10 @@ __global__ void __launch_bounds__(256, MINB) estep_kernel(
 	// segments start at multiples of 8 words: two 16-byte loads, identical for
 	// every lane (broadcast), bring 8 photon words
 	const uint4 *w4 = reinterpret_cast<const uint4 *>(ph);
-	float s[ECH][LW], c[ECH][LW];
+	float s[LW], c[LW];
 #pragma unroll
-	for (int h = 0; h < ECH; ++h)
-#pragma unroll
-		for (int k = 0; k < LW; ++k)
-			s[h][k] = c[h][k] = 0.f;
+	for (int k = 0; k < LW; ++k)
+		s[k] = c[k] = 0.f;
 	// the next 8 words are fetched while the current 8 rows are in flight
 	uint4 a = make_uint4(P, P, P, P), b = a;
 	if (beg < mid) {
@@ -281,7 +277,7 @@ __global__ void __launch_bounds__(256, MINB) estep_kernel(
 		for (int q = 0; q < 8; ++q)
 #pragma unroll
 			for (int k = 0; k < LW; ++k)
-				kahan_add(s[q % ECH][k], c[q % ECH][k], v[q][k]);
+				kahan_add(s[k], c[k], v[q][k]);
 	}
 	for (long long j = mid; j < end; j += 8) {
 		const uint4 a = __ldg(w4 + (j >> 2)), b = __ldg(w4 + (j >> 2) + 1);
@@ -294,7 +290,7 @@ __global__ void __launch_bounds__(256, MINB) estep_kernel(
 		for (int q = 0; q < 8; ++q)
 #pragma unroll
 			for (int k = 0; k < LW; ++k)
-				kahan_add_count(s[q % ECH][k], c[q % ECH][k], e[q] >> IDX_BITS, v[q][k]);
+				kahan_add_count(s[k], c[k], e[q] >> IDX_BITS, v[q][k]);
 	}
 	const double sd = use_scale ? scale[d] : scalars[0];
 	double acc[LW];
@@ -307,9 +303,7 @@ __global__ void __launch_bounds__(256, MINB) estep_kernel(
 		const int r = r0 + k;
 		acc[k] = 0.;
 		if (r < R) {
-			double ph_sum = kahan_value(s[0][k], c[0][k]);
-			if (ECH == 2)
-				ph_sum = dadd(ph_sum, kahan_value(s[ECH - 1][k], c[ECH - 1][k]));
+			double ph_sum = kahan_value(s[k], c[k]);
 			acc[k] = dadd(dsub(logw[r], dmul(u[r], sd)), ph_sum);
 			if (REFINE && !(live >> k & 1u))
 				acc[k] = -INFINITY;
@@ -364,6 +358,7 @@ __global__ void __launch_bounds__(256) refine_count_kernel(RefineMask rm, int N,
 		atomicAdd(out, (unsigned long long)live);
 }
 
+#if DFG_LANE_W == 4   // the products need 128-orientation tiles (hot_choose)
 template <bool REFINE, int MINB>
 __global__ void __launch_bounds__(256, MINB) estep_cold_kernel(
     const float *__restrict__ logW, const double *__restrict__ u, const double *__restrict__ logw, int R,
@@ -371,7 +366,6 @@ __global__ void __launch_bounds__(256, MINB) estep_cold_kernel(
     const double *__restrict__ scale, const uint8_t *__restrict__ blacklist, int d0, int Nc, int use_scale,
     const double *__restrict__ scalars, int P, double *pval, double *__restrict__ tmax, int *__restrict__ targ,
     HotLists full, RefineMask rm) {
-	static_assert(LW == 4, "the products need 128-orientation tiles");
 	const int rt = blockIdx.y, dl = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, d = d0 + dl;
 	if (dl >= Nc || blacklist[d])
 		return;
@@ -486,6 +480,7 @@ __global__ void __launch_bounds__(256, MINB) estep_cold_kernel(
 		targ[(size_t)rt * Nc + dl] = am;
 	}
 }
+#endif
 
 // Near ties of the most likely orientation. The products add the log-slices
 // exactly, the gathers round once per photon word, so two orientations that agree
@@ -668,7 +663,6 @@ constexpr int NORM_RING = 6;
 template <typename F>
 __device__ __forceinline__ void stream_rows(const double *__restrict__ src, size_t stride, int RT,
                                             double *ring, int lane, F &&f) {
-	static_assert(LW % 2 == 0, "rows are copied 16 bytes at a time");
 	double *mine = ring + lane * LW;
 	auto issue = [&](int rt) {
 		const double *g = src + (size_t)rt * stride;
@@ -736,7 +730,7 @@ __global__ void __launch_bounds__(256, DFG_NORM_MINB) norm_kernel(
     double *__restrict__ max_exp, double *__restrict__ p_norm, double *__restrict__ info,
     double *__restrict__ likelihood, double *__restrict__ psum_d, double *__restrict__ quat_norm,
     int *__restrict__ num_prob, double *__restrict__ Pd, uint8_t *__restrict__ tlive, int zero_dead) {
-	constexpr int UNR = LW == 1 ? 4 : 2;
+	constexpr int UNR = 2;
 	// without tile skipping every row of the frame is read, twice: both passes
 	// stream them through a per-warp ring (stream_rows)
 	__shared__ __align__(16) double s_ring[SKIP ? 1 : 8][SKIP ? 1 : NORM_RING * TILE];
@@ -1233,129 +1227,88 @@ __global__ void __launch_bounds__(256, MINB) mstep_kernel(const float *__restric
 	};
 	const long long beg = cs_off[p], mid = cs_mid[p], end = cs_off[p + 1];
 	const uint4 *w4 = reinterpret_cast<const uint4 *>(cs);
-	float s[ECH][LW], c[ECH][LW];
+	float s[LW], c[LW];
+	// orientations in pairs: paired FP32 compensated additions; the next
+	// 8 words are fetched while the current 8 rows are in flight
+	constexpr int NP = NPAIR;
+	f32x2 s2[NP], c2[NP];
 #pragma unroll
-	for (int h = 0; h < ECH; ++h)
-#pragma unroll
-		for (int k = 0; k < LW; ++k)
-			s[h][k] = c[h][k] = 0.f;
-	if constexpr (LW >= 2) {
-		// orientations in pairs: paired FP32 compensated additions; the next
-		// 8 words are fetched while the current 8 rows are in flight
-		constexpr int NP = NPAIR;
-		f32x2 s2[NP], c2[NP];
-#pragma unroll
-		for (int h = 0; h < NP; ++h)
-			s2[h] = c2[h] = 0ull;
-		uint4 a = make_uint4(Nc, Nc, Nc, Nc), b = a;
-		if (beg < mid) {
-			a = __ldg(w4 + (beg >> 2));
-			b = __ldg(w4 + (beg >> 2) + 1);
-		}
-		for (long long j = beg; j < mid; j += 8) {
-			if constexpr (SKIP) {
-				// a group of 8 frames without a live tile adds nothing
-				if (!(live[a.x] | live[a.y] | live[a.z] | live[a.w] | live[b.x] | live[b.y] | live[b.z] |
-				      live[b.w])) {
-					if (j + 8 < mid) {
-						a = __ldg(w4 + ((j + 8) >> 2));
-						b = __ldg(w4 + ((j + 8) >> 2) + 1);
-					}
-					continue;
-				}
-			}
-			f32x2 v[8][NP];
-			ld_pairs(Pr + lv(a.x) * TILE, v[0]);
-			ld_pairs(Pr + lv(a.y) * TILE, v[1]);
-			ld_pairs(Pr + lv(a.z) * TILE, v[2]);
-			ld_pairs(Pr + lv(a.w) * TILE, v[3]);
-			ld_pairs(Pr + lv(b.x) * TILE, v[4]);
-			ld_pairs(Pr + lv(b.y) * TILE, v[5]);
-			ld_pairs(Pr + lv(b.z) * TILE, v[6]);
-			ld_pairs(Pr + lv(b.w) * TILE, v[7]);
-			if (j + 8 < mid) {
-				a = __ldg(w4 + ((j + 8) >> 2));
-				b = __ldg(w4 + ((j + 8) >> 2) + 1);
-			}
-#pragma unroll
-			for (int q = 0; q < 8; ++q)
-#pragma unroll
-				for (int h = 0; h < NP; ++h) {
-					float lo, hi;
-					f2_unpack(v[q][h], lo, hi);
-					kahan_add2(s2[h], c2[h], f2_pack(fmaxf(lo, 0.f), fmaxf(hi, 0.f)));
-				}
-		}
-		for (long long j = mid; j < end; j += 8) {
-			const uint4 a = __ldg(w4 + (j >> 2)), b = __ldg(w4 + (j >> 2) + 1);
-			const uint32_t e[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-			if constexpr (SKIP) {
-				uint32_t any = 0;
-#pragma unroll
-				for (int q = 0; q < 8; ++q)
-					any |= live[e[q] & IDX_MASK];
-				if (!any)
-					continue;
-			}
-			f32x2 v[8][NP];
-#pragma unroll
-			for (int q = 0; q < 8; ++q)
-				ld_pairs(Pr + lv(e[q] & IDX_MASK) * TILE, v[q]);
-#pragma unroll
-			for (int q = 0; q < 8; ++q)
-#pragma unroll
-				for (int h = 0; h < NP; ++h) {
-					float lo, hi;
-					f2_unpack(v[q][h], lo, hi);
-					kahan_add_count2(s2[h], c2[h], e[q] >> IDX_BITS, f2_pack(fmaxf(lo, 0.f), fmaxf(hi, 0.f)));
-				}
-		}
-#pragma unroll
-		for (int h = 0; h < NP; ++h) {
-			f2_unpack(s2[h], s[0][2 * h], s[0][2 * h + 1]);
-			f2_unpack(c2[h], c[0][2 * h], c[0][2 * h + 1]);
-		}
-	} else {
-#pragma unroll 2
+	for (int h = 0; h < NP; ++h)
+		s2[h] = c2[h] = 0ull;
+	uint4 a = make_uint4(Nc, Nc, Nc, Nc), b = a;
+	if (beg < mid) {
+		a = __ldg(w4 + (beg >> 2));
+		b = __ldg(w4 + (beg >> 2) + 1);
+	}
 	for (long long j = beg; j < mid; j += 8) {
-		const uint4 a = __ldg(w4 + (j >> 2)), b = __ldg(w4 + (j >> 2) + 1);
-		float v[8][LW];
-		ld_row(Pr + lv(a.x) * TILE, v[0]);
-		ld_row(Pr + lv(a.y) * TILE, v[1]);
-		ld_row(Pr + lv(a.z) * TILE, v[2]);
-		ld_row(Pr + lv(a.w) * TILE, v[3]);
-		ld_row(Pr + lv(b.x) * TILE, v[4]);
-		ld_row(Pr + lv(b.y) * TILE, v[5]);
-		ld_row(Pr + lv(b.z) * TILE, v[6]);
-		ld_row(Pr + lv(b.w) * TILE, v[7]);
+		if constexpr (SKIP) {
+			// a group of 8 frames without a live tile adds nothing
+			if (!(live[a.x] | live[a.y] | live[a.z] | live[a.w] | live[b.x] | live[b.y] | live[b.z] |
+			      live[b.w])) {
+				if (j + 8 < mid) {
+					a = __ldg(w4 + ((j + 8) >> 2));
+					b = __ldg(w4 + ((j + 8) >> 2) + 1);
+				}
+				continue;
+			}
+		}
+		f32x2 v[8][NP];
+		ld_pairs(Pr + lv(a.x) * TILE, v[0]);
+		ld_pairs(Pr + lv(a.y) * TILE, v[1]);
+		ld_pairs(Pr + lv(a.z) * TILE, v[2]);
+		ld_pairs(Pr + lv(a.w) * TILE, v[3]);
+		ld_pairs(Pr + lv(b.x) * TILE, v[4]);
+		ld_pairs(Pr + lv(b.y) * TILE, v[5]);
+		ld_pairs(Pr + lv(b.z) * TILE, v[6]);
+		ld_pairs(Pr + lv(b.w) * TILE, v[7]);
+		if (j + 8 < mid) {
+			a = __ldg(w4 + ((j + 8) >> 2));
+			b = __ldg(w4 + ((j + 8) >> 2) + 1);
+		}
 #pragma unroll
 		for (int q = 0; q < 8; ++q)
 #pragma unroll
-			for (int k = 0; k < LW; ++k)
-				kahan_add(s[q % ECH][k], c[q % ECH][k], fmaxf(v[q][k], 0.f));
+			for (int h = 0; h < NP; ++h) {
+				float lo, hi;
+				f2_unpack(v[q][h], lo, hi);
+				kahan_add2(s2[h], c2[h], f2_pack(fmaxf(lo, 0.f), fmaxf(hi, 0.f)));
+			}
 	}
 	for (long long j = mid; j < end; j += 8) {
 		const uint4 a = __ldg(w4 + (j >> 2)), b = __ldg(w4 + (j >> 2) + 1);
 		const uint32_t e[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-		float v[8][LW];
+		if constexpr (SKIP) {
+			uint32_t any = 0;
+#pragma unroll
+			for (int q = 0; q < 8; ++q)
+				any |= live[e[q] & IDX_MASK];
+			if (!any)
+				continue;
+		}
+		f32x2 v[8][NP];
 #pragma unroll
 		for (int q = 0; q < 8; ++q)
-			ld_row(Pr + lv(e[q] & IDX_MASK) * TILE, v[q]);
+			ld_pairs(Pr + lv(e[q] & IDX_MASK) * TILE, v[q]);
 #pragma unroll
 		for (int q = 0; q < 8; ++q)
 #pragma unroll
-			for (int k = 0; k < LW; ++k)
-				kahan_add_count(s[q % ECH][k], c[q % ECH][k], e[q] >> IDX_BITS, fmaxf(v[q][k], 0.f));
+			for (int h = 0; h < NP; ++h) {
+				float lo, hi;
+				f2_unpack(v[q][h], lo, hi);
+				kahan_add_count2(s2[h], c2[h], e[q] >> IDX_BITS, f2_pack(fmaxf(lo, 0.f), fmaxf(hi, 0.f)));
+			}
 	}
+#pragma unroll
+	for (int h = 0; h < NP; ++h) {
+		f2_unpack(s2[h], s[2 * h], s[2 * h + 1]);
+		f2_unpack(c2[h], c[2 * h], c[2 * h + 1]);
 	}
 	float *out = T + ((size_t)rl * P + p) * TILE + lane * LW;
 	float o[LW];
 	ld_row_rw(out, o);
 #pragma unroll
 	for (int k = 0; k < LW; ++k) {
-		double t = kahan_value(s[0][k], c[0][k]);
-		if (ECH == 2)
-			t = dadd(t, kahan_value(s[ECH - 1][k], c[ECH - 1][k]));
+		double t = kahan_value(s[k], c[k]);
 		o[k] = (float)((double)o[k] + t);
 	}
 	st_row(out, o);

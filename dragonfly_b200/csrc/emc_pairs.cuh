@@ -37,12 +37,10 @@ __device__ __forceinline__ void pair_photon_sums(const float *__restrict__ L, co
                                                  long long beg, long long mid, long long end, int P,
                                                  double (&out)[LW]) {
 	const uint4 *w4 = reinterpret_cast<const uint4 *>(ph);
-	float s[ECH][LW], c[ECH][LW];
+	float s[LW], c[LW];
 #pragma unroll
-	for (int h = 0; h < ECH; ++h)
-#pragma unroll
-		for (int k = 0; k < LW; ++k)
-			s[h][k] = c[h][k] = 0.f;
+	for (int k = 0; k < LW; ++k)
+		s[k] = c[k] = 0.f;
 	uint4 a = make_uint4(P, P, P, P), b = a;
 	if (beg < mid) {
 		a = __ldg(w4 + (beg >> 2));
@@ -66,7 +64,7 @@ __device__ __forceinline__ void pair_photon_sums(const float *__restrict__ L, co
 		for (int q = 0; q < 8; ++q)
 #pragma unroll
 			for (int k = 0; k < LW; ++k)
-				kahan_add(s[q % ECH][k], c[q % ECH][k], v[q][k]);
+				kahan_add(s[k], c[k], v[q][k]);
 	}
 	for (long long j = mid; j < end; j += 8) {
 		const uint4 a2 = __ldg(w4 + (j >> 2)), b2 = __ldg(w4 + (j >> 2) + 1);
@@ -79,15 +77,11 @@ __device__ __forceinline__ void pair_photon_sums(const float *__restrict__ L, co
 		for (int q = 0; q < 8; ++q)
 #pragma unroll
 			for (int k = 0; k < LW; ++k)
-				kahan_add_count(s[q % ECH][k], c[q % ECH][k], e[q] >> IDX_BITS, v[q][k]);
+				kahan_add_count(s[k], c[k], e[q] >> IDX_BITS, v[q][k]);
 	}
 #pragma unroll
-	for (int k = 0; k < LW; ++k) {
-		double v = kahan_value(s[0][k], c[0][k]);
-		if (ECH == 2)
-			v = dadd(v, kahan_value(s[ECH - 1][k], c[ECH - 1][k]));
-		out[k] = v;
-	}
+	for (int k = 0; k < LW; ++k)
+		out[k] = kahan_value(s[k], c[k]);
 }
 
 // E-step of the pairs [q0, q0 + nq) (all in the orientation block whose first

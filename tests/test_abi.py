@@ -25,6 +25,14 @@ def test_library_exports_every_declared_symbol():
     assert declared == set(_lib._SIGS), sorted(declared ^ set(_lib._SIGS))
 
 
+def test_lane_width_two_compiles(tmp_path):
+    """The narrower orientation tile (DFG_LANE_W 2: 64 orientations, no integer products)."""
+    from dragonfly_b200 import build
+    subprocess.run([build.nvcc(), "-O0", "-std=c++17", "-gencode", "arch=compute_100a,code=compute_100a",
+                    "--expt-relaxed-constexpr", "-DDFG_LANE_W=2", "-ptx", "-o", str(tmp_path / "out"),
+                    os.path.join(build.CSRC, "emc_api.cu")], check=True, stdout=subprocess.DEVNULL)
+
+
 def test_library_loads_and_reports_version():
     lib = _lib.load()
     assert lib.dfg_version().startswith(b"dragonfly_b200")
