@@ -1915,7 +1915,7 @@ static int launch_estep(dfg_ctx *ctx, const Chunk &ch, int use_scale, bool bg, c
 			DFG_ECOLD(false, 4);
 #undef DFG_ECOLD
 		CKL("estep_cold_kernel");
-		estep_ties_kernel<<<blocks_for(Nc, 32), 256, 0, st>>>(
+		estep_ties_kernel<<<blocks_for(Nc, 32), 32 * TIE_WARPS, 0, st>>>(
 		    ctx->logW.p, ctx->u.p, ctx->logw.p, R, ctx->ph.p, ctx->ph_off.p, ctx->ph_mid.p, ctx->scale.p,
 		    ctx->blacklist.p, ctx->fcounts.p, ch.d0, Nc, RT, use_scale, ctx->scalars.p, P, ctx->pval.p, ctx->tmax.p,
 		    ctx->targ.p);

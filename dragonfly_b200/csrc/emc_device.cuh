@@ -493,83 +493,121 @@ __global__ void __launch_bounds__(256, MINB) estep_cold_kernel(
 // roundings of x - comp and, where |s| < |x|, of t - s), a digit by 2^-27. For both
 // forms and two orientations that is 8u sum|x| + n 2^-26 over n photons, and sum|x|
 // <= |sum x| + 2 n 31 while no log-slice is above 31; near_tie_width is twice that.
-// Block = 32 frames: the tile maxima are read with one frame per lane, then each warp
-// looks at four frames, listing the orientations of a frame and summing up to 32
-// of them at once, one per lane.
+// Between two in a thousand and one in a hundred frames have a second orientation there.
+// Block = 32 frames, one per lane while the tile maxima are read (the warps share the
+// tiles) and the widths formed; then each warp takes four frames and counts the near
+// values in the row of their best tile. Only a frame with several, or with another
+// near tile, is slow: its orientations are listed and summed, up to 32 at once, one per
+// lane. Bound by latency: TIMES
 __device__ __forceinline__ double near_tie_width(double sum, int photons) {
 	return 0x1p-20 * (fabs(sum) + 32. * photons);
 }
 
-__global__ void __launch_bounds__(256) estep_ties_kernel(
+constexpr int TIE_WARPS = 8, TIE_FRAMES = 32 / TIE_WARPS;
+
+__global__ void __launch_bounds__(32 * TIE_WARPS) estep_ties_kernel(
     const float *__restrict__ logW, const double *__restrict__ u, const double *__restrict__ logw, int R,
     const uint32_t *__restrict__ ph, const long long *__restrict__ ph_off, const long long *__restrict__ ph_mid,
     const double *__restrict__ scale, const uint8_t *__restrict__ blacklist, const int *__restrict__ fcounts, int d0,
     int Nc, int RT, int use_scale, const double *__restrict__ scalars, int P, double *pval, double *tmax, int *targ) {
-	__shared__ double s_m[8][32];
-	__shared__ int s_a[8][32];
-	__shared__ int s_list[8][64];
-	const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	{
-		const int dl = blockIdx.x * 32 + lane;
-		double m = MAX_EXP_START;
-		int am = -1;
-		if (dl < Nc && !blacklist[d0 + dl]) {
-#pragma unroll 8
-			for (int rt = w; rt < RT; rt += 8) {
-				const double v = tmax[(size_t)rt * Nc + dl];
-				if (v > m) {
-					m = v;
-					am = rt;
-				}
-			}
-			if (am >= 0)
-				am = targ[(size_t)am * Nc + dl];
+	// largest and second largest tile maximum of each frame and warp, the tile of the
+	// largest; then the frame's tile (-1: none) and lowest near value
+	__shared__ double s_m[TIE_WARPS][32], s_n[TIE_WARPS][32], s_low[32];
+	__shared__ int s_t[TIE_WARPS][32], s_tile[32];
+	__shared__ bool s_more[32];   // another tile is near
+	__shared__ int s_list[TIE_WARPS][32 + TILE];
+	const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, dl0 = blockIdx.x * 32;
+	auto take = [](double v, int rt, double &m, double &m2, int &t) {
+		if (v > m) {
+			m2 = m;
+			m = v;
+			t = rt;
+		} else if (v > m2) {
+			m2 = v;
 		}
-		s_m[w][lane] = m;
-		s_a[w][lane] = am;
+	};
+	double m = MAX_EXP_START, m2 = MAX_EXP_START;
+	int best = -1;
+	if (dl0 + lane < Nc && !blacklist[d0 + dl0 + lane])
+#pragma unroll 8
+		for (int rt = w; rt < RT; rt += TIE_WARPS)
+			take(tmax[(size_t)rt * Nc + dl0 + lane], rt, m, m2, best);
+	s_m[w][lane] = m;
+	s_n[w][lane] = m2;
+	s_t[w][lane] = best;
+	__syncthreads();
+	if (w == 0) {
+#pragma unroll
+		for (int k = 1; k < TIE_WARPS; ++k) {
+			take(s_m[k][lane], s_t[k][lane], m, m2, best);
+			m2 = fmax(m2, s_n[k][lane]);
+		}
+		double low = 0.;
+		if (best >= 0) {
+			const int d = d0 + dl0 + lane, r = targ[(size_t)best * Nc + dl0 + lane];
+			const double sd = use_scale ? scale[d] : scalars[0];
+			low = m - near_tie_width(m - (logw[r] - u[r] * sd), fcounts[d]);
+		}
+		s_low[lane] = low;
+		s_tile[lane] = best;
+		s_more[lane] = m2 >= low;
 	}
 	__syncthreads();
+	unsigned todo = 0;   // of this warp's frames
+	double x[TIE_FRAMES][LW];
+#pragma unroll
+	for (int i = 0; i < TIE_FRAMES; ++i) {
+		const int f = w * TIE_FRAMES + i, rt = s_tile[f];
+		if (rt >= 0) {
+			const double *row = pval + ((size_t)rt * Nc + dl0 + f) * TILE + lane * LW;
+#pragma unroll
+			for (int k = 0; k < LW; ++k)
+				x[i][k] = row[k];
+		}
+	}
+#pragma unroll
+	for (int i = 0; i < TIE_FRAMES; ++i) {
+		const int f = w * TIE_FRAMES + i, rt = s_tile[f];
+		if (rt >= 0) {
+			int near = 0;
+#pragma unroll
+			for (int k = 0; k < LW; ++k)
+				near += __popc(__ballot_sync(FULL, rt * TILE + lane * LW + k < R && x[i][k] >= s_low[f]));
+			if (near > 1 || s_more[f])
+				todo |= 1u << i;
+		}
+	}
 	int *const list = s_list[w];
-	for (int f = w; f < 32; f += 8) {
-		double m = MAX_EXP_START;
-		int am = -1;
-#pragma unroll
-		for (int k = 0; k < 8; ++k)
-			if (s_m[k][f] > m) {
-				m = s_m[k][f];
-				am = s_a[k][f];
-			}
-		if (am < 0)
-			continue;
-		const int dl = blockIdx.x * 32 + f, d = d0 + dl;
-		const double sd = use_scale ? scale[d] : scalars[0];
-		const double low = m - near_tie_width(m - (logw[am] - u[am] * sd), fcounts[d]);
+#pragma unroll 1
+	for (; todo; todo &= todo - 1) {
+		const int f = w * TIE_FRAMES + __ffs(todo) - 1, dl = dl0 + f, d = d0 + dl;
+		const double low = s_low[f], sd = use_scale ? scale[d] : scalars[0];
 		const long long beg = ph_off[d], mid = ph_mid[d], end = ph_off[d + 1];
-		// the first n listed orientations, one per lane, as estep_kernel
-		auto again = [&](int n) {
+		// n of the listed orientations, one per lane, as estep_kernel
+		auto again = [&](int i0, int n) {
 			__syncwarp();
-			if (lane < n) {
-				const int r = list[lane], rt = r / TILE, j = r % TILE;
-				const float *L = logW + (size_t)rt * (P + 1) * TILE + j;
-				const uint4 *w4 = reinterpret_cast<const uint4 *>(ph);
-				float s = 0.f, c = 0.f;
-				for (long long q = beg; q < end; q += 8) {
-					const uint4 a = __ldg(w4 + (q >> 2)), b = __ldg(w4 + (q >> 2) + 1);
-					const uint32_t e[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-					const bool ones = q < mid;
-					float v[8];
+			const int r = list[i0 + (lane < n ? lane : 0)], rt = r / TILE, j = r % TILE;
+			const float *L = logW + (size_t)rt * (P + 1) * TILE + j;
+			float s = 0.f, c = 0.f;
+			// a count of 1 adds as estep_kernel's single photons do, bit for bit, and the
+			// zero row past the end (as the lists' padding) leaves s - c as it is: one
+			// form for all words
+			uint32_t next = beg + lane < end ? __ldg(ph + beg + lane) : (uint32_t)P;
+			for (long long q = beg; q < end; q += 32) {
+				const uint32_t word = next;
+				next = q + 32 + lane < end ? __ldg(ph + q + 32 + lane) : (uint32_t)P;
+				const bool one = q + lane < mid;
+				const uint32_t at = (one ? word : word & IDX_MASK) * TILE, count = one ? 1u : word >> IDX_BITS;
+				float v[32];
 #pragma unroll
-					for (int k = 0; k < 8; ++k)
-						v[k] = __ldg(L + (size_t)(ones ? e[k] : e[k] & IDX_MASK) * TILE);
+				for (int k = 0; k < 32; ++k)
+					v[k] = __ldg(L + __shfl_sync(FULL, at, k));
 #pragma unroll
-					for (int k = 0; k < 8; ++k)
-						if (ones)
-							kahan_add(s, c, v[k]);
-						else
-							kahan_add_count(s, c, e[k] >> IDX_BITS, v[k]);
-				}
-				pval[((size_t)rt * Nc + dl) * TILE + j] = dadd(dsub(logw[r], dmul(u[r], sd)), kahan_value(s, c));
+				for (int k = 0; k < 32; ++k)
+					kahan_add_count(s, c, __shfl_sync(FULL, count, k), v[k]);
 			}
+			if (lane < n)
+				pval[((size_t)rt * Nc + dl) * TILE + j] = dadd(dsub(logw[r], dmul(u[r], sd)), kahan_value(s, c));
 			__syncwarp();
 		};
 		// calls f(rt, v) for every tile whose maximum is near, v its row's values of this lane
@@ -588,7 +626,6 @@ __global__ void __launch_bounds__(256) estep_ties_kernel(
 			}
 		};
 		int n = 0;
-		bool any = false;   // several: summed again (one alone stays as it is)
 		near_tiles([&](int rt, const double (&v)[LW]) {
 #pragma unroll
 			for (int k = 0; k < LW; ++k) {
@@ -597,19 +634,11 @@ __global__ void __launch_bounds__(256) estep_ties_kernel(
 				if (got >> lane & 1u)
 					list[n + __popc(got & ((1u << lane) - 1u))] = r;
 				n += __popc(got);
-				if (n >= 32) {
-					again(32);
-					any = true;
-					n -= 32;
-					if (lane < n)
-						list[lane] = list[32 + lane];
-					__syncwarp();
-				}
 			}
+			for (; n >= 32; n -= 32)
+				again(n - 32, 32);
 		});
-		if (!any && n <= 1)
-			continue;
-		again(n);
+		again(0, n);
 		near_tiles([&](int rt, const double (&v)[LW]) {
 			double tm = MAX_EXP_START;
 			int ta = -1;
