@@ -498,7 +498,9 @@ __global__ void __launch_bounds__(256, MINB) estep_cold_kernel(
 // tiles) and the widths formed; then each warp takes four frames and counts the near
 // values in the row of their best tile. Only a frame with several, or with another
 // near tile, is slow: its orientations are listed and summed, up to 32 at once, one per
-// lane. Bound by latency: TIMES
+// lane. Bound by latency, of the few frames with the longest lists: 9 us at 420 x 450,
+// 15 at 3240 x 3000, 50 at 10860 x 30000, 99 at 6300 x 15000 with 1500 photons (with 8
+// rows in flight and the widths formed frame by frame 13, 27, 76 and 155 us).
 __device__ __forceinline__ double near_tie_width(double sum, int photons) {
 	return 0x1p-20 * (fabs(sum) + 32. * photons);
 }
