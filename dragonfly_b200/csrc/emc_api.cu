@@ -751,8 +751,8 @@ static int build_chunks(dfg_ctx *ctx) {
 		ch.nc = (int)std::min<long long>(nc, N - ch.d0);
 		const uint32_t pad = (uint32_t)ch.nc;
 		// contiguous frame ranges, one per host thread (at least a million words each,
-		// and more words than counters): every range counts its words per pixel and fills them in from its
-		// own cursors, so the lists keep the frames' order
+		// and more words than counters): every range counts its words per pixel and
+		// fills them in from its own cursors, so the lists keep the frames' order
 		const int d1 = ch.d0 + ch.nc;
 		const long long given = ctx->h_ones_off[d1] - ctx->h_ones_off[ch.d0] + ctx->h_multi_off[d1] -
 		                        ctx->h_multi_off[ch.d0];
