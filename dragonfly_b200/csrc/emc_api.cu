@@ -925,10 +925,20 @@ static int ensure_buffers(dfg_ctx *ctx) {
 	const size_t logw_n = (size_t)ctx->RT * (ctx->P + 1) * TILE;
 	if (ctx->logW.n < logw_n || ctx->T.n < tiles_px || ctx->logW_P != ctx->P) {
 		CK(ctx->tile_slab.ensure(SlabPart<float>{ctx->logW, logw_n}, SlabPart<float>{ctx->T, tiles_px}));
-		// the zero rows (pixel P of every tile) stay zero: the slice kernel
-		// writes rows 0..P-1 only
-		CK(cudaMemsetAsync(ctx->logW.p, 0, logw_n * sizeof(float), ctx->stream));
 		ctx->logW_P = ctx->P;
+		ctx->logW_tiles = 0;
+	}
+	if (ctx->logW_tiles < ctx->RT) {
+		// the zero rows (pixel P of every tile) stay zero: the slice kernel
+		// writes rows 0..P-1 only. (A buffer with room for more tiles held them at
+		// the rows of another detector: each tile is cleared before its first use.)
+		const size_t pitch = (size_t)(ctx->P + 1) * TILE * sizeof(float);
+		if (pitch <= 0x7fffffff)   // the largest pitch of a 2-D copy
+			CK(cudaMemset2DAsync(ctx->logW.p + (size_t)ctx->P * TILE, pitch, 0, TILE * sizeof(float), ctx->RT,
+			                     ctx->stream));
+		else
+			CK(cudaMemsetAsync(ctx->logW.p, 0, logw_n * sizeof(float), ctx->stream));
+		ctx->logW_tiles = ctx->RT;
 	}
 	CK(ctx->u.ensure((size_t)ctx->R_pad));
 	CK(ctx->logw.ensure((size_t)ctx->R_pad));

@@ -174,7 +174,7 @@ struct dfg_ctx {
 	DevBuf<long long> ph_off;  // [N + 1]
 	DevBuf<long long> ph_mid;  // [N] start of the multi-photon segment
 	long long n_ph = 0;        // photon words without padding
-	int logW_P = -1;           // detector size the zero row of logW was written for
+	int logW_P = -1, logW_tiles = 0;  // detector size and tiles the zero rows of logW were written for
 	DevBuf<double> scale, beta, beta_start, sum_fact;
 	DevBuf<int> fcounts;
 	DevBuf<uint8_t> blacklist;

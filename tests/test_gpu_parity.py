@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 from common import (CASES, GPUEngine, compare_iteration, load_case, rel_l2)
+from dragonfly_b200._lib import Context
 from oracle.oracle import EMCProblem, OracleEngine
 
 pytestmark = pytest.mark.gpu
@@ -130,6 +131,36 @@ def test_gpu_is_deterministic(oracle_built):
     np.testing.assert_array_equal(a["rmax"], b["rmax"])
     np.testing.assert_array_equal(a["likelihood"], b["likelihood"])
     np.testing.assert_array_equal(a["p_norm"], b["p_norm"])
+
+
+def test_gpu_context_reused_for_another_detector():
+    """A context whose log-slices have room from a small detector with many orientations
+    goes to a larger one, first with few orientations, then with more: what it finds is
+    what a new context finds."""
+    from dragonfly_b200 import synth
+    from dragonfly_b200.quatgen import quat_gen
+
+    def load(c, d, div):
+        c.set_detector(d["qvals"], d["corr"], d["mask"])
+        c.set_frames(d["ones"], d["multi"], d["place_ones"], d["place_multi"], d["count_multi"])
+        c.set_quaternions(quat_gen(div))
+        c.set_model(d["model_start"])
+        c.calc_beta(0.1, 0)
+        c.maximize(c.params(1, 0, 0, 0, 1., 100, 1.))
+        return c.frame_results()
+
+    small, large = (synth.small_problem(seed=side, det_side=side, size=side + 3, qmax=side / 2., n_atoms=40,
+                                        atom_radius=4., num_div=1, n_frames=200, mean_count=60., hole_radius=2.)
+                    for side in (24, 40))
+    used = Context(0)
+    load(used, small, 4)
+    for div in (1, 2, 3):
+        new = Context(0)
+        a, b = load(used, large, div), load(new, large, div)
+        for k in ("rmax", "likelihood", "max_exp"):
+            np.testing.assert_array_equal(a[k], b[k])
+        new.close()
+    used.close()
 
 
 def test_gpu_slice_gen_and_merge_match_oracle(oracle_built):
