@@ -143,8 +143,11 @@ extern "C" int dfg_set_detector(dfg_ctx *ctx, int num_pix, const double *qvals, 
 	if (ctx->N > 0) {
 		int rc = dfg_set_frames(ctx, ctx->N, ctx->h_ones.data(), ctx->h_multi.data(), ctx->h_place_ones.data(),
 		                        ctx->h_place_multi.data(), ctx->h_count_multi.data());
-		if (rc != DFG_OK)
+		if (rc != DFG_OK) {
+			ctx->N = 0;  // the frames are not this detector's: to be set again
+			ctx->have_results = false;
 			return rc;
+		}
 	}
 	return DFG_OK;
 }

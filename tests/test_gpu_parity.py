@@ -163,6 +163,41 @@ def test_gpu_context_reused_for_another_detector():
     used.close()
 
 
+def test_gpu_frames_beyond_a_new_detector_are_dropped():
+    """A smaller detector under frames that list pixels past it is refused, and the frames
+    with it: an iteration wants them set again."""
+    from dragonfly_b200 import synth
+    from dragonfly_b200._lib import DFG_ERR_ARG, DFG_ERR_STATE, DFGError
+    from dragonfly_b200.quatgen import quat_gen
+    small, large = (synth.small_problem(seed=side, det_side=side, size=side + 3, qmax=side / 2., n_atoms=40,
+                                        atom_radius=4., num_div=1, n_frames=50, mean_count=60., hole_radius=2.)
+                    for side in (24, 40))
+    c = Context(0)
+
+    def frames(d):
+        c.set_frames(d["ones"], d["multi"], d["place_ones"], d["place_multi"], d["count_multi"])
+
+    c.set_detector(large["qvals"], large["corr"], large["mask"])
+    frames(large)
+    c.set_quaternions(quat_gen(1))
+    c.set_model(small["model_start"])
+    c.calc_beta(0.1, 0)
+    par = c.params(1, 0, 0, 0, 1., 100, 1.)
+    c.maximize(par)
+    with pytest.raises(DFGError) as e:
+        c.set_detector(small["qvals"], small["corr"], small["mask"])
+    assert e.value.code == DFG_ERR_ARG
+    with pytest.raises(DFGError) as e:
+        c.maximize(par)
+    assert e.value.code == DFG_ERR_STATE
+    c.set_detector(small["qvals"], small["corr"], small["mask"])
+    frames(small)
+    c.calc_beta(0.1, 0)
+    c.maximize(par)
+    assert np.all(np.isfinite(c.frame_results()["likelihood"]))
+    c.close()
+
+
 def test_gpu_slice_gen_and_merge_match_oracle(oracle_built):
     import ctypes as C
     prob, _ = load_case("beta1")
