@@ -19,6 +19,9 @@
 // the gathers add; the probabilities are taken relative to their orientation's
 // largest in the chunk (4.2e9 steps), 1.2e-10 of it, far below the FP32 rounding of
 // the tomogram they end in. The remaining (cold) photons are gathered as before.
+// Errors against 64 bits over those of the gathers alone (seven shapes, 16 seeds each):
+// log-likelihoods 0.62 to 0.81, models 0.83 to 1.03, within their seeds' spread of
+// 0.6 to 1.5; with |log W| small everywhere (one photon per pixel) 0.78 and 0.97.
 //
 // One CTA per SM walks tiles of 256 rows (frames or pixels) x 64 orientations:
 //   warp 0      TMA producer: per 128-deep block the 256 x 128 count tile and
@@ -482,7 +485,8 @@ __global__ void __launch_bounds__(256) hot_counts_kernel(const uint32_t *__restr
 // list's two segments (counts), then the lists, each segment padded to 8 words
 // with `pad`. A count of up to COLD_REPEAT becomes that many count-1 words: the
 // few such photons of a cold pixel would take a segment of their own, padded to 8
-// rows. One warp per list. BY_LIST false: lists of pixels per frame (E-step), hot
+// rows. (Each of them rounds by itself, where a counted word's product is exact; the
+// errors at the head of this file include that.) One warp per list. BY_LIST false: lists of pixels per frame (E-step), hot
 // words dropped; true: lists of frames per pixel (M-step), hot lists dropped.
 // Words naming `limit` or above are padding.
 constexpr uint32_t COLD_REPEAT = 4;
